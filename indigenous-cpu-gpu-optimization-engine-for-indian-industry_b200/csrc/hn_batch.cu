@@ -17,18 +17,42 @@
 //     with the reference's pivot clamp (factorization.cpp:1299-1305), level-
 //     synchronously in 64-column blocks: per block one launch factorises every
 //     instance's diagonal block, one spreads all instances' panel rows and one
-//     all instances' trailing tiles over the GPU. This is a deliberate
+//     all instances' output tiles over the GPU. This is a deliberate
 //     deviation from keeping factorisations on the host: thousands of
 //     factorisations per iteration do not fit in host time;
-//   - the two triangular solves, level-synchronous in the same blocks, and
-//     iterative refinement (refinement.cpp:7-37: up to 5 sweeps, stop at
+//   - the two triangular solves, one launch for the batch (a CTA or a cluster
+//     of CTAs per instance), and iterative refinement (refinement.cpp:7-37: up to 5 sweeps, stop at
 //     1e-10 relative) per instance, with N x as one SpMV over the packed N.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include "hn_spmv.cuh"
+
+namespace hn {
+// Where an instance lies: one 32-byte load instead of a chain through the offsets.
+struct __align__(16) InstInfo {
+    int64_t r0;  // first packed row
+    int64_t dn;  // offset of its dense block
+    int32_t m;
+    int32_t pad[3];
+};
+
+// A chunk of 256 (kT) rows below a diagonal block: its instance and its number there.
+struct Chunk {
+    int32_t inst, local;
+};
+
+// What a CTA of the solve kernel works on.
+struct SolveSlot {
+    int32_t inst;   // -1: nothing (its cluster's barriers only)
+    int32_t rank, size;
+    int32_t steps;  // blocks of the largest instance in the cluster, 0: its instances are all one CTA's
+};
+
+}  // namespace hn
 
 struct hn_batch {
     int64_t K = 0, m = 0, n = 0;
@@ -49,20 +73,23 @@ struct hn_batch {
     double *carry_val = nullptr, *head_val = nullptr;
     double* r = nullptr;         // refinement residual, m
     double* ax = nullptr;        // N x, m
+    hn::InstInfo* info = nullptr;  // K
     // level schedule of the blocked factorisation: at block step s the
-    // instances order[0 .. cnt[s]) still have a block; step_pairs (offset
-    // pair_off[s]) holds, per such instance, the cumulative count of trailing
-    // 32x32 tile pairs, so one launch spreads every instance's tiles over the GPU
+    // instances order[0 .. cnt[s]) still have a block. Their 64 x 64 output
+    // tiles of the update that follows step s (the next block column after an
+    // even step, the whole trailing triangle after an odd one) as cumulative
+    // counts per (step, instance), and the kT-row chunks below their diagonal
+    // blocks as a list per step, spread every instance's work over the GPU.
     int64_t nsteps = 0;
-    std::vector<int32_t> step_cnt;       // host, nsteps
-    std::vector<int64_t> step_pairs_h;   // host, total pairs per step
-    std::vector<int64_t> pair_off_h;     // host, nsteps+1 offsets into step_pairs
-    int64_t* step_pairs = nullptr;       // device, cumulative pairs per (step, instance)
-    // panel rows below each instance's diagonal block, in chunks of kT rows
-    std::vector<int64_t> step_chunks_h;  // host, total chunks per step
-    std::vector<int64_t> chunk_off_h;    // host, nsteps+1 offsets into step_chunks
-    int64_t* step_chunks = nullptr;      // device, cumulative chunks per (step, instance)
-    double* solve_part = nullptr;        // backward-solve partial dot products, 64 per chunk
+    std::vector<int32_t> step_cnt;                       // host, nsteps
+    std::vector<int64_t> tile_off_h, chunk_off_h;        // host, nsteps+1 offsets into the two tables
+    std::vector<int64_t> step_tiles_h;                   // host, tiles per step
+    int64_t* step_tiles = nullptr;                       // device
+    hn::Chunk* chunks = nullptr;                         // device
+    int64_t nslots = 0, solve_smem = 0;
+    hn::SolveSlot* slots = nullptr;  // the solve kernel's CTAs, whole clusters
+    double* work = nullptr;          // solved blocks of the forward pass, m
+    double* solve_part = nullptr;    // backward partial dot products, two times 64 per chunk
     // relative KKT residual per instance and the tightening past the
     // reference's stop (hn_batch_set_kkt): ru / cu / offset are caller-owned
     // unscale factors (null = not measured); kkt and kkt_ref hold K x 4
@@ -383,16 +410,16 @@ __global__ void batch_dense_kernel(int64_t m, const int64_t* __restrict__ row_of
     }
 }
 
-// Blocked right-looking LDL^T, level-synchronous over the batch, in blocks of
-// kFb columns: block step s runs two launches for every instance that still
-// has a block s --
+// Blocked LDL^T, level-synchronous over the batch, in blocks of kFb columns:
+// block step s runs for every instance that still has a block s --
 //   batch_ldlt_diag_kernel: one CTA per instance factorises the kFb x kFb
 //     diagonal block (pivot clamp of factorization.cpp:1299-1305);
 //   batch_ldlt_panel_kernel: every instance's panel below its diagonal block,
 //     in chunks of kT rows spread over the GPU, one row per thread;
-//   batch_ldlt_update_kernel: all instances' trailing kFb x kFb tiles
-//     A_rc -= sum_q (L_rq D_q) L_cq, spread over every CTA of the GPU, on the
-//     FP64 tensor cores (mma.sync m8n8k4, FP64 in and out).
+//   batch_ldlt_update_kernel: A_rc -= sum_q (L_rq D_q) L_cq on the FP64 tensor
+//     cores (mma.sync m8n8k4, FP64 in and out), after an even step for the
+//     next block column only, after an odd one for the rest of the trailing
+//     matrix by both panels.
 constexpr int kFb = 64;
 
 // D(8x8) += A(8x4) B(4x8) in FP64 on the tensor cores. Fragments: lane l
@@ -403,324 +430,224 @@ __device__ __forceinline__ void dmma_m8n8k4(double* d, double a, double b) {
                  : "d"(a), "d"(b));
 }
 constexpr int kFbP = kFb + 1;  // padded smem row (conflict-free column walks)
-constexpr size_t kPanelSmem = sizeof(double) * (2 * kFb * kFbP + 2 * kFb);
 
-__global__ void __launch_bounds__(kT) batch_ldlt_diag_kernel(int s, const int64_t* __restrict__ row_off,
-                                                             const int64_t* __restrict__ dn_off,
+// Quotients by a common divisor, correctly rounded as a / d is, from its
+// correctly rounded reciprocal y: two residual corrections q + (a - d q) y
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990: a quotient within one ulp, its
+// exact residual and a correctly rounded reciprocal give the rounded
+// quotient; the first step brings a y within one ulp). Independent quotients
+// overlap, which divisions -- each a branch around its rare cases -- do not:
+// 43 cycles of latency against 127 each. Holds while nothing under- or
+// overflows on the way: in_range() of both (zeros are fine) and
+// good_divisor(d); a / d otherwise.
+__device__ __forceinline__ double quotient(double a, double d, double y) {
+    double q = a * y;
+    q = __fma_rn(__fma_rn(-d, q, a), y, q);
+    return __fma_rn(__fma_rn(-d, q, a), y, q);
+}
+// 2^-400 <= |v| < 2^401: exponent field 623 .. 1423
+__device__ __forceinline__ bool in_range(double v) {
+    return ((static_cast<unsigned>(__double2hiint(v)) >> 20) & 0x7ffu) - 623u <= 800u;
+}
+
+// A divisor whose reciprocal() is the rounded one: the last Newton step may
+// miss it for a mantissa of all ones.
+__device__ __forceinline__ bool good_divisor(double d) {
+    const bool ones = static_cast<unsigned>(__double2loint(d)) == 0xffffffffu &&
+                      (static_cast<unsigned>(__double2hiint(d)) & 0xfffffu) == 0xfffffu;
+    return in_range(d) && !ones;
+}
+
+// 1 / d, correctly rounded, for good_divisor(d): Newton steps from the hardware's
+// approximation, the last one from an iterate within one ulp (Markstein, as
+// above); no branch.
+__device__ __forceinline__ double reciprocal(double d) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) y = __fma_rn(__fma_rn(-d, y, 1.0), y, y);
+    return __fma_rn(__fma_rn(-d, y, 1.0), y, y);
+}
+
+// LDL^T of one instance's diagonal block per CTA: a chain of 64 pivots (form
+// the clamped pivot, divide its column, update), so its time is the latency
+// of a pivot. Four pivots go per round, to share the exchange between the
+// warps. Thread (r, g) keeps of row r the column quads 4 i + g (i = 0 .. 3) in
+// registers. The threads that own quad 4 i + g read its 4 x 4 pivot block
+// from shared memory, factorise it (all of them the same) and divide their
+// row's four columns; a barrier later the owners of the next quad bring it up
+// to date and publish its pivot block; the other columns are updated while
+// the next round's divisions are under way. A barrier per pivot, its shuffle
+// and its trip through shared memory cost more than the division. An element
+// takes A_rc -= (l_rj d_j) l_cj for j ascending, each product and difference
+// rounded, the reference's elimination order; what a thread computes above
+// the diagonal or past the block is never read.
+// 384 LPs of m 50-2000 (31 blocks): 588 us, 1,558 with the block in shared
+// memory and two barriers per pivot; one wave of blocks 15 us (41 before).
+struct DiagShared {
+    double A[kFb][kFbP];
+    double lc[2][4][kFb];  // the round's four columns of L, by the parity of the round
+    double pb[4][4];       // the next pivot block (its lower triangle)
+    double d[kFb];
+};
+
+// a[4] -= a round's four columns: row factors w[q] = l_rq d_q, columns c .. c + 3
+__device__ __forceinline__ void diag_update(double* a, const double* w, const double (*lc)[kFb], int c) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[e] -= w[q] * lc[q][c + e];
+}
+
+// Four pivots: the pivot block pb (lower triangle) gives d[q] and, in a, row
+// r's four columns of L. `plain` divides; the other way is the fast one and
+// returns false where its quotients may not be the rounded ones.
+template <bool plain>
+__device__ __forceinline__ bool diag_pivots(const double (*pb)[4], double tol, double* a, double* d) {
+    double l[4][4], t[4][4];
+    bool fine = true;
+    auto ok = [](double v) { return in_range(v) || v == 0.0; };
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = q; e < 4; ++e) t[e][q] = pb[e][q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        d[q] = t[q][q];
+        if (d[q] <= tol) d[q] = tol;  // SparseCholesky pivot clamp
+        const double y = plain ? 0.0 : reciprocal(d[q]);
+        if (!plain) fine = fine && good_divisor(d[q]) && ok(a[q]);
+#pragma unroll
+        for (int e = q + 1; e < 4; ++e) {
+            l[e][q] = plain ? t[e][q] / d[q] : quotient(t[e][q], d[q], y);
+            if (!plain) fine = fine && ok(t[e][q]);
+        }
+        a[q] = plain ? a[q] / d[q] : quotient(a[q], d[q], y);
+        const double wr = a[q] * d[q];
+#pragma unroll
+        for (int e = q + 1; e < 4; ++e) {
+            const double we = l[e][q] * d[q];
+#pragma unroll
+            for (int f = q + 1; f <= e; ++f) t[e][f] -= we * l[f][q];
+            a[e] -= wr * l[e][q];
+        }
+    }
+    return fine;
+}
+__device__ __noinline__ void diag_pivots_plain(const double (*pb)[4], double tol, double* a, double* d) {
+    diag_pivots<true>(pb, tol, a, d);
+}
+
+// Rounds 4 I .. 4 I + 3 (pivots 16 I .. 16 I + 15). On entry and return the
+// columns right of the previous round's successor still lack that round (row
+// factors w, columns of L of the parity before): each round's owners take it
+// after their pivots, the others before the round's first barrier.
+template <int I>
+__device__ __forceinline__ void diag_rounds(DiagShared& sh, double (*a)[4], double* w, int nb, double tol, int r,
+                                            int g) {
+#pragma unroll 1
+    for (int og = 0; og < 4; ++og) {
+        const int j0 = 16 * I + 4 * og;
+        if (j0 >= nb) return;
+        double(*lc)[kFb] = sh.lc[og & 1];
+        // the previous round's update right of this round's quad
+        auto rest = [&]() {
+            if (I == 0 && og == 0) return;
+            const double(*lp)[kFb] = sh.lc[(og & 1) ^ 1];
+            if (g > og) diag_update(a[I], w, lp, 16 * I + 4 * g);
+#pragma unroll
+            for (int i = I + 1; i < 4; ++i) diag_update(a[i], w, lp, 16 * i + 4 * g);
+        };
+        if (g == og) {
+            double d[4], t[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) t[q] = a[I][q];
+            if (!diag_pivots<false>(sh.pb, tol, a[I], d)) {
+                diag_pivots_plain(sh.pb, tol, t, d);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a[I][q] = t[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                lc[q][r] = a[I][q];
+                sh.A[r][j0 + q] = a[I][q];
+                if (r == 0) sh.d[j0 + q] = d[q];
+            }
+        } else {
+            rest();
+        }
+        __syncthreads();
+        if (g == og) rest();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[q] = lc[q][r] * sh.d[j0 + q];
+        if (g == ((og + 1) & 3) && j0 + 4 < kFb) {  // the next round's owners
+            if (og < 3)
+                diag_update(a[I], w, lc, j0 + 4);
+            else
+                diag_update(a[I < 3 ? I + 1 : 3], w, lc, j0 + 4);
+            if (r >= j0 + 4 && r < j0 + 8) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sh.pb[r - j0 - 4][e] = og < 3 ? a[I][e] : a[I < 3 ? I + 1 : 3][e];
+            }
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kT) batch_ldlt_diag_kernel(int s, const InstInfo* __restrict__ info,
                                                              const int32_t* __restrict__ order,
                                                              const int32_t* __restrict__ status,
                                                              double* __restrict__ dense, double* __restrict__ dD,
                                                              double tol) {
-    extern __shared__ double smem[];
-    double(*sA)[kFbP] = reinterpret_cast<double(*)[kFbP]>(smem);
-    double(*sL)[kFbP] = reinterpret_cast<double(*)[kFbP]>(smem + kFb * kFbP);
-    double* sD = smem + 2 * kFb * kFbP;
-    double* sLc = sD + kFb;  // column j of L during pivot j
+    __shared__ DiagShared sh;
     const int tid = threadIdx.x;
     const int inst = order[blockIdx.x];
     if (status[inst] != ST_RUN) return;
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
+    const InstInfo in = info[inst];
+    const int ld = dense_ld(in.m);
     const int k0 = s * kFb;
-    if (k0 >= m) return;
-    const int nb = min(kFb, m - k0);
-    double* A = dense + dn_off[inst];
-    for (int idx = tid; idx < kFb * kFb; idx += kT) {
-        const int r = idx / kFb, c = idx % kFb;
-        sA[r][c] = (r < nb && c <= r) ? A[(int64_t)(k0 + r) * ld + k0 + c] : 0.0;
+    const int nb = min(kFb, in.m - k0);
+    double* A = dense + in.dn + (int64_t)k0 * ld + k0;
+    const int col = tid & (kFb - 1), row = tid >> 6;
+    double v[kFb / 4];
+#pragma unroll
+    for (int i = 0; i < kFb / 4; ++i) {
+        const int rr = 4 * i + row;
+        v[i] = (rr < nb && col <= rr) ? A[(int64_t)rr * ld + col] : 0.0;
     }
+#pragma unroll
+    for (int i = 0; i < kFb / 4; ++i) sh.A[4 * i + row][col] = v[i];
     __syncthreads();
-    // pivot j: every thread forms the clamped pivot itself; column j of L,
-    // l = A_.,j / d, is divided out once (to sLc and sL; column j of sA stays
-    // unscaled); then warp w takes rows rr = j + 1 + w, j + 9 + w, ..., lanes
-    // the columns j < cc <= rr, and each element takes A_rr,cc -= (l_rr d) l_cc:
-    // the sequence and roundings of the column-by-column elimination
-    const int lane = tid & 31, warp = tid >> 5;
-    for (int j = 0; j < nb; ++j) {
-        double d = sA[j][j];
-        if (d <= tol) d = tol;  // SparseCholesky pivot clamp
-        if (tid == 0) sD[j] = d;
-        for (int cc = j + 1 + tid; cc < nb; cc += kT) {
-            const double l = sA[cc][j] / d;
-            sLc[cc] = l;
-            sL[cc][j] = l;
-        }
-        __syncthreads();
-        for (int rr = j + 1 + warp; rr < nb; rr += kT / 32) {
-            const double wr = sLc[rr] * d;
-            for (int cc = j + 1 + lane; cc <= rr; cc += 32) sA[rr][cc] -= wr * sLc[cc];
-        }
-        __syncthreads();
+    const int r = tid & (kFb - 1), g = tid >> 6;
+    double a[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[i][e] = sh.A[r][16 * i + 4 * g + e];
+    if (tid < 16) sh.pb[tid >> 2][tid & 3] = sh.A[tid >> 2][tid & 3];
+    __syncthreads();  // the columns of L overwrite sh.A
+    double w[4];
+    diag_rounds<0>(sh, a, w, nb, tol, r, g);
+    diag_rounds<1>(sh, a, w, nb, tol, r, g);
+    diag_rounds<2>(sh, a, w, nb, tol, r, g);
+    diag_rounds<3>(sh, a, w, nb, tol, r, g);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kFb / 4; ++i) {
+        const int rr = 4 * i + row;
+        if (rr < nb && col < rr) A[(int64_t)rr * ld + col] = sh.A[rr][col];
     }
-    for (int idx = tid; idx < nb * nb; idx += kT) {
-        const int r = idx / nb, c = idx % nb;
-        if (c < r) A[(int64_t)(k0 + r) * ld + k0 + c] = sL[r][c];
-    }
-    if (tid < nb) dD[r0 + k0 + tid] = sD[tid];
+    if (tid < nb) dD[in.r0 + k0 + tid] = sh.d[tid];
 }
 
-// L[r, k0:k1] = A[r, k0:k1] (L_blk D)^-T for the kT rows of chunk `local`
-// of one instance's panel (the instance: first b with chunks[b] > chunk).
-__global__ void __launch_bounds__(kT) batch_ldlt_panel_kernel(int s, int cnt, const int64_t* __restrict__ chunks,
-                                                              const int64_t* __restrict__ row_off,
-                                                              const int64_t* __restrict__ dn_off,
-                                                              const int32_t* __restrict__ order,
-                                                              const int32_t* __restrict__ status,
-                                                              double* __restrict__ dense,
-                                                              const double* __restrict__ dD) {
-    __shared__ double sL[kFb][kFbP];
-    __shared__ double sD[kFb];
-    const int tid = threadIdx.x;
-    const int64_t chunk = blockIdx.x;
+// The entry of `cum` (inclusive cumulative counts of cnt instances) that item
+// `idx` falls into.
+__device__ __forceinline__ int item_instance(const int64_t* cum, int cnt, int64_t idx) {
     int lo = 0, hi = cnt - 1;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (chunks[mid] <= chunk)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    const int inst = order[lo];
-    if (status[inst] != ST_RUN) return;
-    const int64_t local = chunk - (lo > 0 ? chunks[lo - 1] : 0);
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
-    const int k0 = s * kFb;
-    const int nb = min(kFb, m - k0), k1 = k0 + nb;
-    double* A = dense + dn_off[inst];
-    for (int idx = tid; idx < kFb * kFb; idx += kT) {
-        const int r = idx / kFb, c = idx % kFb;
-        sL[r][c] = (r < nb && c < r) ? A[(int64_t)(k0 + r) * ld + k0 + c] : 0.0;
-    }
-    if (tid < kFb) sD[tid] = tid < nb ? dD[r0 + k0 + tid] : 1.0;
-    __syncthreads();
-    const int r = k1 + static_cast<int>(local) * kT + tid;
-    if (r >= m) return;
-    // lv[c] holds A[r, k0 + c] until column c is final; then L[r, c] goes to
-    // memory and lv[c] keeps L[r, c] D_c, the factor every later column
-    // multiplies (the same single rounding as computing it there each time)
-    double lv[kFb];
-    double* Ar = A + (int64_t)r * ld + k0;
-#pragma unroll
-    for (int c = 0; c < kFb; ++c) lv[c] = (c < nb) ? Ar[c] : 0.0;
-#pragma unroll
-    for (int c = 0; c < kFb; ++c) {
-        if (c < nb) {
-            double v = lv[c];
-#pragma unroll
-            for (int q = 0; q < c; ++q) v -= lv[q] * sL[c][q];
-            const double l = v / sD[c];
-            Ar[c] = l;
-            lv[c] = l * sD[c];
-        }
-    }
-}
-
-// Trailing update of one 64 x 64 tile pair per CTA iteration. Both 64-column
-// panel slices arrive by 16-byte asynchronous copies (rows start on 16-byte
-// boundaries: even row stride), in two commit groups of 32 columns, so the
-// second half is in flight while the first is multiplied; the output tile
-// arrives the same way (a third group) and is read back from shared memory in
-// the epilogue. D is applied at the
-// fragment load: a = L[r, k] D_k rounds once, as a staged product would, and
-// every output fragment takes the same DMMA sequence (k ascending in steps of
-// 4), so the result does not depend on the staging.
-constexpr int kUpdP = kFb + 4;  // smem row stride: a half-warp's fragment loads hit 16 distinct bank pairs
-constexpr size_t kUpdSmem = sizeof(double) * (3 * kFb * kUpdP + kFb);
-
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
-
-struct UpdPair {
-    int m, ld, rb, cb;
-    int64_t r0;
-    double* A;
-};
-
-// Persistent: each CTA walks pairs blockIdx.x, + grid, ... and overlaps the
-// next pair's panel copies with the current pair's epilogue (the panels are
-// free once the multiply is done; the output tile's buffer once the epilogue
-// has read it).
-__global__ void __launch_bounds__(kT, 2) batch_ldlt_update_kernel(int s, int cnt, int64_t npairs,
-                                                               const int64_t* __restrict__ pairs,
-                                                               const int64_t* __restrict__ row_off,
-                                                               const int64_t* __restrict__ dn_off,
-                                                               const int32_t* __restrict__ order,
-                                                               const int32_t* __restrict__ status,
-                                                               double* __restrict__ dense,
-                                                               const double* __restrict__ dD) {
-    extern __shared__ __align__(16) double upd_smem[];
-    double(*sW)[kUpdP] = reinterpret_cast<double(*)[kUpdP]>(upd_smem);                // L[rb + r, k0 + k]
-    double(*sL)[kUpdP] = reinterpret_cast<double(*)[kUpdP]>(upd_smem + kFb * kUpdP);  // L[cb + c, k0 + k]
-    double(*sC)[kUpdP] = reinterpret_cast<double(*)[kUpdP]>(upd_smem + 2 * kFb * kUpdP);  // A[rb + r, cb + c]
-    double* sD = upd_smem + 3 * kFb * kUpdP;
-    const int tid = threadIdx.x;
-    const int k0 = s * kFb;
-    const int k1 = k0 + kFb;  // a trailing part exists only below a full block
-    int lo = 0;               // the instance of the previous pair: pairs arrive in increasing order
-    int64_t pidx = blockIdx.x;
-    // the next pair of a running instance from pidx on (pidx moves past it);
-    // the same answer in every thread
-    auto next_pair = [&](UpdPair& P) -> bool {
-        for (; pidx < npairs; pidx += gridDim.x) {
-            // instance of this pair: first b with pairs[b] > pidx (pairs is
-            // inclusive), searched from the previous one by doubling steps
-            if (pairs[lo] <= pidx) {
-                int step = 1, base = lo;
-                while (base + step < cnt - 1 && pairs[base + step] <= pidx) {
-                    base += step;
-                    step <<= 1;
-                }
-                int a = base + 1, b = min(base + step, cnt - 1);
-                while (a < b) {
-                    const int mid = (a + b) >> 1;
-                    if (pairs[mid] <= pidx)
-                        a = mid + 1;
-                    else
-                        b = mid;
-                }
-                lo = a;
-            }
-            const int inst = order[lo];
-            if (status[inst] != ST_RUN) continue;
-            const int64_t local = pidx - (lo > 0 ? pairs[lo - 1] : 0);
-            int ti = static_cast<int>((sqrt(8.0 * (double)local + 1.0) - 1.0) * 0.5);
-            while ((int64_t)(ti + 1) * (ti + 2) / 2 <= local) ++ti;
-            while ((int64_t)ti * (ti + 1) / 2 > local) --ti;
-            const int tj = static_cast<int>(local - (int64_t)ti * (ti + 1) / 2);
-            P.r0 = row_off[inst];
-            P.m = static_cast<int>(row_off[inst + 1] - P.r0);
-            P.ld = dense_ld(P.m);
-            P.rb = k1 + ti * kFb;
-            P.cb = k1 + tj * kFb;
-            P.A = dense + dn_off[inst];
-            pidx += gridDim.x;
-            return true;
-        }
-        return false;
-    };
-    // 2 slices x 64 rows x 16 chunks of 16 bytes per half, one commit group
-    // per half; rows past m are zero-filled
-    auto issue_panels = [&](const UpdPair& P) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            for (int idx = tid; idx < 2 * kFb * 16; idx += kT) {
-                const int side = idx >> 10, rr = (idx >> 4) & (kFb - 1), q2 = idx & 15;
-                const int row = (side ? P.cb : P.rb) + rr;
-                const bool ok = row < P.m;
-                const double* src = P.A + (int64_t)(ok ? row : P.rb) * P.ld + k0 + h * 32 + 2 * q2;
-                double* dst = (side ? sL[rr] : sW[rr]) + h * 32 + 2 * q2;
-                cp_async16(dst, src, ok);
-            }
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-        }
-    };
-    // the output tile, one commit group: rows or columns past m are zero-filled
-    auto issue_tile = [&](const UpdPair& P) {
-        for (int idx = tid; idx < kFb * 32; idx += kT) {
-            const int rr = idx >> 5, q2 = idx & 31;
-            const int row = P.rb + rr, col = P.cb + 2 * q2;
-            const bool ok = row < P.m && col < P.m;
-            const double* src = P.A + (ok ? (int64_t)row * P.ld + col : (int64_t)P.rb * P.ld + k0);
-            cp_async16(sC[rr] + 2 * q2, src, ok);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    UpdPair cur;
-    if (!next_pair(cur)) return;
-    issue_panels(cur);
-    issue_tile(cur);
-    if (tid < kFb) sD[tid] = dD[cur.r0 + k0 + tid];
-    // warp w: rows 16 (w >> 1) .. + 16 (two 8-row tiles), columns
-    // 32 (w & 1) .. + 32 (four 8-column tiles) of the 64 x 64 output
-    const int lane = tid & 31, warp = tid >> 5;
-    const int wr = (warp >> 1) * 16, wc = (warp & 1) * 32;
-    const int fr = lane >> 2, fk = lane & 3;
-    for (;;) {
-        // in flight: this pair's panel halves, then its output tile
-        double acc[2][4][2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 0)
-                asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-            else
-                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-            __syncthreads();
-#pragma unroll
-            for (int kq = h * 32; kq < h * 32 + 32; kq += 4) {
-                const double dk = sD[kq + fk];
-                double a[2], b[4];
-#pragma unroll
-                for (int i = 0; i < 2; ++i) a[i] = sW[wr + 8 * i + fr][kq + fk] * dk;  // A(8x4)[fr][fk]
-#pragma unroll
-                for (int j = 0; j < 4; ++j) b[j] = sL[wc + 8 * j + fr][kq + fk];  // B(4x8)[fk][fr]
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) dmma_m8n8k4(acc[i][j], a[i], b[j]);
-            }
-        }
-        __syncthreads();  // every warp is done with the panels and D
-        UpdPair nxt;
-        const bool more = next_pair(nxt);
-        if (more) {
-            issue_panels(nxt);
-            if (tid < kFb) sD[tid] = dD[nxt.r0 + k0 + tid];
-            asm volatile("cp.async.wait_group 2;\n" ::: "memory");  // this pair's tile; the next panels stay in flight
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        }
-        __syncthreads();  // the output tile is in shared memory
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int gr = cur.rb + wr + 8 * i + fr;
-            if (gr >= cur.m) continue;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const int gc = cur.cb + wc + 8 * j + 2 * fk + t;
-                    if (gc <= gr)
-                        cur.A[(int64_t)gr * cur.ld + gc] = sC[wr + 8 * i + fr][wc + 8 * j + 2 * fk + t] - acc[i][j][t];
-                }
-            }
-        }
-        if (!more) break;
-        __syncthreads();  // every warp is done reading the output tile
-        issue_tile(nxt);
-        cur = nxt;
-    }
-}
-
-// ---- batched triangular solves: N_i x = b in place, N_i = L_i D_i L_i^T ----
-// Level-synchronous in the factorisation's 64-row blocks and its schedule
-// (instances in decreasing size, panel rows in chunks of kT): per block,
-// forward: one launch solves every instance's unit-lower diagonal block,
-// one launch subtracts the block's contribution from the rows below (chunks
-// spread over the GPU, one warp per row, coalesced loads); then x /= D;
-// backward: one launch forms, per chunk, the column-block dot products of
-// L^T x over the rows below, one launch sums them in chunk order per
-// instance and solves the diagonal block. Every sum has a fixed order.
-// An instance takes part when it is iterating and, with a refine mask, still
-// refining.
-__device__ __forceinline__ bool solving(const int32_t* status, const int32_t* refine, int inst) {
-    return status[inst] == ST_RUN && (!refine || refine[inst]);
-}
-
-__device__ __forceinline__ int chunk_instance(const int64_t* chunks, int cnt, int64_t chunk) {
-    int lo = 0, hi = cnt - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (chunks[mid] <= chunk)
+        if (cum[mid] <= idx)
             lo = mid + 1;
         else
             hi = mid;
@@ -728,187 +655,679 @@ __device__ __forceinline__ int chunk_instance(const int64_t* chunks, int cnt, in
     return lo;
 }
 
-__global__ void __launch_bounds__(kFb) batch_fwd_diag_kernel(int s, const int64_t* __restrict__ row_off,
-                                                            const int64_t* __restrict__ dn_off,
-                                                            const int32_t* __restrict__ order,
-                                                            const int32_t* __restrict__ status,
-                                                            const int32_t* __restrict__ refine,
-                                                            const double* __restrict__ dense, double* __restrict__ xv) {
-    __shared__ double sL[kFb][kFbP];
-    __shared__ double sy[kFb];
-    const int inst = order[blockIdx.x];
-    if (!solving(status, refine, inst)) return;
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
-    const int k0 = s * kFb;
-    if (k0 >= m) return;
-    const int nb = min(kFb, m - k0);
-    const double* L = dense + dn_off[inst];
-    double* x = xv + r0;
-    const int i = threadIdx.x;
-    for (int idx = i; idx < kFb * kFb; idx += kFb) {
-        const int r = idx / kFb, c = idx % kFb;
-        sL[r][c] = (r < nb && c < r) ? L[(int64_t)(k0 + r) * ld + k0 + c] : 0.0;
-    }
-    sy[i] = i < nb ? x[k0 + i] : 0.0;
-    __syncthreads();
-    // warp 0 runs the substitution, rows lane and lane + 32, broadcasting
-    // each solved entry by a shuffle (no barriers); same operations per
-    // entry in the same order as a row-per-thread substitution
-    if (i >= 32) return;
-    double v0 = sy[i], v1 = sy[i + 32];
-    for (int j = 0; j < nb; ++j) {
-        const double yj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-        if (i > j && i < nb) v0 -= sL[i][j] * yj;
-        if (i + 32 > j && i + 32 < nb) v1 -= sL[i + 32][j] * yj;
-    }
-    if (i < nb) x[k0 + i] = v0;
-    if (i + 32 < nb) x[k0 + i + 32] = v1;
+// L[r, k0:k1] = A[r, k0:k1] (L_blk D)^-T for kPanelT rows of one instance's
+// panel, a row per thread (kT / kPanelT CTAs per chunk). A panel row exists
+// only below a full block, so all 64 columns are there. As soon as L[r, q] is
+// final it is taken from every later column, which leaves independent updates
+// in flight instead of one chain of subtractions per column; each element
+// sees the same products in the same order (q ascending). The columns go in
+// two halves of 32 registers through the same code (a loop over the first
+// half's columns, then the unrolled triangle): half the code of 64 unrolled
+// columns, which missed the instruction cache. What bounds it is the L1 data
+// path: 16 bytes of L to every lane per four FP64 instructions, and, while
+// each thread read and wrote its own row of memory, 32 sectors per access. The
+// rows now pass through shared memory (16-byte copies in, whole lines out)
+// except the second half's way in, which there is no room for at three CTAs
+// per SM. Two rows per thread halve the L loads but also the warps: 2,880
+// against 1,475 us over the 30 panels of 384 LPs of m 50-2000.
+// 384 LPs of m 50-2000 (30 panels): 1,209 us; 2,156 with a chain per column.
+constexpr int kPanelT = 128;
+constexpr int kPanelP = kFb + 2;  // even: 16-byte loads of two entries
+constexpr int kHalf = kFb / 2;
+constexpr int kRowP = kHalf + 2;  // staged rows: 16-byte accesses of eight lanes hit distinct banks
+constexpr size_t kPanelSmem = sizeof(double) * (kFb * kPanelP + 2 * kFb + kPanelT * kRowP);
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-__global__ void __launch_bounds__(kT) batch_fwd_gemv_kernel(int s, int cnt, const int64_t* __restrict__ chunks,
-                                                           const int64_t* __restrict__ row_off,
-                                                           const int64_t* __restrict__ dn_off,
-                                                           const int32_t* __restrict__ order,
-                                                           const int32_t* __restrict__ status,
-                                                           const int32_t* __restrict__ refine,
-                                                           const double* __restrict__ dense, double* __restrict__ xv) {
+__global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, const Chunk* __restrict__ chunks,
+                                                                      const InstInfo* __restrict__ info,
+                                                                      const int32_t* __restrict__ status, double* dense,
+                                                                      const double* __restrict__ dD) {
+    extern __shared__ __align__(16) double panel_sm[];
+    double(*sLt)[kPanelP] = reinterpret_cast<double(*)[kPanelP]>(panel_sm);  // sLt[q][c] = L[k0 + c, k0 + q]
+    double* sD = panel_sm + kFb * kPanelP;
+    double* sY = sD + kFb;  // 1 / D, zero where a quotient needs the division
+    double(*sRow)[kRowP] = reinterpret_cast<double(*)[kRowP]>(sY + kFb);  // half the columns of every row
+    const int tid = threadIdx.x;
+    const Chunk ch = chunks[blockIdx.x / (kT / kPanelT)];
+    if (status[ch.inst] != ST_RUN) return;
+    const InstInfo in = info[ch.inst];
+    const int ld = dense_ld(in.m);
+    const int k0 = s * kFb;
+    const int rb = k0 + kFb + ch.local * kT + static_cast<int>(blockIdx.x % (kT / kPanelT)) * kPanelT;
+    const int rows = min(kPanelT, in.m - rb);
+    if (rows <= 0) return;
+    double* A = dense + in.dn;
+    double* P = A + (int64_t)rb * ld + k0;  // the panel's rows
+    const int piece = tid & 15, line = tid >> 4;  // copies: 16 lanes a row
+#pragma unroll 4
+    for (int r = line; r < rows; r += kPanelT / 16) cp_async16(&sRow[r][2 * piece], P + (int64_t)r * ld + 2 * piece);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+#pragma unroll 8
+    for (int idx = tid; idx < kFb * kFb; idx += kPanelT) {
+        const int rr = idx / kFb, c = idx % kFb;
+        sLt[c][rr] = c < rr ? A[(int64_t)(k0 + rr) * ld + k0 + c] : 0.0;
+    }
+    if (tid < kFb) {
+        const double d = dD[in.r0 + k0 + tid];
+        sD[tid] = d;
+        sY[tid] = good_divisor(d) ? reciprocal(d) : 0.0;
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    double* mine = sRow[tid];
+    // whole lines of half h of the rows; called by all threads once the half is in sRow
+    auto store = [&](int h) {
+        __syncthreads();
+#pragma unroll 4
+        for (int r = line; r < rows; r += kPanelT / 16)
+            *reinterpret_cast<double2*>(P + (int64_t)r * ld + h * kHalf + 2 * piece) =
+                *reinterpret_cast<const double2*>(&sRow[r][2 * piece]);
+    };
+    double v[kHalf];
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const double* from = h == 0 ? mine : P + (int64_t)min(tid, rows - 1) * ld + kHalf;
+#pragma unroll
+        for (int c = 0; c < kHalf; c += 2) {
+            const double2 t = *reinterpret_cast<const double2*>(from + c);
+            v[c] = t.x;
+            v[c + 1] = t.y;
+        }
+        if (h == 1) {
+#pragma unroll 1
+            for (int q = 0; q < kHalf; q += 2) {
+                // L[r, q] D_q, rounded once as every column uses it
+                const double2 lq = *reinterpret_cast<const double2*>(mine + q);
+                const double w0 = lq.x * sD[q], w1 = lq.y * sD[q + 1];
+                const double *l0 = &sLt[q][kHalf], *l1 = &sLt[q + 1][kHalf];
+#pragma unroll
+                for (int c = 0; c < kHalf; c += 2) {
+                    const double2 t = *reinterpret_cast<const double2*>(l0 + c);
+                    const double2 u = *reinterpret_cast<const double2*>(l1 + c);
+                    v[c] -= w0 * t.x;
+                    v[c + 1] -= w0 * t.y;
+                    v[c] -= w1 * u.x;
+                    v[c + 1] -= w1 * u.y;
+                }
+            }
+        }
+        const double* sLh = &sLt[h * kHalf][h * kHalf];
+#pragma unroll
+        for (int q = 0; q < kHalf; ++q) {
+            const double d = sD[h * kHalf + q], y = sY[h * kHalf + q];
+            double l = quotient(v[q], d, y);
+            if (y == 0.0 || !(in_range(v[q]) || v[q] == 0.0)) l = v[q] / d;
+            const double w = l * d;
+            v[q] = l;
+            const int c0 = q + 1;
+            if ((c0 & 1) && c0 < kHalf) v[c0] -= w * sLh[q * kPanelP + c0];
+#pragma unroll
+            for (int c = c0 + (c0 & 1); c < kHalf; c += 2) {
+                const double2 t = *reinterpret_cast<const double2*>(sLh + q * kPanelP + c);
+                v[c] -= w * t.x;
+                v[c + 1] -= w * t.y;
+            }
+        }
+        if (h == 1) __syncthreads();  // the first half has left sRow
+#pragma unroll
+        for (int c = 0; c < kHalf; c += 2) *reinterpret_cast<double2*>(mine + c) = make_double2(v[c], v[c + 1]);
+        store(h);
+    }
+}
+
+// Trailing update by NP (1 or 2) neighbouring 64-column panels at once:
+// A[rows, cols] -= sum over the panels p of (L_p D_p) L_p^T, in 64 x 64 tiles
+// spread over persistent CTAs, two per SM (one multiplies while the other
+// changes tiles). Two panels per visit halve the reads and writes of the
+// trailing matrix, which is far larger than L2. A producer warp finds the
+// tiles (a chain of dependent loads) and copies the panels in slices of 16
+// columns into a ring of kUpdStages stages that runs on across tiles, and the
+// output tile with a slice of the first panel; 4 consumer warps multiply.
+// Everything is handed over with named barriers: no polling. How far the
+// producer is ahead decides the rate, so rows are packed and swizzled by
+// 16-byte pieces instead of padded, to fit a fifth stage; output tiles read
+// straight into registers at the tile's start held the products up. A consumer
+// warp owns 32 x 32 of the tile: per 4 columns 8 fragment loads feed 16 DMMAs.
+// D is applied at the fragment load (a = L[r, k] D_k rounds once). An
+// element's accumulator starts at zero for every panel and is subtracted after
+// it, so it goes through the same operations in the same order whatever the
+// grouping of the panels. Rows past m keep what the stage held before: they
+// only reach outputs past m.
+// 384 LPs of m 50-2000: 3,797 us (2,650 at the FP64 tensor rate of 37 TFLOP/s);
+// 5,641 with one panel per visit and one commit group ahead. Products alone
+// take 2,780 us of that, the copies alone 2,720.
+constexpr int kUpdN = kFb, kUpdK = 16;         // tile edge, columns of a slice
+constexpr int kUpdWarps = 4;                   // consumers
+constexpr int kUpdT = 32 * (kUpdWarps + 1);    // and the producer warp
+constexpr int kUpdStages = 5;
+constexpr int kUpdAhead = 3;                   // slices in flight when one is handed over
+constexpr int kUpdStage = 2 * kUpdN * kUpdK + kUpdK;  // doubles: A rows, B rows, D
+constexpr size_t kUpdSmem = sizeof(double) * (kUpdStages * kUpdStage + kUpdN * kUpdN);
+static_assert(2 * (kUpdSmem + 1280) <= 228 * 1024, "two update CTAs per SM");
+
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(kUpdT) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id) {
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(kUpdT) : "memory");
+}
+
+// 64 x 64 tiles of a trailing matrix of T block rows: its lower triangle, or its first block column.
+__host__ __device__ __forceinline__ int64_t update_tiles(int64_t T, bool column) {
+    return column ? T : T * (T + 1) / 2;
+}
+
+struct UpdTile {
+    double* A;  // the instance's dense block, null: no more tiles
+    int m, ld, rb, cb;
+};
+
+template <int NP>
+__global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int kt, int column, int cnt, int64_t ntiles,
+                                                                  const int64_t* __restrict__ tiles,
+                                                                  const InstInfo* __restrict__ info,
+                                                                  const int32_t* __restrict__ order,
+                                                                  const int32_t* __restrict__ status,
+                                                                  double* __restrict__ dense,
+                                                                  const double* __restrict__ dD) {
+    extern __shared__ __align__(16) double upd_smem[];
+    __shared__ UpdTile s_tile[kUpdStages];
+    double* sC = upd_smem + kUpdStages * kUpdStage;
+    constexpr int kPanel = kFb / kUpdK;  // slices of a panel
+    constexpr int kSlices = NP * kPanel;  // slices of a tile
+    constexpr int kFull = 1, kEmpty = 1 + kUpdStages, kOut = 1 + 2 * kUpdStages;  // named barriers: stages, output tile
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (warp == kUpdWarps) {
+        bool out_used = false;  // the consumers still have to release the output tile
+        int64_t n = 0;  // slices issued; slice i goes to stage i mod kUpdStages
+        for (int64_t idx = blockIdx.x; idx < ntiles; idx += gridDim.x) {
+            const int b = item_instance(tiles, cnt, idx);
+            const int inst = order[b];
+            if (status[inst] != ST_RUN) continue;
+            const int64_t local = idx - (b > 0 ? tiles[b - 1] : 0);
+            int I = static_cast<int>(local), J = 0;
+            if (!column) {
+                I = static_cast<int>((sqrt(8.0 * (double)local + 1.0) - 1.0) * 0.5);
+                while ((int64_t)(I + 1) * (I + 2) / 2 <= local) ++I;
+                while ((int64_t)I * (I + 1) / 2 > local) --I;
+                J = static_cast<int>(local - (int64_t)I * (I + 1) / 2);
+            }
+            const InstInfo in = info[inst];
+            UpdTile t;
+            t.m = in.m;
+            t.ld = dense_ld(t.m);
+            t.rb = kt + I * kUpdN;
+            t.cb = kt + J * kUpdN;
+            t.A = dense + in.dn;
+            // a lane copies 16-byte piece `lane mod 8` of every fourth row;
+            // piece c of row r lies at c ^ (r mod 8)
+            const int quad = lane >> 3, piece = lane & 7;
+            const int nA = min(kUpdN, t.m - t.rb), nB = min(kUpdN, t.m - t.cb);
+            const int64_t step = 4 * (int64_t)t.ld;
+            auto copy_rows = [&](double* dst, int row0, int n, int kc) {
+                const double* src = t.A + (int64_t)(row0 + quad) * t.ld + kc + 2 * piece;
+#pragma unroll 8
+                for (int r = quad; r < n; r += 4, src += step)
+                    cp_async16(dst + r * kUpdK + 2 * (piece ^ (r & 7)), src);
+            };
+            for (int h = 0; h < kSlices; ++h, ++n) {
+                const int st = static_cast<int>(n % kUpdStages);
+                if (n >= kUpdStages) named_sync(kEmpty + st);
+                double* base = upd_smem + st * kUpdStage;
+                const int kc = k0 + h * kUpdK;
+                copy_rows(base, t.rb, nA, kc);
+                copy_rows(base + kUpdN * kUpdK, t.cb, nB, kc);
+                if (lane < kUpdK) cp_async8(base + 2 * kUpdN * kUpdK + lane, dD + in.r0 + kc + lane);
+                if (h == kPanel - 1) {
+                    if (out_used) named_sync(kOut);
+                    out_used = true;
+                    // piece c of output row r lies at c ^ 4 (r mod 2)
+                    if (t.cb + 2 * lane < t.m) {
+                        const double* src = t.A + (int64_t)t.rb * t.ld + t.cb + 2 * lane;
+#pragma unroll 8
+                        for (int r = 0; r < nA; ++r, src += t.ld)
+                            cp_async16(sC + r * kUpdN + 2 * (lane ^ ((r & 1) << 2)), src);
+                    }
+                }
+                if (lane == 0) s_tile[st] = t;
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                if (n >= kUpdAhead) {  // slice n - kUpdAhead has arrived
+                    asm volatile("cp.async.wait_group %0;\n" ::"n"(kUpdAhead) : "memory");
+                    named_arrive(kFull + static_cast<int>((n - kUpdAhead) % kUpdStages));
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        for (int64_t i = n >= kUpdAhead ? n - kUpdAhead : 0; i < n; ++i) named_arrive(kFull + static_cast<int>(i % kUpdStages));
+        // the end mark, then every barrier the consumers still arrive at
+        const int st = static_cast<int>(n % kUpdStages);
+        if (n >= kUpdStages) named_sync(kEmpty + st);
+        if (lane == 0) s_tile[st].A = nullptr;
+        __syncwarp();
+        named_arrive(kFull + st);
+        for (int64_t i = n >= kUpdStages ? n - kUpdStages + 1 : 0; i < n; ++i)
+            named_sync(kEmpty + static_cast<int>(i % kUpdStages));
+        if (out_used) named_sync(kOut);
+        return;
+    }
+    const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
+    const int fr = lane >> 2, fk = lane & 3, sw = (fk >> 1) ^ fr;
+    int st = 0;
+    for (;;) {
+        named_sync(kFull + st);
+        const UpdTile t = s_tile[st];
+        if (!t.A) return;
+        // this lane's output elements: rows gr(i), column pairs gc(j), gc(j) + 1
+        double c[4][4][2];
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            double acc[4][4][2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll 1
+            for (int h = 0; h < kPanel; ++h) {
+                if (p + h > 0) named_sync(kFull + st);
+                const double* sA = upd_smem + st * kUpdStage + (wr + fr) * kUpdK;
+                const double* sB = upd_smem + st * kUpdStage + (kUpdN + wc + fr) * kUpdK;
+                const double* sD = upd_smem + st * kUpdStage + 2 * kUpdN * kUpdK + fk;
+#pragma unroll
+                for (int kq = 0; kq < kUpdK; kq += 4) {
+                    const int at = 2 * ((kq >> 1) ^ sw) + (fk & 1);  // column kq + fk of a row = fr mod 8
+                    const double dk = sD[kq];
+                    double a[4], b[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) a[i] = sA[8 * i * kUpdK + at] * dk;  // A(8x4)[fr][fk]
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) b[j] = sB[8 * j * kUpdK + at];  // B(4x8)[fk][fr]
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) dmma_m8n8k4(acc[i][j], a[i], b[j]);
+                }
+                named_arrive(kEmpty + st);
+                st = (st + 1) % kUpdStages;
+            }
+            const double* o = sC + (wr + fr) * kUpdN + wc + 2 * fk;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (p == 0) {
+                        const double2 v = *reinterpret_cast<const double2*>(o + 8 * i * kUpdN + 8 * (j ^ (fr & 1)));
+                        c[i][j][0] = v.x;
+                        c[i][j][1] = v.y;
+                    }
+                    c[i][j][0] -= acc[i][j][0];
+                    c[i][j][1] -= acc[i][j][1];
+                }
+            if (p == 0) named_arrive(kOut);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int gr = t.rb + wr + 8 * i + fr;
+            if (gr >= t.m) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int gc = t.cb + wc + 8 * j + 2 * fk;
+                double* o = t.A + (int64_t)gr * t.ld + gc;
+                if (gc < gr)
+                    *reinterpret_cast<double2*>(o) = make_double2(c[i][j][0], c[i][j][1]);
+                else if (gc == gr)
+                    *o = c[i][j][0];
+            }
+        }
+    }
+}
+
+// ---- batched triangular solves: N_i x = b in place, N_i = L_i D_i L_i^T ----
+// One launch per solve. An instance belongs to one CTA, which then keeps its
+// vector in shared memory, or to 2, 4 or 8 CTAs of a cluster; the CTAs walk
+// its 64-row blocks together, forward and then backward, one cluster barrier
+// per block. (A launch per block and direction spent 8 us and more each on
+// starting, finding its place and draining, for microseconds of products.)
+//   forward : every CTA solves the unit-lower diagonal block itself (64 steps
+//     of one warp) and takes the block's contribution from its chunks' right-
+//     hand sides, in place; the first CTA keeps the block of y / D in `work`.
+//   backward: every CTA forms its chunks' column-block dot products of L^T x;
+//     after the barrier the first CTA sums them in chunk order and solves the
+//     diagonal block while the others go on to the next block's products.
+//     (Only the first chunk of the next block touches the solution it writes,
+//     and that chunk is the first CTA's; the others reach it blocks later.)
+// Rows below a block come in chunks of kT, chunk c to CTA c mod the group's
+// size. L does not depend on x, so each warp's next 16 rows and the next
+// diagonal block load ahead of the barriers. Every sum has a fixed order
+// whatever the group size: a row's forward sum is a butterfly over the lanes;
+// a backward sum runs over a warp's rows (every eighth of the chunk), then
+// the warps, then the chunks.
+// An instance takes part when it is iterating and, with a refine mask, still
+// refining.
+// 384 LPs of m 50-2000, both solves of an iteration: 1,139 us; 3,853 with a
+// launch per block (the factors alone are 3 GB of reads, 470 us).
+__device__ __forceinline__ bool solving(const int32_t* status, const int32_t* refine, int inst) {
+    return status[inst] == ST_RUN && (!refine || refine[inst]);
+}
+
+constexpr int kSolveCluster = 8;
+constexpr int kSolveRows = 16;                      // rows of L a warp has in flight
+constexpr int kSolveBatches = kT / 8 / kSolveRows;  // such batches of a warp per chunk
+constexpr int kSolveP = kFb + 2;                    // smem row stride: 16-byte copies
+
+// One butterfly level over lane bit o of 2 R partial sums per lane: a lane
+// keeps the R sums of its half and adds its partner's, own + partner as the
+// one-sum butterfly adds them.
+template <int R>
+__device__ __forceinline__ void fold(double* p, int lane, int o) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const double keep = up ? p[u + R] : p[u], give = up ? p[u] : p[u + R];
+        p[u] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+}
+
+__device__ __forceinline__ double ld_l2(const double* p) {  // written by other CTAs: past L1
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ double ld_once(const double* p) {  // in program order, so that the batch stays in flight
+    double v;
+    asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+// The strictly lower part of the diagonal block at k0 (rows below m only), asynchronously.
+__device__ __forceinline__ void copy_diag_block(double (*sL)[kSolveP], const double* L, int ld, int k0, int nb) {
+#pragma unroll
+    for (int q = 0; q < kFb * kFb / 2 / kT; ++q) {
+        const int u = threadIdx.x + q * kT, r = u / (kFb / 2), c = 2 * (u % (kFb / 2));
+        if (r < nb && c < r) cp_async16(&sL[r][c], L + (int64_t)(k0 + r) * ld + k0 + c);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
+// y = L^-1 v of a unit-lower diagonal block by one warp, rows lane and lane + 32
+// (v0, v1), four columns per step: every lane solves the 4 x 4 corner itself
+// from four broadcasts. Unrolled in full, so that the loads of L run ahead of
+// the chain (3,130 cycles; 4,700 in a loop, 3,450 with a broadcast per column,
+// unrolled by 8). A row takes its columns in order. Rows past the block only
+// reach themselves and later ones.
+__device__ __forceinline__ void forward_block(const double (*sL)[kSolveP], double& v0, double& v1, int lane) {
+#pragma unroll
+    for (int j = 0; j < kFb; j += 4) {
+        double y[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y[q] = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, (j + q) & 31);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+            for (int e = q + 1; e < 4; ++e) y[e] -= sL[j + e][j + q] * y[q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (j < 32 && lane > j + q) v0 -= sL[lane][j + q] * y[q];
+            if (j < 32 || lane + 32 > j + q) v1 -= sL[lane + 32][j + q] * y[q];
+        }
+    }
+}
+
+// x = L^-T v likewise, columns descending from nb - 1.
+__device__ __forceinline__ void backward_block(const double (*sL)[kSolveP], double& v0, double& v1, int nb, int lane) {
+    if (nb < kFb) {  // the instance's last block: one column per step
+        for (int j = nb - 1; j >= 0; --j) {
+            const double xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
+            if (lane < j) v0 -= sL[j][lane] * xj;
+            if (lane + 32 < j) v1 -= sL[j][lane + 32] * xj;
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = kFb - 1; j >= 0; j -= 4) {
+        double y[4];  // entries j, j - 1, j - 2, j - 3
+#pragma unroll
+        for (int q = 0; q < 4; ++q) y[q] = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, (j - q) & 31);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+            for (int e = q + 1; e < 4; ++e) y[e] -= sL[j - q][j - e] * y[q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (j >= 32 || lane < j - q) v0 -= sL[j - q][lane] * y[q];
+            if (j >= 32 && lane + 32 < j - q) v1 -= sL[j - q][lane + 32] * y[q];
+        }
+    }
+}
+
+__global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
+    batch_solve_kernel(const SolveSlot* __restrict__ slots, const InstInfo* __restrict__ info,
+                       const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
+                       const double* __restrict__ dense, const double* __restrict__ dD, double* work, double* part,
+                       double* xv) {
+    extern __shared__ __align__(16) double solve_smem[];
+    double(*sLb)[kFb][kSolveP] = reinterpret_cast<double(*)[kFb][kSolveP]>(solve_smem);  // two diagonal blocks
+    double* s_x = solve_smem + 2 * kFb * kSolveP;  // a single CTA's instance: right-hand side, y / D, solution
+    __shared__ double sacc[kT / 32][kFb];
     __shared__ double sx[kFb];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = chunk_instance(chunks, cnt, blockIdx.x);
-    const int inst = order[b];
-    if (!solving(status, refine, inst)) return;
-    const int64_t local = blockIdx.x - (b > 0 ? chunks[b - 1] : 0);
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
-    const int k0 = s * kFb;
-    const int nb = min(kFb, m - k0), k1 = k0 + nb;
-    const double* L = dense + dn_off[inst];
-    double* x = xv + r0;
-    if (tid < kFb) sx[tid] = tid < nb ? x[k0 + tid] : 0.0;
-    __syncthreads();
-    const int rb = k1 + static_cast<int>(local) * kT, re = min(m, rb + kT);
-    for (int rw = rb + warp * 4; rw < re; rw += (kT / 32) * 4) {
-        double p[4];
+    const SolveSlot slot = slots[blockIdx.x];
+    const bool on = slot.inst >= 0 && solving(status, refine, slot.inst);
+    InstInfo in = {0, 0, 0, {0, 0, 0}};
+    if (on) in = info[slot.inst];
+    const int m = in.m, ld = dense_ld(m);
+    const double* L = dense + in.dn;
+    double* x = xv + in.r0;
+    double* y = work + in.r0;
+    const double* D = dD + in.r0;
+    const int nblk = (m + kFb - 1) / kFb;
+    const bool alone = slot.size == 1;
+    const int steps = slot.steps > 0 ? slot.steps : nblk;
+    if (alone)
+        for (int i = tid; i < m; i += kT) s_x[i] = x[i];
+    auto barrier = [&]() {
+        if (slot.steps > 0) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    };
+    double p0[kSolveRows], p1[kSolveRows];
+
+    // ---- forward ----
+    // batch h of this warp's rows in chunk c below the block at k0: rows first, first + 1, ...
+    auto fwd_row = [&](int k0, int c, int h) { return k0 + kFb + c * kT + warp * (kT / 8) + h * kSolveRows; };
+    auto fwd_load = [&](int k0, int c, int h) {
+        const int r = fwd_row(k0, c, h);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int r = rw + u;
-            double a = 0.0;
-            if (r < re) {
-                const double* Lr = L + (int64_t)r * ld + k0;
-                const double p0 = lane < nb ? Lr[lane] * sx[lane] : 0.0;
-                const double p1 = lane + 32 < nb ? Lr[lane + 32] * sx[lane + 32] : 0.0;
-                a = p0 + p1;
+        for (int u = 0; u < kSolveRows; ++u) {
+            p0[u] = p1[u] = 0.0;
+            if (r + u < m) {
+                const double* Lr = L + (int64_t)(r + u) * ld + k0;
+                p0[u] = ld_once(Lr + lane);
+                p1[u] = ld_once(Lr + lane + 32);
             }
-            p[u] = a;
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) p[u] += __shfl_xor_sync(0xffffffffu, p[u], o);
-        }
-        if (lane < 4 && rw + lane < re) {
-            const double t = lane == 0 ? p[0] : lane == 1 ? p[1] : lane == 2 ? p[2] : p[3];
-            x[rw + lane] -= t;
-        }
+    };
+    if (nblk > 0) {
+        copy_diag_block(sLb[0], L, ld, 0, min(kFb, m));
+        fwd_load(0, slot.rank, 0);
     }
-}
-
-__global__ void batch_scale_kernel(int64_t m, const int32_t* __restrict__ row_inst,
-                                   const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
-                                   const double* __restrict__ dD, double* __restrict__ x) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= m) return;
-    if (solving(status, refine, row_inst[k])) x[k] /= dD[k];
-}
-
-// part[chunk][q] = sum over the chunk's rows c (in order, per warp, then the
-// warps in order) of L[c][k0 + q] x[c]
-__global__ void __launch_bounds__(kT) batch_bwd_gemv_kernel(int s, int cnt, const int64_t* __restrict__ chunks,
-                                                           const int64_t* __restrict__ row_off,
-                                                           const int64_t* __restrict__ dn_off,
-                                                           const int32_t* __restrict__ order,
-                                                           const int32_t* __restrict__ status,
-                                                           const int32_t* __restrict__ refine,
-                                                           const double* __restrict__ dense,
-                                                           const double* __restrict__ xv, double* __restrict__ part) {
-    __shared__ double sacc[kT / 32][kFb];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int b = chunk_instance(chunks, cnt, blockIdx.x);
-    const int inst = order[b];
-    if (!solving(status, refine, inst)) return;
-    const int64_t local = blockIdx.x - (b > 0 ? chunks[b - 1] : 0);
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
-    const int k0 = s * kFb;
-    const int nb = min(kFb, m - k0), k1 = k0 + nb;
-    const double* L = dense + dn_off[inst];
-    const double* x = xv + r0;
-    const int rb = k1 + static_cast<int>(local) * kT, re = min(m, rb + kT);
-    double a0 = 0.0, a1 = 0.0;
-    for (int c = rb + warp; c < re; c += kT / 32) {
-        const double* Lc = L + (int64_t)c * ld + k0;
-        const double xc = x[c];
-        if (lane < nb) a0 += Lc[lane] * xc;
-        if (lane + 32 < nb) a1 += Lc[lane + 32] * xc;
+    for (int s = 0; s < steps; ++s) {
+        if (s < nblk) {
+            const int k0 = s * kFb, nb = min(kFb, m - k0);
+            const auto sL = sLb[s & 1];
+            // the other buffer was last read a barrier ago
+            if (s + 1 < nblk)
+                copy_diag_block(sLb[(s + 1) & 1], L, ld, k0 + kFb, min(kFb, m - k0 - kFb));
+            else
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+            // a lane's share of each row batch: row first + mine
+            const int mine = (lane >> 1);
+            double xr = 0.0;
+            if (!alone) {
+                const int r = fwd_row(k0, slot.rank, 0) + mine;
+                if (r < m) xr = ld_l2(x + r);
+                if (tid < kFb) sx[tid] = tid < nb ? ld_l2(x + k0 + tid) : 0.0;
+            }
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            __syncthreads();
+            if (warp == 0) {
+                double v0, v1;
+                if (alone) {
+                    v0 = lane < nb ? s_x[k0 + lane] : 0.0;
+                    v1 = lane + 32 < nb ? s_x[k0 + lane + 32] : 0.0;
+                } else {
+                    v0 = sx[lane];
+                    v1 = sx[lane + 32];
+                }
+                forward_block(sL, v0, v1, lane);
+                sx[lane] = v0;
+                sx[lane + 32] = v1;
+                if (slot.rank == 0) {
+                    double* o = alone ? s_x : y;
+                    if (lane < nb) o[k0 + lane] = v0 / D[k0 + lane];
+                    if (lane + 32 < nb) o[k0 + lane + 32] = v1 / D[k0 + lane + 32];
+                }
+            }
+            __syncthreads();
+            const double x0 = sx[lane], x1 = sx[lane + 32];
+            for (int c = slot.rank; k0 + kFb + c * kT < m; c += slot.size) {
+#pragma unroll 1
+                for (int h = 0; h < kSolveBatches; ++h) {
+                    double p[kSolveRows];
+#pragma unroll
+                    for (int u = 0; u < kSolveRows; ++u) p[u] = p0[u] * x0 + p1[u] * x1;
+                    const int row = fwd_row(k0, c, h) + mine;
+                    const double old = alone ? (row < m ? s_x[row] : 0.0) : xr;
+                    int nc = c, nh = h + 1;
+                    if (nh == kSolveBatches) {
+                        nc = c + slot.size;
+                        nh = 0;
+                    }
+                    if (k0 + kFb + nc * kT < m) {
+                        fwd_load(k0, nc, nh);
+                        const int r = fwd_row(k0, nc, nh) + mine;
+                        if (!alone && r < m) xr = ld_l2(x + r);
+                    } else {
+                        fwd_load(k0 + kFb, slot.rank, 0);
+                    }
+                    fold<8>(p, lane, 16);
+                    fold<4>(p, lane, 8);
+                    fold<2>(p, lane, 4);
+                    fold<1>(p, lane, 2);
+                    double t = p[0];
+                    t = t + __shfl_xor_sync(0xffffffffu, t, 1);
+                    if (!(lane & 1) && row < m) (alone ? s_x : x)[row] = old - t;
+                }
+            }
+        }
+        barrier();
     }
-    sacc[warp][lane] = a0;
-    sacc[warp][lane + 32] = a1;
-    __syncthreads();
-    if (tid < kFb) {
+
+    // ---- backward ----
+    // batch h of this warp's rows in chunk c below the block at k0: rows first, first + 8, ...
+    auto bwd_row = [&](int k0, int c, int h) { return k0 + kFb + c * kT + warp + h * kSolveRows * (kT / 32); };
+    auto bwd_load = [&](int k0, int c, int h) {
+        const int r = bwd_row(k0, c, h);
+#pragma unroll
+        for (int u = 0; u < kSolveRows; ++u) {
+            p0[u] = p1[u] = 0.0;
+            if (r + u * (kT / 32) < m) {
+                const double* Lr = L + (int64_t)(r + u * (kT / 32)) * ld + k0;
+                p0[u] = ld_once(Lr + lane);
+                p1[u] = ld_once(Lr + lane + 32);
+            }
+        }
+    };
+    // this instance's partial sums: chunk c of an even (odd) block at part_i + 64 c (+ half)
+    const int64_t half = 64 * (int64_t)((m + kT - 1) / kT);
+    double* part_i = part + 2 * 64 * (in.r0 / kT + (slot.inst >= 0 ? slot.inst : 0));
+    int s = nblk - 1;
+    if (s >= 0) {
+        if (slot.rank == 0) copy_diag_block(sLb[s & 1], L, ld, s * kFb, m - s * kFb);
+        bwd_load(s * kFb, slot.rank, 0);
+    }
+    for (int i = 0; i < steps; ++i, --s) {
+        double* ps = part_i + (s & 1) * half;
+        const int k0 = s * kFb;
+        const auto sL = sLb[s & 1];
+        if (slot.rank == 0) {  // as forward; only the first CTA solves
+            if (s > 0)
+                copy_diag_block(sLb[(s - 1) & 1], L, ld, k0 - kFb, kFb);
+            else
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+        }
+        const int nch = s >= 0 ? (max(0, m - k0 - kFb) + kT - 1) / kT : 0;
         double t = 0.0;
-        for (int w = 0; w < kT / 32; ++w) t += sacc[w][tid];
-        part[blockIdx.x * (int64_t)kFb + tid] = t;
+        for (int c = slot.rank; c < nch; c += slot.size) {
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll 1
+            for (int h = 0; h < kSolveBatches; ++h) {
+                const int r = bwd_row(k0, c, h);
+                double xc[kSolveRows];
+#pragma unroll
+                for (int u = 0; u < kSolveRows; ++u) {
+                    const int row = r + u * (kT / 32);
+                    xc[u] = 0.0;
+                    if (row < m) xc[u] = alone ? s_x[row] : ld_l2(x + row);
+                }
+#pragma unroll
+                for (int u = 0; u < kSolveRows; ++u) {
+                    const bool row = r + u * (kT / 32) < m;
+                    const double t0 = a0 + p0[u] * xc[u], t1 = a1 + p1[u] * xc[u];
+                    a0 = row ? t0 : a0;
+                    a1 = row ? t1 : a1;
+                }
+                if (h + 1 < kSolveBatches)
+                    bwd_load(k0, c, h + 1);
+                else if (c + slot.size < nch)
+                    bwd_load(k0, c + slot.size, 0);
+                else if (s > 0)
+                    bwd_load(k0 - kFb, slot.rank, 0);
+            }
+            sacc[warp][lane] = a0;
+            sacc[warp][lane + 32] = a1;
+            __syncthreads();
+            if (tid < kFb) {
+                t = 0.0;
+                for (int w = 0; w < kT / 32; ++w) t += sacc[w][tid];
+                if (nch > 1) ps[64 * c + tid] = t;  // read back by this thread, or past the barrier
+            }
+            __syncthreads();
+        }
+        if (slot.rank >= nch && s > 0) bwd_load(k0 - kFb, slot.rank, 0);  // no chunk here, maybe at the next block
+        barrier();
+        if (s >= 0 && slot.rank == 0) {
+            const int nb = min(kFb, m - k0);
+            if (tid < kFb) {
+                if (nch > 1) {
+                    t = 0.0;
+                    for (int c = 0; c < nch; ++c) t += ld_l2(ps + 64 * c + tid);
+                }
+                sx[tid] = tid < nb ? (alone ? s_x[k0 + tid] : y[k0 + tid]) - t : 0.0;
+            }
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            __syncthreads();
+            if (warp == 0) {
+                double v0 = sx[lane], v1 = sx[lane + 32];
+                backward_block(sL, v0, v1, nb, lane);
+                double* o = alone ? s_x : x;
+                if (lane < nb) o[k0 + lane] = v0;
+                if (lane + 32 < nb) o[k0 + lane + 32] = v1;
+            }
+            __syncthreads();
+        }
     }
-}
-
-__global__ void __launch_bounds__(kFb) batch_bwd_diag_kernel(int s, const int64_t* __restrict__ chunks,
-                                                            const int64_t* __restrict__ row_off,
-                                                            const int64_t* __restrict__ dn_off,
-                                                            const int32_t* __restrict__ order,
-                                                            const int32_t* __restrict__ status,
-                                                            const int32_t* __restrict__ refine,
-                                                            const double* __restrict__ dense,
-                                                            const double* __restrict__ part,
-                                                            double* __restrict__ xv) {
-    __shared__ double sL[kFb][kFbP];
-    __shared__ double sxj[kFb];
-    const int b = blockIdx.x;
-    const int inst = order[b];
-    if (!solving(status, refine, inst)) return;
-    const int64_t r0 = row_off[inst];
-    const int m = static_cast<int>(row_off[inst + 1] - r0);
-    const int ld = dense_ld(m);
-    const int k0 = s * kFb;
-    if (k0 >= m) return;
-    const int nb = min(kFb, m - k0);
-    const double* L = dense + dn_off[inst];
-    double* x = xv + r0;
-    const int q = threadIdx.x;
-    for (int idx = q; idx < kFb * kFb; idx += kFb) {
-        const int r = idx / kFb, c = idx % kFb;
-        sL[r][c] = (r < nb && c < r) ? L[(int64_t)(k0 + r) * ld + k0 + c] : 0.0;
-    }
-    const int64_t c0 = b > 0 ? chunks[b - 1] : 0, c1 = chunks[b];
-    double t = 0.0;
-    if (q < nb)
-        for (int64_t ch = c0; ch < c1; ++ch) t += part[ch * kFb + q];
-    sxj[q] = q < nb ? x[k0 + q] - t : 0.0;
-    __syncthreads();
-    // warp 0 runs the back substitution over rows lane and lane + 32 with
-    // shuffle broadcasts (no barriers), operations as row-per-thread
-    if (q >= 32) return;
-    double v0 = sxj[q], v1 = sxj[q + 32];
-    for (int j = nb - 1; j >= 0; --j) {
-        const double xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-        if (q < j) v0 -= sL[j][q] * xj;
-        if (q + 32 < j) v1 -= sL[j][q + 32] * xj;
-    }
-    if (q < nb) x[k0 + q] = v0;
-    if (q + 32 < nb) x[k0 + q + 32] = v1;
+    if (alone)
+        for (int i = tid; i < m; i += kT) x[i] = s_x[i];  // past the last block's barrier
 }
 
 // Refinement bookkeeping per instance (refinement.cpp:15-30): with r = rhs - N x,
@@ -984,8 +1403,8 @@ void free_batch(hn_batch* B) {
     for (void* p : {(void*)B->row_off, (void*)B->col_off, (void*)B->row_inst, (void*)B->dn_off, (void*)B->order,
                     (void*)B->dense, (void*)B->dD, (void*)B->refine, (void*)B->nref, (void*)B->nrp,
                     (void*)B->tile_row, (void*)B->tile_nz, (void*)B->carry_row, (void*)B->head_row,
-                    (void*)B->carry_val, (void*)B->head_val, (void*)B->r, (void*)B->ax, (void*)B->step_pairs, (void*)B->step_chunks,
-                    (void*)B->solve_part, (void*)B->kkt, (void*)B->kkt_ref, (void*)B->ref_iter, (void*)B->xb,
+                    (void*)B->carry_val, (void*)B->head_val, (void*)B->r, (void*)B->ax, (void*)B->step_tiles, (void*)B->chunks,
+                    (void*)B->info, (void*)B->slots, (void*)B->work, (void*)B->solve_part, (void*)B->kkt, (void*)B->kkt_ref, (void*)B->ref_iter, (void*)B->xb,
                     (void*)B->zb, (void*)B->lb})
         dfree(p);
     delete B;
@@ -1001,34 +1420,11 @@ SpmvMat n_mat(const hn_batch* B, const double* nval) {
                    B->carry_val, B->head_row, B->head_val, B->ntiles};
 }
 
+// x holds the right-hand sides of the taking-part instances on entry, their solutions on return.
 void solve_all(hn_batch* B, const int32_t* status, const int32_t* refine, double* x, cudaStream_t s) {
-    for (int64_t st = 0; st < B->nsteps; ++st) {
-        const int cnt = B->step_cnt[st];
-        batch_fwd_diag_kernel<<<cnt, kFb, 0, s>>>((int)st, B->row_off, B->dn_off, B->order, status, refine, B->dense, x);
-        launched("batch_fwd_diag_kernel");
-        const int64_t nc = B->step_chunks_h[st];
-        if (nc > 0) {
-            batch_fwd_gemv_kernel<<<(unsigned)nc, kT, 0, s>>>((int)st, cnt, B->step_chunks + B->chunk_off_h[st],
-                                                              B->row_off, B->dn_off, B->order, status, refine,
-                                                              B->dense, x);
-            launched("batch_fwd_gemv_kernel");
-        }
-    }
-    batch_scale_kernel<<<(unsigned)((B->m + 255) / 256), 256, 0, s>>>(B->m, B->row_inst, status, refine, B->dD, x);
-    launched("batch_scale_kernel");
-    for (int64_t st = B->nsteps - 1; st >= 0; --st) {
-        const int cnt = B->step_cnt[st];
-        const int64_t nc = B->step_chunks_h[st];
-        const int64_t* ch = B->step_chunks + B->chunk_off_h[st];
-        if (nc > 0) {
-            batch_bwd_gemv_kernel<<<(unsigned)nc, kT, 0, s>>>((int)st, cnt, ch, B->row_off, B->dn_off, B->order,
-                                                              status, refine, B->dense, x, B->solve_part);
-            launched("batch_bwd_gemv_kernel");
-        }
-        batch_bwd_diag_kernel<<<cnt, kFb, 0, s>>>((int)st, ch, B->row_off, B->dn_off, B->order, status, refine,
-                                                  B->dense, B->solve_part, x);
-        launched("batch_bwd_diag_kernel");
-    }
+    batch_solve_kernel<<<(unsigned)B->nslots, kT, (size_t)B->solve_smem, s>>>(B->slots, B->info, status, refine, B->dense,
+                                                          B->dD, B->work, B->solve_part, x);
+    launched("batch_solve_kernel");
 }
 
 }  // namespace
@@ -1077,12 +1473,14 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             B->r = dmalloc<double>(m);
             B->ax = dmalloc<double>(m);
             B->nrp = dmalloc<int32_t>(m + 1);
-            check_cuda(cudaFuncSetAttribute(batch_ldlt_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kUpdSmem),
-                       "update smem attribute");
-            check_cuda(cudaFuncSetAttribute(batch_ldlt_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            B->work = dmalloc<double>(m);
+            B->solve_part = dmalloc<double>(2 * kFb * (m / kT + K + 1));
+            check_cuda(cudaFuncSetAttribute(batch_ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)kPanelSmem),
-                       "diagonal-block smem attribute");
+                       "panel smem attribute");
+            for (auto* k : {batch_ldlt_update_kernel<1>, batch_ldlt_update_kernel<2>})
+                check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdSmem),
+                           "update smem attribute");
             B->ref_iter = dmalloc<int32_t>(K);
             B->kkt = dmalloc<double>(4 * K);
             B->kkt_ref = dmalloc<double>(4 * K);
@@ -1103,39 +1501,78 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             // at step s form a prefix of `order`)
             const int64_t mmax = row_off_host[order[0] + 1] - row_off_host[order[0]];
             B->nsteps = (mmax + kFb - 1) / kFb;
-            B->pair_off_h.assign(1, 0);
+            B->tile_off_h.assign(1, 0);
             B->chunk_off_h.assign(1, 0);
-            std::vector<int64_t> flat, cflat;
+            std::vector<int64_t> tiles;
+            std::vector<Chunk> chunks;
             for (int64_t st = 0; st < B->nsteps; ++st) {
                 int32_t cnt = 0;
-                int64_t acc = 0, cacc = 0;
+                int64_t acc = 0;
                 for (int64_t b = 0; b < K; ++b) {
                     const int64_t mi = row_off_host[order[b] + 1] - row_off_host[order[b]];
                     if (mi <= st * kFb) break;
                     const int64_t rest = mi - std::min<int64_t>(mi, (st + 1) * kFb);
-                    const int64_t T = (rest + kFb - 1) / kFb;
-                    acc += T * (T + 1) / 2;
-                    flat.push_back(acc);
-                    cacc += (rest + kT - 1) / kT;
-                    cflat.push_back(cacc);
+                    acc += update_tiles((rest + kFb - 1) / kFb, st % 2 == 0);
+                    tiles.push_back(acc);
+                    for (int32_t c = 0; c * kT < rest; ++c) chunks.push_back(Chunk{order[b], c});
                     ++cnt;
                 }
                 B->step_cnt.push_back(cnt);
-                B->step_pairs_h.push_back(acc);
-                B->pair_off_h.push_back((int64_t)flat.size());
-                B->step_chunks_h.push_back(cacc);
-                B->chunk_off_h.push_back((int64_t)cflat.size());
+                B->step_tiles_h.push_back(acc);
+                B->tile_off_h.push_back((int64_t)tiles.size());
+                B->chunk_off_h.push_back((int64_t)chunks.size());
             }
-            B->step_pairs = dmalloc<int64_t>(flat.size());
-            B->step_chunks = dmalloc<int64_t>(cflat.size());
-            int64_t maxc = 1;
-            for (int64_t c : B->step_chunks_h) maxc = std::max(maxc, c);
-            B->solve_part = dmalloc<double>(maxc * kFb);
-            check_cuda(cudaMemcpy(B->step_chunks, cflat.data(), sizeof(int64_t) * cflat.size(),
-                                  cudaMemcpyHostToDevice),
-                       "H2D chunks");
-            check_cuda(cudaMemcpy(B->step_pairs, flat.data(), sizeof(int64_t) * flat.size(), cudaMemcpyHostToDevice),
-                       "H2D schedule");
+            // the solve's clusters, largest instances first. An instance gets
+            // the CTAs that leave each of them at most `per` chunks of rows
+            // below the first block, per as small as keeps the batch within
+            // five CTAs per SM: few instances are split for latency, many
+            // run side by side (one solve of 384 LPs of m 50-2000: per = 1, 2,
+            // 4, 8 give 864, 568, 727, 951 us)
+            auto group = [](int64_t mi, int64_t per) {
+                const int64_t ch = (std::max<int64_t>(mi - kFb, 0) + kT - 1) / kT;
+                int g = 1;
+                while (g < kSolveCluster && ch > per * g) g *= 2;
+                return g;
+            };
+            int64_t per = 1;
+            for (;; per *= 2) {
+                int64_t total = 0;
+                for (int64_t i = 0; i < K; ++i) total += group(row_off_host[i + 1] - row_off_host[i], per);
+                if (per == 8 || total <= 5 * (int64_t)ctx().sm_count) break;
+            }
+            std::vector<InstInfo> info(K);
+            std::vector<SolveSlot> slots;
+            int64_t alone_m = 1;
+            for (int64_t b = 0; b < K; ++b) {
+                const int32_t i = order[b];
+                const int64_t mi = row_off_host[i + 1] - row_off_host[i];
+                info[i] = InstInfo{row_off_host[i], dn[i], (int32_t)mi, {0, 0, 0}};
+                const int size = group(mi, per);
+                if (size == 1) alone_m = std::max(alone_m, mi);
+                if (!slots.empty() && slots.back().size != size)
+                    while (slots.size() % kSolveCluster)
+                        slots.push_back(SolveSlot{-1, 0, 1, slots.back().steps});
+                const int32_t steps = size == 1 ? 0
+                                      : slots.size() % kSolveCluster ? slots.back().steps
+                                                                     : (int32_t)((mi + kFb - 1) / kFb);
+                for (int32_t r = 0; r < size; ++r) slots.push_back(SolveSlot{i, r, size, steps});
+            }
+            while (slots.size() % kSolveCluster) slots.push_back(SolveSlot{-1, 0, 1, slots.back().steps});
+            B->nslots = (int64_t)slots.size();
+            B->solve_smem = sizeof(double) * (2 * kFb * kSolveP + alone_m);  // alone_m <= 8 kT + kFb
+            check_cuda(cudaFuncSetAttribute(batch_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(double) * (2 * kFb * kSolveP + 8 * kT + kFb)),
+                       "solve smem attribute");
+            auto upload = [&](auto*& dst, const auto& src) {
+                using T = std::remove_reference_t<decltype(*dst)>;
+                dst = dmalloc<T>(src.size());
+                if (!src.empty())
+                    check_cuda(cudaMemcpy(dst, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice), "H2D schedule");
+            };
+            upload(B->step_tiles, tiles);
+            upload(B->chunks, chunks);
+            upload(B->info, info);
+            upload(B->slots, slots);
             check_cuda(cudaStreamSynchronize(s), "batch create sync");
         } catch (...) {
             free_batch(B);
@@ -1229,26 +1666,28 @@ int hn_batch_factor(hn_batch* B, const double* D, double reg, double singular_to
         batch_dense_kernel<<<(unsigned)((B->m * 32 + 255) / 256), 256, 0, s>>>(
             B->m, B->row_off, B->row_inst, B->dn_off, status, B->P->rp, B->P->ci, nval, B->dense);
         launched("batch_dense_kernel");
+        // steps in pairs: after an even step only the next block column is
+        // brought up to date, after an odd one the rest, by both panels at once
         for (int64_t st = 0; st < B->nsteps; ++st) {
             const int cnt = B->step_cnt[st];
-            batch_ldlt_diag_kernel<<<cnt, kT, kPanelSmem, s>>>((int)st, B->row_off, B->dn_off, B->order, status,
-                                                               B->dense, B->dD, singular_tol);
+            batch_ldlt_diag_kernel<<<cnt, kT, 0, s>>>((int)st, B->info, B->order, status, B->dense, B->dD, singular_tol);
             launched("batch_ldlt_diag_kernel");
-            const int64_t nc = B->step_chunks_h[st];
-            if (nc > 0) {
-                batch_ldlt_panel_kernel<<<(unsigned)nc, kT, 0, s>>>((int)st, cnt, B->step_chunks + B->chunk_off_h[st],
-                                                                    B->row_off, B->dn_off, B->order, status,
-                                                                    B->dense, B->dD);
-                launched("batch_ldlt_panel_kernel");
-            }
-            const int64_t np = B->step_pairs_h[st];
-            if (np > 0) {
-                const int grid = (int)std::min<int64_t>(np, (int64_t)ctx().sm_count * 2);
-                batch_ldlt_update_kernel<<<grid, kT, kUpdSmem, s>>>((int)st, cnt, np, B->step_pairs + B->pair_off_h[st],
-                                                             B->row_off, B->dn_off, B->order, status, B->dense,
-                                                             B->dD);
-                launched("batch_ldlt_update_kernel");
-            }
+            const int64_t nc = B->chunk_off_h[st + 1] - B->chunk_off_h[st];
+            if (nc == 0) continue;
+            batch_ldlt_panel_kernel<<<(unsigned)(nc * (kT / kPanelT)), kPanelT, kPanelSmem, s>>>(
+                (int)st, B->chunks + B->chunk_off_h[st], B->info, status, B->dense, B->dD);
+            launched("batch_ldlt_panel_kernel");
+            const int64_t nt = B->step_tiles_h[st];
+            const unsigned grid = (unsigned)std::min<int64_t>(nt, 2 * (int64_t)ctx().sm_count);
+            const int kt = (int)(st + 1) * kFb;
+            const int64_t* tiles = B->step_tiles + B->tile_off_h[st];
+            if (st % 2 == 0)
+                batch_ldlt_update_kernel<1><<<grid, kUpdT, kUpdSmem, s>>>(kt - kFb, kt, 1, cnt, nt, tiles, B->info,
+                                                                          B->order, status, B->dense, B->dD);
+            else
+                batch_ldlt_update_kernel<2><<<grid, kUpdT, kUpdSmem, s>>>(kt - 2 * kFb, kt, 0, cnt, nt, tiles, B->info,
+                                                                          B->order, status, B->dense, B->dD);
+            launched("batch_ldlt_update_kernel");
         }
     });
 }

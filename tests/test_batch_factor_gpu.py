@@ -1,0 +1,87 @@
+"""GPU: hn_batch_factor + hn_batch_solve against numpy on each instance's N.
+
+Sizes sit on the edges of the kernels' blocks: 64-column steps and their
+pairs, 128-row panel parts, 256-row chunks, and the row counts at which an
+instance's solve goes from one CTA to two, four and eight. Values far outside
+2^-400 .. 2^400 take the factorisation's dividing path.
+
+Bar: forward error of a backward-stable factorisation, 50 m eps cond(N) in
+the 2-norm (numpy's own included).
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import lpgen
+
+pytestmark = pytest.mark.gpu
+
+
+def solve_batch(hn, torch, ms, scale=1.0, masked=()):
+    lps = [lpgen.lp_uniform(m, 3 * m, min(4, m), 50 + i) for i, m in enumerate(ms)]
+    ro = np.cumsum([0] + list(ms)).astype(np.int64)
+    co = np.cumsum([0] + [3 * m for m in ms]).astype(np.int64)
+    rp = np.concatenate([[0]] + [lp["rp"][1:] + sum(len(p["ci"]) for p in lps[:i]) for i, lp in enumerate(lps)])
+    ci = np.concatenate([lp["ci"] + co[i] for i, lp in enumerate(lps)])
+    val = np.concatenate([lp["val"] for lp in lps])
+    A = hn.Csr(int(ro[-1]), int(co[-1]), rp, ci, val, autotune=False)
+    P = hn.Pattern(A)
+    rng = np.random.default_rng(7)
+    D, rhs = rng.uniform(0.5, 2.0, co[-1]) * scale, rng.standard_normal(ro[-1])
+    dev = lambda a: torch.as_tensor(a, device="cuda")  # noqa: E731
+    nval = torch.empty(P.nnz, dtype=torch.float64, device="cuda")
+    status = np.zeros(len(ms), np.int32)
+    status[list(masked)] = 1
+    Dd, rd, st, x = dev(D), dev(rhs), dev(status), torch.empty(int(ro[-1]), dtype=torch.float64, device="cuda")
+    lib, h = hn.load(), C.c_void_p()
+    p64 = C.POINTER(C.c_int64)
+    hn.check(lib.hn_batch_create(len(ms), ro.ctypes.data_as(p64), co.ctypes.data_as(p64), P.h, C.byref(h)))
+    try:
+        hn.check(lib.hn_batch_factor(h, Dd.data_ptr(), 0.0, 1e-300, nval.data_ptr(), st.data_ptr(), None))
+        hn.check(lib.hn_batch_solve(h, nval.data_ptr(), rd.data_ptr(), x.data_ptr(), st.data_ptr(), None))
+        torch.cuda.synchronize()
+    finally:
+        hn.check(lib.hn_batch_destroy(h))
+    return lps, ro, co, D, rhs, x.cpu().numpy()
+
+
+def check(i, lps, ro, co, D, rhs, x, scale):
+    lp = lps[i]
+    m, n = lp["m"], lp["n"]
+    A = np.zeros((m, n))
+    A[np.repeat(np.arange(m), np.diff(lp["rp"])), lp["ci"]] = lp["val"]
+    N = (A * (D[co[i]:co[i + 1]] / scale)) @ A.T
+    N[np.diag_indices(m)] += 1e-12 * N.diagonal().max()
+    ref = np.linalg.solve(N, rhs[ro[i]:ro[i + 1]])
+    got = x[ro[i]:ro[i + 1]] * scale
+    tol = 50 * m * np.finfo(float).eps * np.linalg.cond(N)
+    assert np.linalg.norm(got - ref) <= tol * np.linalg.norm(ref), (m, np.linalg.norm(got - ref), tol)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-140, 1e130])
+def test_block_edges(hn, torch_cuda, scale):
+    ms = [1, 2, 63, 64, 65, 127, 128, 129, 191, 192, 193, 256, 257, 319, 320, 321]
+    r = solve_batch(hn, torch_cuda, ms, scale)
+    for i in range(len(ms)):
+        check(i, *r, scale)
+
+
+@pytest.mark.parametrize("ms", [[1100, 1089, 1088, 833, 832, 577, 576, 449, 322], [1345], [400, 1, 400]])
+def test_solve_groups_and_masks(hn, torch_cuda, ms):
+    """Few instances: several CTAs each; a masked instance keeps its right-hand side."""
+    masked = [1] if len(ms) > 1 else []
+    r = solve_batch(hn, torch_cuda, ms, masked=masked)
+    for i in range(len(ms)):
+        if i in masked:
+            assert np.array_equal(r[5][r[1][i]:r[1][i + 1]], r[4][r[1][i]:r[1][i + 1]])
+        else:
+            check(i, *r, 1.0)
+
+
+def test_many_instances_one_cta_each(hn, torch_cuda):
+    """Enough instances that those with several row chunks still get one CTA."""
+    ms = [330, 70] * 400 + [900]
+    r = solve_batch(hn, torch_cuda, ms)
+    for i in list(range(0, 800, 97)) + [800]:
+        check(i, *r, 1.0)
