@@ -45,6 +45,7 @@ Workspace& workspace(cudaStream_t s) {
     w.partials = dmalloc<double>(4 * kMaxReduceBlocks + 8);
     w.counter = dmalloc<unsigned>(4);
     w.select = dmalloc<unsigned long long>(kSelectWords);
+    w.price = dmalloc<unsigned long long>(kPriceWords);
     check_cuda(cudaMemsetAsync(w.counter, 0, 4 * sizeof(unsigned), s), "workspace init");
     check_cuda(cudaMemsetAsync(w.select, 0, kSelectWords * sizeof(unsigned long long), s), "workspace init");
     check_cuda(cudaStreamSynchronize(s), "workspace init sync");
@@ -241,6 +242,7 @@ int hn_shutdown(void) {
             dfree(kv.second.partials);
             dfree(kv.second.counter);
             dfree(kv.second.select);
+            dfree(kv.second.price);
             dfree(kv.second.staging_d);
             if (kv.second.staging_h) cudaFreeHost(kv.second.staging_h);
         }

@@ -45,9 +45,12 @@ struct Workspace {
     size_t staging_bytes = 0;
     double* staging_d = nullptr;   // device staging for *_host calls
     size_t staging_d_bytes = 0;
-    unsigned long long* select = nullptr;  // pricing selection state, kSelectWords words
+    unsigned long long* select = nullptr;  // flags of calls that report from the device, kSelectWords words
+    unsigned long long* price = nullptr;   // pricing selection: blocks' lists and counts, kPriceWords words
 };
 constexpr int kSelectWords = 8;
+constexpr int kPriceLists = 148;  // blocks of the ranked selection, a list of HN_PRICE_MAX_K (score, index) each
+constexpr int kPriceWords = kPriceLists * (2 * HN_PRICE_MAX_K + 1);
 
 constexpr int kMaxReduceBlocks = 1184;  // 148 SMs x 8
 

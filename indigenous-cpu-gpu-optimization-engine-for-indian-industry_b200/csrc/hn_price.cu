@@ -14,8 +14,8 @@
 // A^T x sums each column's contributions in increasing row order, which is
 // the order of SparseMatrix::transpose_multiply's and update_devex_weights's
 // scatters, so reduced costs and Devex rows are bit-identical to the
-// reference's. Selection reduces with atomic max/min on integer keys, whose
-// result does not depend on the order the blocks arrive in.
+// reference's. Selection compares integer keys (score bits, then index) in
+// fixed trees, so its result does not depend on the order the blocks arrive in.
 #include <algorithm>
 #include <climits>
 
@@ -27,8 +27,7 @@ namespace {
 constexpr int kPT = 256;
 constexpr int kPriceBlocks = 148 * 4;
 
-// workspace select words
-constexpr int W_COUNT = 0, W_FIRST = 1, W_PREV_S = 2, W_PREV_I = 3, W_BEST_S = 4, W_BEST_I = 5, W_HAVE_PREV = 6;
+constexpr int W_BAD = 0;  // workspace select word: column indices out of range
 
 struct EpiReducedCost {
     const double* cost;
@@ -88,153 +87,252 @@ struct PriceArgs {
     double tol;
 };
 
-// Improving nonbasic column j (the filters of ranked_candidates and of the
+// What the choice reads of a column; loaded apart from its use, so that several are in flight.
+struct Column {
+    double rc, w;
+    bool skip;
+};
+__device__ __forceinline__ Column load_column(const PriceArgs& a, int64_t j) {
+    Column c{0.0, 1.0, true};
+    if (j >= a.n) return c;
+    c.skip = a.nonbasis[j] < 0 || (!a.phase1 && a.artificial && a.artificial[j]);
+    c.rc = a.rc[j];
+    if (a.w) c.w = a.w[j];
+    return c;
+}
+
+// Improving nonbasic column (the filters of ranked_candidates and of the
 // Bland scan); score = |rc_j| / sqrt(w_j) with w guarded to 1.
-__device__ __forceinline__ bool eligible(const PriceArgs& a, int64_t j, double& score) {
-    if (a.nonbasis[j] < 0) return false;
-    if (!a.phase1 && a.artificial && a.artificial[j]) return false;
-    double rc = a.rc[j];
-    if (a.maximize) rc = -rc;
-    if (!(rc < -a.tol)) return false;
-    double w = a.w ? a.w[j] : 1.0;
+__device__ __forceinline__ bool eligible(const PriceArgs& a, const Column& c, double& score) {
+    const double rc = a.maximize ? -c.rc : c.rc;
+    if (c.skip || !(rc < -a.tol)) return false;
+    double w = c.w;
     if (!(w > 0.0) || !isfinite(w)) w = 1.0;
     score = fabs(rc) / sqrt(w);
     return true;
 }
 
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
+__device__ __forceinline__ int64_t min_i64(int64_t a, int64_t b) { return a < b ? a : b; }
+template <int THREADS>
+__device__ __forceinline__ int64_t block_min_i64(int64_t v, int64_t* sh) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = u > v ? u : v;
-    }
-    return v;
-}
-__device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v) {
+    for (int o = 16; o > 0; o >>= 1) v = min_i64(v, __shfl_down_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if (lane == 0) sh[wid] = v;
+    __syncthreads();
+    int64_t r = INT64_MAX;
+    if (wid == 0) {
+        r = lane < THREADS / 32 ? sh[lane] : INT64_MAX;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = u < v ? u : v;
+        for (int o = 16; o > 0; o >>= 1) r = min_i64(r, __shfl_down_sync(0xffffffffu, r, o));
     }
-    return v;
+    return r;  // valid in thread 0
 }
 
-__global__ void price_init_kernel(unsigned long long* sel) {
-    if (threadIdx.x == 0) {
-        sel[W_COUNT] = 0ull;
-        sel[W_FIRST] = ULLONG_MAX;
-        sel[W_PREV_S] = 0ull;
-        sel[W_PREV_I] = 0ull;
-        sel[W_BEST_S] = 0ull;
-        sel[W_BEST_I] = ULLONG_MAX;
-        sel[W_HAVE_PREV] = 0ull;
+// A column of the ranking: score bits (scores are positive doubles, whose bit
+// patterns order like their values; 0 = none) and index. Order: score
+// descending, index ascending.
+struct Pick {
+    unsigned long long s, j;
+};
+__device__ __forceinline__ bool before(const Pick& a, const Pick& b) { return a.s > b.s || (a.s == b.s && a.j < b.j); }
+// The warp's first pick, by word reductions (a butterfly of pairs takes twenty
+// shuffles). Indices need their upper word only where n reaches 2^32 (wide).
+__device__ __forceinline__ Pick warp_best(const Pick& v, bool wide) {
+    const unsigned hi = static_cast<unsigned>(v.s >> 32), lo = static_cast<unsigned>(v.s);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    bool c = hi == mh && lo == ml;
+    unsigned jh = 0u;
+    if (wide) {
+        jh = __reduce_min_sync(0xffffffffu, c ? static_cast<unsigned>(v.j >> 32) : ~0u);
+        c = c && static_cast<unsigned>(v.j >> 32) == jh;
+    }
+    const unsigned jl = __reduce_min_sync(0xffffffffu, c ? static_cast<unsigned>(v.j) : ~0u);
+    return Pick{(unsigned long long)mh << 32 | ml, (unsigned long long)jh << 32 | jl};
+}
+
+constexpr int kSelT = 512;  // threads of the ranked selection
+constexpr int kSelE = 8;    // picks a thread holds of a chunk
+constexpr int kSelChunk = kSelT * kSelE;
+static_assert(HN_PRICE_MAX_K <= kSelT && kSelT / 32 == 16, "ranked selection shape");
+
+// The k first picks of the block's chunks (chunk c: picks c kSelChunk ..) into
+// list (shared memory, k entries, none = 0). load(i0, key) fills a thread's
+// kSelE picks of the chunk at i0. The list so far competes as one more pick of
+// k threads. One barrier per place: every warp reduces the warps' bests itself.
+template <class Load>
+__device__ __forceinline__ void select_chunks(int64_t first, int64_t step, int64_t n, int k, bool wide, Pick* list,
+                                              Pick (*sw)[16], Load load) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < k) list[tid] = Pick{0ull, ~0ull};
+    __syncthreads();
+    for (int64_t i0 = first; i0 < n; i0 += step) {
+        Pick key[kSelE];
+        load(i0, key);
+        Pick held = tid < k ? list[tid] : Pick{0ull, ~0ull};
+        const Pick last = list[k - 1];
+        bool any = false;
+#pragma unroll
+        for (int e = 0; e < kSelE; ++e) any |= key[e].s != 0ull && before(key[e], last);
+        if (!__syncthreads_or(any)) continue;  // nothing of this chunk places
+        auto own_best = [&]() {
+            Pick b = held;
+#pragma unroll
+            for (int e = 0; e < kSelE; ++e)
+                if (before(key[e], b)) b = key[e];
+            return b;
+        };
+        Pick own = own_best();  // changes only where a place was taken
+        for (int r = 0; r < k; ++r) {
+            Pick best = warp_best(own, wide);
+            if (lane == 0) sw[r & 1][warp] = best;
+            __syncthreads();
+            best = warp_best(sw[r & 1][lane & 15], wide);
+            if (tid == 0) list[r] = best;
+            if (best.s == 0ull) {  // the rest of the list keeps what it had: none of it is left
+                for (int q = r + tid; q < k; q += kSelT) list[q] = Pick{0ull, ~0ull};
+                break;
+            }
+            if (own.s == best.s && own.j == best.j) {
+                if (held.j == best.j) held.s = 0ull;
+#pragma unroll
+                for (int e = 0; e < kSelE; ++e)
+                    if (key[e].j == best.j) key[e].s = 0ull;
+                own = own_best();
+            }
+        }
+        __syncthreads();
     }
 }
 
-// Count of improving columns and the first one (Bland).
-__global__ void __launch_bounds__(kPT) price_count_kernel(PriceArgs a, unsigned long long* sel) {
-    unsigned long long cnt = 0, first = ULLONG_MAX;
+// Ranked selection in one pass: each block keeps the k first columns of its
+// chunks, the last block to finish merges the blocks' lists the same way. (A
+// pass for the best score, one for its lowest index and a close per place took
+// 300 us for 16 places of 500,000 columns; this takes 33.)
+__global__ void __launch_bounds__(kSelT, 1) price_ranked_kernel(PriceArgs a, int k, Pick* lists,
+                                                             unsigned long long* counts, unsigned* ticket,
+                                                             int64_t* out) {
+    __shared__ Pick list[HN_PRICE_MAX_K];
+    __shared__ Pick sw[2][16];
+    __shared__ int64_t sh[32];
+    __shared__ bool s_last;
+    const int tid = threadIdx.x;
+    const bool wide = a.n > (int64_t(1) << 32);
+    int64_t cnt = 0;
+    select_chunks(blockIdx.x * (int64_t)kSelChunk, gridDim.x * (int64_t)kSelChunk, a.n, k, wide, list, sw,
+                  [&](int64_t i0, Pick* key) {
+                      Column c[kSelE];
+#pragma unroll
+                      for (int e = 0; e < kSelE; ++e) c[e] = load_column(a, i0 + e * kSelT + tid);
+#pragma unroll
+                      for (int e = 0; e < kSelE; ++e) {
+                          double sc;
+                          const bool in = eligible(a, c[e], sc);
+                          cnt += in;
+                          key[e] = Pick{in ? (unsigned long long)__double_as_longlong(sc) : 0ull,
+                                        (unsigned long long)(i0 + e * kSelT + tid)};
+                      }
+                  });
+    cnt = block_sum_i64<kSelT>(cnt, sh);
+    if (gridDim.x > 1) {
+        if (tid < k) lists[blockIdx.x * k + tid] = list[tid];
+        if (tid == 0) counts[blockIdx.x] = (unsigned long long)cnt;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        const int64_t all = (int64_t)gridDim.x * k;
+        select_chunks(0, kSelChunk, all, k, wide, list, sw, [&](int64_t i0, Pick* key) {
+#pragma unroll
+            for (int e = 0; e < kSelE; ++e) {
+                const int64_t i = i0 + e * kSelT + tid;
+                key[e] = Pick{0ull, ~0ull};
+                if (i < all) key[e] = Pick{__ldcg(&lists[i].s), __ldcg(&lists[i].j)};
+            }
+        });
+        cnt = tid < (int)gridDim.x ? (int64_t)__ldcg(counts + tid) : 0;
+        cnt = block_sum_i64<kSelT>(cnt, sh);
+    }
+    if (tid == 0) {
+        out[0] = cnt;
+        *ticket = 0u;
+    }
+    if (tid < k) out[1 + tid] = list[tid].s ? (int64_t)list[tid].j : -1;
+}
+
+// Count of improving columns and the first one (Bland), the last block closing.
+__global__ void __launch_bounds__(kPT) price_bland_kernel(PriceArgs a, unsigned long long* part, unsigned* ticket,
+                                                          int64_t* out) {
+    __shared__ int64_t sh[32];
+    __shared__ bool s_last;
+    int64_t cnt = 0, first = INT64_MAX;
     for (int64_t j = blockIdx.x * (int64_t)kPT + threadIdx.x; j < a.n; j += (int64_t)gridDim.x * kPT) {
         double sc;
-        if (eligible(a, j, sc)) {
+        if (eligible(a, load_column(a, j), sc)) {
             ++cnt;
-            if ((unsigned long long)j < first) first = (unsigned long long)j;
+            if (j < first) first = j;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    first = warp_min_u64(first);
-    if ((threadIdx.x & 31) == 0) {
-        if (cnt) atomicAdd(sel + W_COUNT, cnt);
-        if (first != ULLONG_MAX) atomicMin(sel + W_FIRST, first);
+    cnt = block_sum_i64<kPT>(cnt, sh);
+    first = block_min_i64<kPT>(first, sh);
+    if (threadIdx.x == 0) {
+        part[2 * blockIdx.x] = (unsigned long long)cnt;
+        part[2 * blockIdx.x + 1] = (unsigned long long)first;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    cnt = 0;
+    first = INT64_MAX;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kPT) {
+        cnt += (int64_t)__ldcg(part + 2 * b);
+        const int64_t f = (int64_t)__ldcg(part + 2 * b + 1);
+        if (f < first) first = f;
+    }
+    cnt = block_sum_i64<kPT>(cnt, sh);
+    first = block_min_i64<kPT>(first, sh);
+    if (threadIdx.x == 0) {
+        out[0] = cnt;
+        out[1] = first == INT64_MAX ? -1 : first;
+        *ticket = 0u;
     }
 }
 
-// The previous pick of the ranking; (score, j) is eligible for this round when
-// it comes after it in the order (score desc, index asc).
-struct Prev {
-    bool have;
-    unsigned long long s, i;
-    __device__ __forceinline__ explicit Prev(const unsigned long long* sel)
-        : have(sel[W_HAVE_PREV] != 0ull), s(sel[W_PREV_S]), i(sel[W_PREV_I]) {}
-    __device__ __forceinline__ bool admits(unsigned long long sb, int64_t j) const {
-        return !have || sb < s || (sb == s && (unsigned long long)j > i);
-    }
-};
-
-// Round stage 1: the best score among columns after the previous pick.
-// Scores are positive doubles, whose bit patterns order like their values.
-__global__ void __launch_bounds__(kPT) price_best_score_kernel(PriceArgs a, unsigned long long* sel) {
-    const Prev prev(sel);
-    unsigned long long best = 0ull;
-    for (int64_t j = blockIdx.x * (int64_t)kPT + threadIdx.x; j < a.n; j += (int64_t)gridDim.x * kPT) {
-        double sc;
-        if (!eligible(a, j, sc)) continue;
-        const unsigned long long sb = (unsigned long long)__double_as_longlong(sc);
-        if (prev.admits(sb, j) && sb > best) best = sb;
-    }
-    best = warp_max_u64(best);
-    if ((threadIdx.x & 31) == 0 && best) atomicMax(sel + W_BEST_S, best);
-}
-
-// Round stage 2: the lowest index holding that score.
-__global__ void __launch_bounds__(kPT) price_best_index_kernel(PriceArgs a, unsigned long long* sel) {
-    const unsigned long long target = sel[W_BEST_S];
-    if (!target) return;
-    const Prev prev(sel);
-    unsigned long long bi = ULLONG_MAX;
-    for (int64_t j = blockIdx.x * (int64_t)kPT + threadIdx.x; j < a.n; j += (int64_t)gridDim.x * kPT) {
-        double sc;
-        if (!eligible(a, j, sc)) continue;
-        const unsigned long long sb = (unsigned long long)__double_as_longlong(sc);
-        if (sb == target && prev.admits(sb, j) && (unsigned long long)j < bi) bi = (unsigned long long)j;
-    }
-    bi = warp_min_u64(bi);
-    if ((threadIdx.x & 31) == 0 && bi != ULLONG_MAX) atomicMin(sel + W_BEST_I, bi);
-}
-
-// Round close: record the pick (or -1) and make it the new "previous".
-__global__ void price_round_close_kernel(unsigned long long* sel, int64_t* out, int64_t r) {
-    if (threadIdx.x != 0) return;
-    if (sel[W_BEST_S]) {
-        out[1 + r] = (int64_t)sel[W_BEST_I];
-        sel[W_PREV_S] = sel[W_BEST_S];
-        sel[W_PREV_I] = sel[W_BEST_I];
-        sel[W_HAVE_PREV] = 1ull;
-    } else {
-        out[1 + r] = -1;
-        sel[W_PREV_S] = 0ull;  // nothing sorts after a score of 0: later rounds find nothing
-        sel[W_PREV_I] = ULLONG_MAX;
-        sel[W_HAVE_PREV] = 1ull;
-    }
-    sel[W_BEST_S] = 0ull;
-    sel[W_BEST_I] = ULLONG_MAX;
-}
-
-__global__ void price_bland_close_kernel(const unsigned long long* sel, int64_t* out) {
-    if (threadIdx.x != 0) return;
-    out[0] = (int64_t)sel[W_COUNT];
-    out[1] = sel[W_FIRST] == ULLONG_MAX ? -1 : (int64_t)sel[W_FIRST];
-}
-
-__global__ void price_count_close_kernel(const unsigned long long* sel, int64_t* out) {
-    if (threadIdx.x == 0) out[0] = (int64_t)sel[W_COUNT];
-}
-
-// Columns outside [0, n) are left zero and counted in *bad.
-__global__ void __launch_bounds__(kPT) column_gather_kernel(int64_t m, int64_t n, const int32_t* __restrict__ rpT,
+// Column cols[r], rows [i0, i0 + kColRows) of slice blockIdx.x: zeros, then
+// the entries that lie there (a row of A^T ascends). Columns outside [0, n)
+// are left zero and counted in *bad.
+constexpr int kColRows = 8192;
+__global__ void __launch_bounds__(kPT) column_gather_kernel(int64_t m, int64_t n, int64_t k,
+                                                            const int32_t* __restrict__ rpT,
                                                             const int32_t* __restrict__ ciT,
                                                             const double* __restrict__ valT,
                                                             const int64_t* __restrict__ cols, double* __restrict__ out,
                                                             unsigned long long* bad) {
-    const int64_t r = blockIdx.x;
-    const int64_t j = cols[r];
-    if (j < 0 || j >= n) {
-        if (threadIdx.x == 0) atomicAdd(bad, 1ull);
-        return;
+    __shared__ int64_t sh[32];
+    const int64_t slices = m > 0 ? (m + kColRows - 1) / kColRows : 1;
+    const int64_t r = blockIdx.x / slices, i0 = (blockIdx.x % slices) * kColRows;
+    if (blockIdx.x == 0) {
+        int64_t b = 0;
+        for (int64_t q = threadIdx.x; q < k; q += kPT) b += cols[q] < 0 || cols[q] >= n;
+        b = block_sum_i64<kPT>(b, sh);
+        if (threadIdx.x == 0) *bad = (unsigned long long)b;
     }
+    const int64_t j = cols[r];
+    const int64_t i1 = i0 + kColRows < m ? i0 + kColRows : m;
     double* o = out + r * m;
-    for (int32_t e = rpT[j] + threadIdx.x; e < rpT[j + 1]; e += kPT) o[ciT[e]] = valT[e];
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += kPT) o[i] = 0.0;
+    if (j < 0 || j >= n) return;
+    __syncthreads();
+    for (int32_t e = rpT[j] + threadIdx.x; e < rpT[j + 1]; e += kPT) {
+        const int32_t i = ciT[e];
+        if (i >= i0 && i < i1) o[i] = valT[e];
+    }
 }
 
 int price_grid(int64_t n) {
@@ -287,26 +385,16 @@ int hn_price_select(int64_t n, const double* rc, const double* weights, const in
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
         const PriceArgs a{n, rc, weights, nonbasis, artificial, phase1, maximize, optimality_tol};
-        const int g = price_grid(n);
-        price_init_kernel<<<1, 32, 0, s>>>(w.select);
-        launched("price_init_kernel");
-        price_count_kernel<<<g, kPT, 0, s>>>(a, w.select);
-        launched("price_count_kernel");
         if (rule == HN_PRICE_BLAND) {
-            price_bland_close_kernel<<<1, 32, 0, s>>>(w.select, out);
-            launched("price_bland_close_kernel");
+            price_bland_kernel<<<price_grid(n), kPT, 0, s>>>(a, w.price, w.counter + 1, out);
+            launched("price_bland_kernel");
             return;
         }
-        price_count_close_kernel<<<1, 32, 0, s>>>(w.select, out);
-        launched("price_count_close_kernel");
-        for (int64_t r = 0; r < k; ++r) {
-            price_best_score_kernel<<<g, kPT, 0, s>>>(a, w.select);
-            launched("price_best_score_kernel");
-            price_best_index_kernel<<<g, kPT, 0, s>>>(a, w.select);
-            launched("price_best_index_kernel");
-            price_round_close_kernel<<<1, 32, 0, s>>>(w.select, out, r);
-            launched("price_round_close_kernel");
-        }
+        const int64_t chunks = (n + kSelChunk - 1) / kSelChunk;
+        const int g = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, kPriceLists));
+        price_ranked_kernel<<<g, kSelT, 0, s>>>(a, (int)k, reinterpret_cast<Pick*>(w.price),
+                                                w.price + 2 * kPriceLists * HN_PRICE_MAX_K, w.counter + 1, out);
+        launched("price_ranked_kernel");
     });
 }
 
@@ -318,13 +406,13 @@ int hn_price_columns(const hn_csr* A, int64_t k, const int64_t* cols, double* ou
         if (k == 0) return;
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
-        check_cuda(cudaMemsetAsync(out, 0, sizeof(double) * (size_t)A->m * (size_t)k, s), "memset columns");
-        check_cuda(cudaMemsetAsync(w.select + W_COUNT, 0, sizeof(unsigned long long), s), "memset flag");
-        column_gather_kernel<<<(unsigned)k, kPT, 0, s>>>(A->m, A->n, A->rpT, A->ciT, A->valT, cols, out,
-                                                         w.select + W_COUNT);
+        const int64_t slices = std::max<int64_t>(1, (A->m + kColRows - 1) / kColRows);
+        if (k > INT32_MAX / slices) fail(HN_ERR_INVALID_ARG, "too many columns for one call");
+        column_gather_kernel<<<(unsigned)(k * slices), kPT, 0, s>>>(A->m, A->n, k, A->rpT, A->ciT, A->valT, cols, out,
+                                                                    w.select + W_BAD);
         launched("column_gather_kernel");
         unsigned long long bad = 0;
-        check_cuda(cudaMemcpyAsync(&bad, w.select + W_COUNT, sizeof(bad), cudaMemcpyDeviceToHost, s), "D2H flag");
+        check_cuda(cudaMemcpyAsync(&bad, w.select + W_BAD, sizeof(bad), cudaMemcpyDeviceToHost, s), "D2H flag");
         check_cuda(cudaStreamSynchronize(s), "column gather sync");
         if (bad) fail(HN_ERR_INVALID_ARG, "column index out of range");
     });

@@ -103,3 +103,38 @@ def test_columns_match_extract_column(hn, torch_cuda):
     bad = dev(torch, np.array([1, 1250], dtype=np.int64))
     with pytest.raises(hn.HnError):
         hn.price_columns(A, bad, out[:2])
+
+
+@pytest.mark.parametrize("n,k,improving", [(1, 1, 1), (511, 64, 300), (4096, 16, 4000), (4097, 64, 3000),
+                                           (8192 + 3, 7, 5), (700_001, 64, 200_000), (700_001, 3, 1)])
+def test_select_chunk_edges(hn, torch_cuda, n, k, improving):
+    """Sizes around a block's chunk (4,096 columns) and past 148 blocks, few
+    and many improving columns, repeated scores: order (score descending,
+    index ascending), exact."""
+    rng = np.random.default_rng(n + k)
+    rc = np.abs(rng.standard_normal(n))
+    rc[rng.permutation(n)[:improving]] = -np.round(rng.uniform(1.0, 3.0, improving), 3)
+    w = rng.choice([1.0, 4.0, 0.25], n)
+    nb = np.arange(n, dtype=np.int32)
+    out = torch_cuda.empty(k + 1, dtype=torch_cuda.int64, device="cuda")
+    args = (dev(torch_cuda, rc), dev(torch_cuda, w), dev(torch_cuda, nb), None, out)
+    hn.price_select(n, *args, rule=hn.PRICE_RANKED, k=k)
+    got = out.cpu().numpy()
+    score = np.where(rc < -1e-9, np.abs(rc) / np.sqrt(w), 0.0)
+    want = np.lexsort((np.arange(n), -score))[:min(k, improving)]
+    assert got[0] == improving
+    assert np.array_equal(got[1:1 + want.size], want) and np.all(got[1 + want.size:] == -1)
+    hn.price_select(n, *args, rule=hn.PRICE_BLAND)
+    assert out.cpu().tolist()[:2] == [improving, int(np.flatnonzero(rc < -1e-9)[0])]
+
+
+@pytest.mark.parametrize("m", [1, 8191, 8192, 8193, 20_000])
+def test_columns_row_slices(hn, torch_cuda, m):
+    """Rows around the gather's slice of 8,192."""
+    lp = lpgen.lp_uniform(m, 40, min(m, 9), 3)
+    A = hn.Csr(m, 40, lp["rp"], lp["ci"], lp["val"])
+    cols = np.array([39, 0, 17], dtype=np.int64)
+    out = torch_cuda.full((3, m), np.nan, dtype=torch_cuda.float64, device="cuda")
+    hn.price_columns(A, dev(torch_cuda, cols), out)
+    for r, j in enumerate(cols):
+        assert np.array_equal(out[r].cpu().numpy(), O.extract_column(m, lp["rp"], lp["ci"], lp["val"], int(j)))
