@@ -72,21 +72,20 @@ void ensure_staging(Workspace& w, size_t bytes, cudaStream_t s);
 
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Device memory of the library's objects, from a bounded cache of freed
+// blocks (hn_core.cu). pool_free waits for the device, as cudaFree does, so a
+// block in the cache is idle on every stream.
+void* pool_alloc(size_t bytes);
+cudaError_t pool_free(void* p);
+void pool_release();  // gives the cached blocks back
+
 template <class T>
 T* dmalloc(size_t count) {
     if (count == 0) count = 1;
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        fail(e == cudaErrorMemoryAllocation ? HN_ERR_OUT_OF_MEMORY : HN_ERR_CUDA,
-             std::string("cudaMalloc of ") + std::to_string(count * sizeof(T)) +
-                 " bytes failed: " + cudaGetErrorString(e));
-    }
-    return static_cast<T*>(p);
+    return static_cast<T*>(pool_alloc(count * sizeof(T)));
 }
 inline void dfree(void* p) {
-    if (p) cudaFree(p);
+    if (p) pool_free(p);
 }
 
 inline int grid_for(int64_t n, int threads, int cap) {
