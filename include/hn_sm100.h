@@ -441,6 +441,12 @@ int hn_gnn_set_wait_limit(uint32_t polls);
 int hn_gnn_linear_bwd(int64_t M, int K1, int K2, const float* X1_dev, const float* X2_dev, const void* Wb_bf16_dev,
                       const float* Y_dev, const float* dY_dev, int relu, float* G_dev, float* dX_dev, float* dW_dev,
                       float* db_dev, float* scratch_dev, int64_t scratch_floats, void* stream);
+/* The same for K1 = K2 = 64 with dX as two arrays: dX1 (M x 64) for X1, dX2
+ * (M x 64) for X2, both 16-byte aligned. */
+int hn_gnn_linear_bwd_split(int64_t M, int K1, int K2, const float* X1_dev, const float* X2_dev,
+                            const void* Wb_bf16_dev, const float* Y_dev, const float* dY_dev, int relu, float* G_dev,
+                            float* dX1_dev, float* dX2_dev, float* dW_dev, float* db_dev, float* scratch_dev,
+                            int64_t scratch_floats, void* stream);
 /* dH (M x 64) += dX[:, :64]; dAgg (M x 64) = dX[:, 64:] (dX M x 128). */
 int hn_gnn_split_grad(int64_t M, const float* dX_dev, float* dH_dev, float* dAgg_dev, void* stream);
 /* dO (M x 64) = scale * 2 (O - T) in the first nt columns (T: M x 2), 0 in the

@@ -40,6 +40,9 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, const uint
 }
 
 // ---- SpMM: one warp per output row, each lane two of the 64 columns ----
+// Bound by the L2: every entry reads a 256-byte row of H (808,000 entries in
+// 26 us, 8 TB/s). More rows of H in flight (half a warp per row, eight rows
+// each) ran 32 us.
 __global__ void gnn_spmm_kernel(int rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                 const double* __restrict__ val, const float* __restrict__ H, int accumulate,
                                 float* __restrict__ out) {
@@ -260,13 +263,16 @@ __device__ __forceinline__ int umma_rows(int64_t M, int64_t tile) {
     return (int)(r < kUmmaM ? r : kUmmaM);
 }
 
-// Y (M x N, row stride N) = act([X1 | X2] Bt^T + bias), Bt: N x K BF16.
+// Y (M x N, row stride N) = act([X1 | X2] Bt^T + bias), Bt: N x K BF16. With
+// Y2, columns 64 .. N - 1 go there and Y's row stride is 64 (the gradients of a
+// concatenated input as two arrays, without a pass that splits them).
 template <int N, int KMAX>
 __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_kernel(int64_t M, int K1, int K2, const float* __restrict__ X1,
                                                              const float* __restrict__ X2,
                                                              const __nv_bfloat16* __restrict__ Bt,
                                                              const float* __restrict__ bias, int relu,
-                                                             float* __restrict__ Y, int* err, uint32_t spin) {
+                                                             float* __restrict__ Y, float* __restrict__ Y2, int* err,
+                                                             uint32_t spin) {
     using P = UmmaPlan<N, KMAX>;
     extern __shared__ __align__(1024) uint8_t umma_smem[];
     uint8_t* sA = umma_smem + P::kOffA;
@@ -419,8 +425,10 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_kernel(int64_t M, int K1, 
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int rr = 32 * q + 4 * j + (lane >> 3);
+                float* o = Y2 ? (cb < kH ? Y : Y2) + (t * kUmmaM + rr) * kH + (cb & (kH - 1))
+                              : Y + (t * kUmmaM + rr) * N + cb;
                 if (rr < rows)
-                    *reinterpret_cast<float4*>(Y + (t * kUmmaM + rr) * N + cb + 4 * (lane & 7)) =
+                    *reinterpret_cast<float4*>(o + 4 * (lane & 7)) =
                         *reinterpret_cast<const float4*>(sOut + rr * (N * 4) + cb * 4 + 16 * (lane & 7));
             }
             __syncwarp();
@@ -452,10 +460,13 @@ __global__ void gnn_relu_bwd_kernel(int64_t len, const float* __restrict__ dY, c
 
 // ---- weight gradient on the tcgen05 tensor cores ----
 // Per-CTA partial dW (K x 64) = [X1 | X2]^T G and db = column sums of G over
-// the CTA's 64-row tiles (t, t + grid, ...). One MMA operand pair per tile:
+// the CTA's 64-row tiles (t, t + grid, ...). G = dY relu'(Y) is formed in
+// shared memory from the tile's rows of dY and Y and written out on the way
+// (Gout; null: dY is G already): a pass of its own took 115 of 1,500 us of a
+// training step of 24 LPs. One MMA operand pair per tile:
 // A = [X1 | X2]^T (M = 128 feature rows, the rows past K kept zero) and B =
 // G^T (N = 64 outputs), both K-major over the tile's 64 rows. The tile's
-// rows of X1, X2 and G arrive by bulk copies into one of three FP32 stages;
+// rows of X1, X2, dY and Y arrive by bulk copies into one of three FP32 stages;
 // the CTA transposes them into the BF16 operands (a thread packs 8
 // consecutive rows of one column into one 16-byte core-matrix row), one
 // thread issues 4 tcgen05.mma (K = 16 each) accumulating into the same 64
@@ -466,10 +477,10 @@ __global__ void gnn_relu_bwd_kernel(int64_t len, const float* __restrict__ dY, c
 // rows in order. Every wait is bounded as in the layer kernel.
 constexpr int kWR = 64;                                 // rows per tile (the MMA's K extent)
 constexpr int kWStages = 3;
-constexpr int kWStage = kWR * (kMaxK + kH) * 4;         // 48 KB of FP32 rows
-constexpr int kWOffA = kWStages * kWStage;              // 144 KB
+constexpr int kWStage = kWR * (kMaxK + 2 * kH) * 4;     // 64 KB of FP32 rows
+constexpr int kWOffA = kWStages * kWStage;              // 192 KB
 constexpr int kWOffB = kWOffA + kUmmaM * kWR * 2;       // + 16 KB
-constexpr int kWSmem = kWOffB + kH * kWR * 2;           // + 8 KB = 168 KB
+constexpr int kWSmem = kWOffB + kH * kWR * 2;           // + 8 KB = 216 KB
 constexpr uint32_t kWLboA = (kUmmaM / 8) * 128;         // 2048
 constexpr uint32_t kWLboB = (kH / 8) * 128;             // 1024
 constexpr uint32_t kWIdesc = UmmaPlan<kH, kMaxK>::kIdesc;  // M = 128, N = 64
@@ -488,7 +499,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_wgrad_kernel(int64_t M, int K1, int K2,
                                                                    const float* __restrict__ X1,
                                                                    const float* __restrict__ X2,
-                                                                   const float* __restrict__ G,
+                                                                   const float* __restrict__ dY,
+                                                                   const float* __restrict__ Y, float* __restrict__ Gout,
                                                                    float* __restrict__ part_w,
                                                                    float* __restrict__ part_b, int* err,
                                                                    uint32_t spin) {
@@ -512,14 +524,17 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_wgrad_kernel(int64_t M, in
     }
     const uint32_t bar_full0 = smem_u32(&full[0]), bar_mma = smem_u32(&mma_bar);
     const uint32_t stage0 = smem_u32(wg_smem);
-    // tile t into stage s: X1 rows, then X2 rows (64 K1 floats on), then G rows (64 K floats on)
+    // tile t into stage s: X1 rows, then X2 rows (64 K1 floats on), then dY rows
+    // (64 K floats on) and, under a ReLU, Y rows
+    const int Kg = Y ? K + 2 * kH : K + kH;
     auto issue = [&](int64_t t, int s) {
         const uint32_t rows = (uint32_t)wgrad_rows(M, t), bar = bar_full0 + 8 * s;
         const uint32_t base = stage0 + s * kWStage;
-        mbar_expect(bar, rows * 4u * (uint32_t)(K + kH));
+        mbar_expect(bar, rows * 4u * (uint32_t)Kg);
         bulk_load(base, X1 + t * kWR * K1, rows * 4u * (uint32_t)K1, bar);
         if (K2) bulk_load(base + kWR * 4 * K1, X2 + t * kWR * K2, rows * 4u * (uint32_t)K2, bar);
-        bulk_load(base + kWR * 4 * K, G + t * kWR * kH, rows * 4u * (uint32_t)kH, bar);
+        bulk_load(base + kWR * 4 * K, dY + t * kWR * kH, rows * 4u * (uint32_t)kH, bar);
+        if (Y) bulk_load(base + kWR * 4 * (K + kH), Y + t * kWR * kH, rows * 4u * (uint32_t)kH, bar);
     };
     if (tid == 0) {
         for (int p = 0; p < kWStages; ++p) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_full0 + 8 * p));
@@ -543,6 +558,23 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_wgrad_kernel(int64_t M, in
         bool ok = !bad && mbar_wait(bar_full0 + 8 * s, (uint32_t)((i / kWStages) & 1), spin);
         // the previous tile's MMAs read A and B: restage only after they completed
         if (ok && i > 0) ok = mbar_wait(bar_mma, (uint32_t)((i - 1) & 1), spin);
+        if (ok) {
+            float* gs = reinterpret_cast<float*>(wg_smem + s * kWStage) + kWR * K;
+            if (Gout) {  // G in place of dY, and out
+                const float4* ys = reinterpret_cast<const float4*>(gs + kWR * kH);
+                for (int u = tid; u < rows * (kH / 4); u += kUmmaT) {
+                    float4 g = reinterpret_cast<float4*>(gs)[u];
+                    if (Y) {
+                        const float4 y = ys[u];
+                        g = make_float4(y.x > 0.f ? g.x : 0.f, y.y > 0.f ? g.y : 0.f, y.z > 0.f ? g.z : 0.f,
+                                        y.w > 0.f ? g.w : 0.f);
+                        reinterpret_cast<float4*>(gs)[u] = g;
+                    }
+                    reinterpret_cast<float4*>(Gout + t * kWR * kH)[u] = g;
+                }
+            }
+        }
+        if (Gout && Y) __syncthreads();  // G is complete (every thread, whatever its wait gave)
         if (ok) {
             const float* x1 = reinterpret_cast<const float*>(wg_smem + s * kWStage);
             const float* x2 = x1 + kWR * K1;
@@ -644,13 +676,34 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_wgrad_kernel(int64_t M, in
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kH));
 }
 
-// out[i] = sum over blocks b (in order) of part[b * len + i]
-__global__ void gnn_sum_parts_kernel(int64_t nb, int64_t len, const float* __restrict__ part, float* __restrict__ out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= len) return;
+// dW and db: sums over blocks b (in order) of their partials; 32 entries per
+// CTA, whose partials eight warps bring into shared memory before one adds them
+// up (the adds of an entry are a chain, and with its loads in that chain too a
+// launch took 7 us; 24 of them, 172 us, a training step).
+constexpr int kSumT = 256, kSumB = 256;  // threads, partials staged at a time
+__global__ void __launch_bounds__(kSumT) gnn_sum_parts_kernel(int64_t nb, int64_t len, const float* __restrict__ pw,
+                                                              const float* __restrict__ pb, float* __restrict__ dW,
+                                                              float* __restrict__ db) {
+    __shared__ float sp[kSumB][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t i = blockIdx.x * (int64_t)32 + lane;  // len and kH are multiples of 32: a CTA has entries of one kind
+    const bool bias = i >= len;
+    if (bias) i -= len;
+    const int64_t stride = bias ? kH : len;
+    const float* p = (bias ? pb : pw) + i;
     float s = 0.f;
-    for (int64_t b = 0; b < nb; ++b) s += part[b * len + i];
-    out[i] = s;
+    for (int64_t b0 = 0; b0 < nb; b0 += kSumB) {
+        const int n = (int)(nb - b0 < kSumB ? nb - b0 : kSumB);
+#pragma unroll 8
+        for (int b = warp; b < n; b += kSumT / 32) sp[b][lane] = p[(b0 + b) * stride];
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll 16
+            for (int b = 0; b < n; ++b) s += sp[b][lane];
+        }
+        __syncthreads();
+    }
+    if (warp == 0) (bias ? db : dW)[i] = s;
 }
 
 // W (K x 64, FP32 master, row-major) -> Wt (64 x K, BF16) and Wb (K x 64, BF16)
@@ -697,17 +750,66 @@ void smem_attribute(F* kernel, int bytes, int& done_device, const char* what) {
 // The tcgen05 layer kernel, one persistent CTA per SM (at most one per tile).
 template <int N, int KMAX>
 void launch_umma(int64_t M, int K1, int K2, const float* X1, const float* X2, const __nv_bfloat16* Bt,
-                 const float* bias, int relu, float* Y, cudaStream_t s) {
+                 const float* bias, int relu, float* Y, float* Y2, cudaStream_t s) {
     using P = UmmaPlan<N, KMAX>;
     static int attr_device = -1;
     smem_attribute(gnn_umma_kernel<N, KMAX>, P::kSmem, attr_device, "umma smem attribute");
     const int64_t tiles = (M + kUmmaM - 1) / kUmmaM;
     gnn_umma_kernel<N, KMAX><<<(unsigned)std::min<int64_t>(tiles, ctx().sm_count), kUmmaT, P::kSmem, s>>>(
-        M, K1, K2, X1, X2, Bt, bias, relu, Y, umma_flag(s), g_umma_spin.load());
+        M, K1, K2, X1, X2, Bt, bias, relu, Y, Y2, umma_flag(s), g_umma_spin.load());
     launched("gnn_umma_kernel");
 }
 
 bool misaligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
+
+void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, const void* Wb_bf16, const float* Y,
+                const float* dY, int relu, float* G, float* dX, float* dX2, float* dW, float* db, float* scratch,
+                int64_t scratch_floats, cudaStream_t s) {
+    const int K = K1 + K2;
+    if (M < 0 || K1 <= 0 || K2 < 0 || K > kMaxK || K1 % 16 || K2 % 16 || !X1 || (K2 && !X2) || !Y || !dY || !G ||
+        !dW || !db || !scratch)
+        fail(HN_ERR_INVALID_ARG, "bad arguments");
+    if (misaligned16(X1) || (K2 && misaligned16(X2)) || misaligned16(G) || (dX && misaligned16(dX)) ||
+        (dX2 && misaligned16(dX2)) || misaligned16(Wb_bf16) || misaligned16(scratch))
+        fail(HN_ERR_INVALID_ARG, "X1, X2, G, dX, the weights and the scratch must be 16-byte aligned");
+    if (dX && M > 0 && K != 64 && K != 128) fail(HN_ERR_INVALID_ARG, "dX needs K1 + K2 of 64 or 128");
+    const int64_t nb = std::max<int64_t>(1, std::min<int64_t>((M + kWR - 1) / kWR, ctx().sm_count));
+    if (scratch_floats < nb * (int64_t)(kH * K + kH)) fail(HN_ERR_INVALID_ARG, "scratch too small");
+    float* pw = scratch;
+    float* pb = scratch + nb * kH * K;
+    if (M > 0) {
+        // the weight-gradient kernel forms G; dY and Y that no bulk copy can
+        // read, or dY that G overwrites, take a pass of their own
+        const float *dy = dY, *y = relu ? Y : nullptr;
+        float* gout = G;
+        if (misaligned16(dY) || (relu && misaligned16(Y)) || G == dY || G == Y) {
+            const int64_t len = M * kH;
+            gnn_relu_bwd_kernel<<<(unsigned)std::min<int64_t>((len + 255) / 256, 148 * 16), 256, 0, s>>>(len, dY, Y,
+                                                                                                     relu, G);
+            launched("gnn_relu_bwd_kernel");
+            dy = G;
+            y = nullptr;
+            gout = nullptr;
+        }
+        static int attr_device = -1;
+        smem_attribute(gnn_umma_wgrad_kernel, kWSmem, attr_device, "wgrad smem attribute");
+        gnn_umma_wgrad_kernel<<<(unsigned)nb, kUmmaT, kWSmem, s>>>(M, K1, K2, X1, X2, dy, y, gout, pw, pb,
+                                                                    umma_flag(s), g_umma_spin.load());
+        launched("gnn_umma_wgrad_kernel");
+        // dX = G W^T on the tcgen05 layer kernel: input G (M x 64), N = K
+        // outputs, B = W (K x 64 row-major BF16), no bias, no activation
+        const auto* Bw = static_cast<const __nv_bfloat16*>(Wb_bf16);
+        if (dX && K == 64)
+            launch_umma<64, kH>(M, kH, 0, G, nullptr, Bw, nullptr, 0, dX, nullptr, s);
+        else if (dX)
+            launch_umma<128, kH>(M, kH, 0, G, nullptr, Bw, nullptr, 0, dX, dX2, s);
+    } else {
+        check_cuda(cudaMemsetAsync(scratch, 0, sizeof(float) * (kH * K + kH), s), "memset");
+    }
+    const int64_t len = (int64_t)kH * K;
+    gnn_sum_parts_kernel<<<(unsigned)((len + kH) / 32), kSumT, 0, s>>>(nb, len, pw, pb, dW, db);
+    launched("gnn_sum_parts_kernel");
+}
 
 }  // namespace
 }  // namespace hn
@@ -774,7 +876,7 @@ int hn_gnn_linear_umma(int64_t M, int K1, int K2, const float* X1, const float* 
             fail(HN_ERR_INVALID_ARG, "X1, X2, Y and the weights must be 16-byte aligned (bulk copies)");
         if (M == 0) return;
         launch_umma<kH, kMaxK>(M, K1, K2, X1, X2, static_cast<const __nv_bfloat16*>(Wt_bf16), bias, relu, Y,
-                               as_stream(stream));
+                               nullptr, as_stream(stream));
     });
 }
 
@@ -801,47 +903,19 @@ int hn_gnn_linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X
                       float* scratch, int64_t scratch_floats, void* stream) {
     return guard("hn_gnn_linear_bwd", [&] {
         require_init();
-        const int K = K1 + K2;
-        if (M < 0 || K1 <= 0 || K2 < 0 || K > kMaxK || K1 % 16 || K2 % 16 || !X1 || (K2 && !X2) || !Y || !dY ||
-            !G || !dW || !db || !scratch)
-            fail(HN_ERR_INVALID_ARG, "bad arguments");
-        if (misaligned16(X1) || (K2 && misaligned16(X2)) || misaligned16(G) || (dX && misaligned16(dX)) ||
-            misaligned16(Wb_bf16) || misaligned16(scratch))
-            fail(HN_ERR_INVALID_ARG, "X1, X2, G, dX, the weights and the scratch must be 16-byte aligned");
-        cudaStream_t s = as_stream(stream);
-        const int64_t nb = std::max<int64_t>(1, std::min<int64_t>((M + kWR - 1) / kWR, ctx().sm_count));
-        if (scratch_floats < nb * (int64_t)(kH * K + kH)) fail(HN_ERR_INVALID_ARG, "scratch too small");
-        const int64_t len = M * kH;
-        if (len > 0) {
-            gnn_relu_bwd_kernel<<<(unsigned)std::min<int64_t>((len + 255) / 256, 148 * 16), 256, 0, s>>>(len, dY, Y,
-                                                                                                     relu, G);
-            launched("gnn_relu_bwd_kernel");
-        }
-        // dX = G W^T on the tcgen05 layer kernel: input G (M x 64), N = K
-        // outputs, B = W (K x 64 row-major BF16), no bias, no activation
-        if (dX && M > 0) {
-            if (K != 64 && K != 128) fail(HN_ERR_INVALID_ARG, "dX needs K1 + K2 of 64 or 128");
-            const auto* B = static_cast<const __nv_bfloat16*>(Wb_bf16);
-            if (K == 64)
-                launch_umma<64, kH>(M, kH, 0, G, nullptr, B, nullptr, 0, dX, s);
-            else
-                launch_umma<128, kH>(M, kH, 0, G, nullptr, B, nullptr, 0, dX, s);
-        }
-        float* pw = scratch;
-        float* pb = scratch + nb * kH * K;
-        if (M > 0) {
-            static int attr_device = -1;
-            smem_attribute(gnn_umma_wgrad_kernel, kWSmem, attr_device, "wgrad smem attribute");
-            gnn_umma_wgrad_kernel<<<(unsigned)nb, kUmmaT, kWSmem, s>>>(M, K1, K2, X1, X2, G, pw, pb, umma_flag(s),
-                                                                        g_umma_spin.load());
-            launched("gnn_umma_wgrad_kernel");
-        } else {
-            check_cuda(cudaMemsetAsync(scratch, 0, sizeof(float) * (kH * K + kH), s), "memset");
-        }
-        gnn_sum_parts_kernel<<<(unsigned)((kH * K + 255) / 256), 256, 0, s>>>(nb, (int64_t)kH * K, pw, dW);
-        launched("gnn_sum_parts_kernel");
-        gnn_sum_parts_kernel<<<1, kH, 0, s>>>(nb, kH, pb, db);
-        launched("gnn_sum_parts_kernel");
+        linear_bwd(M, K1, K2, X1, X2, Wb_bf16, Y, dY, relu, G, dX, nullptr, dW, db, scratch, scratch_floats,
+                   as_stream(stream));
+    });
+}
+
+int hn_gnn_linear_bwd_split(int64_t M, int K1, int K2, const float* X1, const float* X2, const void* Wb_bf16,
+                            const float* Y, const float* dY, int relu, float* G, float* dX1, float* dX2, float* dW,
+                            float* db, float* scratch, int64_t scratch_floats, void* stream) {
+    return guard("hn_gnn_linear_bwd_split", [&] {
+        require_init();
+        if (K1 != kH || K2 != kH || !dX1 || !dX2) fail(HN_ERR_INVALID_ARG, "two inputs of 64 columns are wanted");
+        linear_bwd(M, K1, K2, X1, X2, Wb_bf16, Y, dY, relu, G, dX1, dX2, dW, db, scratch, scratch_floats,
+                   as_stream(stream));
     });
 }
 

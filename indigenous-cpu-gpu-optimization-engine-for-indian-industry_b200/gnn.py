@@ -262,35 +262,37 @@ def backward(model: Model, B: Batch, cache: dict):
     scratch = torch.empty(scratch_len, dtype=torch.float32, device="cuda")
     G = torch.empty(rows_max * H, dtype=torch.float32, device="cuda")
 
-    def lin_bwd(X1, X2, name, Y, dY, relu, rows, dX):
-        K1 = X1.shape[1]
-        K2 = 0 if X2 is None else X2.shape[1]
-        hn.check(lib.hn_gnn_linear_bwd(rows, K1, K2, X1.data_ptr(), None if X2 is None else X2.data_ptr(),
-                                       model.wb[name].data_ptr(), Y.data_ptr(), dY.data_ptr(), relu, G.data_ptr(),
+    def lin_bwd(X1, name, Y, dY, relu, rows, dX):
+        hn.check(lib.hn_gnn_linear_bwd(rows, X1.shape[1], 0, X1.data_ptr(), None, model.wb[name].data_ptr(),
+                                       Y.data_ptr(), dY.data_ptr(), relu, G.data_ptr(),
                                        None if dX is None else dX.data_ptr(), model.dW(name).data_ptr(),
                                        model.db(name).data_ptr(), scratch.data_ptr(), scratch_len, None))
 
+    def lin_bwd2(X1, X2, name, Y, dY, rows):
+        """Gradients of a message-passing layer's two inputs."""
+        d1, d2 = _empty(torch, rows), _empty(torch, rows)
+        hn.check(lib.hn_gnn_linear_bwd_split(rows, H, H, X1.data_ptr(), X2.data_ptr(), model.wb[name].data_ptr(),
+                                             Y.data_ptr(), dY.data_ptr(), 1, G.data_ptr(), d1.data_ptr(),
+                                             d2.data_ptr(), model.dW(name).data_ptr(), model.db(name).data_ptr(),
+                                             scratch.data_ptr(), scratch_len, None))
+        return d1, d2
+
     hv, hc, ac, av = cache["hv"], cache["hc"], cache["ac"], cache["av"]
     dhv, dhc = _empty(torch, B.n), _empty(torch, B.m)
-    lin_bwd(hv[-1], None, "hv", cache["ov"], dov, 0, B.n, dhv)
-    lin_bwd(hc[-1], None, "hc", cache["oc"], doc, 0, B.m, dhc)
-    dXv, dXc = _empty(torch, B.n, 2 * H), _empty(torch, B.m, 2 * H)
+    lin_bwd(hv[-1], "hv", cache["ov"], dov, 0, B.n, dhv)
+    lin_bwd(hc[-1], "hc", cache["oc"], doc, 0, B.m, dhc)
     for l in reversed(range(LAYERS)):
         # h_v[l+1] = relu([h_v[l] | a_v[l]] W_v[l] + b)
-        lin_bwd(hv[l], av[l], f"v{l}", hv[l + 1], dhv, 1, B.n, dXv)
-        ndhv, dav = torch.zeros((B.n, H), dtype=torch.float32, device="cuda"), _empty(torch, B.n)
-        hn.check(lib.hn_gnn_split_grad(B.n, dXv.data_ptr(), ndhv.data_ptr(), dav.data_ptr(), None))
+        ndhv, dav = lin_bwd2(hv[l], av[l], f"v{l}", hv[l + 1], dhv, B.n)
         # a_v[l] = A_c^T h_c[l+1]  ->  d h_c[l+1] += A_c d a_v[l]
         hn.check(lib.hn_gnn_spmm(B.Ac.h, 0, dav.data_ptr(), dhc.data_ptr(), 1, None))
         # h_c[l+1] = relu([h_c[l] | a_c[l]] W_c[l] + b)
-        lin_bwd(hc[l], ac[l], f"c{l}", hc[l + 1], dhc, 1, B.m, dXc)
-        ndhc, dac = torch.zeros((B.m, H), dtype=torch.float32, device="cuda"), _empty(torch, B.m)
-        hn.check(lib.hn_gnn_split_grad(B.m, dXc.data_ptr(), ndhc.data_ptr(), dac.data_ptr(), None))
+        ndhc, dac = lin_bwd2(hc[l], ac[l], f"c{l}", hc[l + 1], dhc, B.m)
         # a_c[l] = A_r h_v[l]  ->  d h_v[l] += A_r^T d a_c[l]
         hn.check(lib.hn_gnn_spmm(B.Ar.h, 1, dac.data_ptr(), ndhv.data_ptr(), 1, None))
         dhv, dhc = ndhv, ndhc
-    lin_bwd(B.Fv, None, "ev", hv[0], dhv, 1, B.n, None)
-    lin_bwd(B.Fc, None, "ec", hc[0], dhc, 1, B.m, None)
+    lin_bwd(B.Fv, "ev", hv[0], dhv, 1, B.n, None)
+    lin_bwd(B.Fc, "ec", hc[0], dhc, 1, B.m, None)
     hn.check(lib.hn_gnn_check(None))
     return float(lp_v.sum().item()) / B.n + float(lp_c.sum().item()) / B.m
 

@@ -108,6 +108,8 @@ SIGNATURES = {
     "hn_gnn_set_wait_limit": [C.c_uint32],
     "hn_gnn_linear_bwd": [_i64, C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, C.c_int, _vp, _vp, _vp, _vp, _vp, _i64,
                           _vp],
+    "hn_gnn_linear_bwd_split": [_i64, C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, C.c_int, _vp, _vp, _vp, _vp, _vp,
+                                _vp, _i64, _vp],
     "hn_gnn_split_grad": [_i64, _vp, _vp, _vp, _vp],
     "hn_gnn_head_grad": [_i64, _vp, _vp, C.c_int, C.c_float, _vp, _vp, _i64, _vp],
     "hn_gnn_adam": [_i64, _vp, _vp, _vp, _vp, C.c_float, C.c_float, C.c_float, C.c_float, _i64, _vp],

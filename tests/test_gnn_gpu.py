@@ -282,3 +282,48 @@ def test_tcgen05_backward_wait_timeout_is_reported_and_the_context_recovers(hn, 
     hn.check(lib.hn_gnn_check(None))
     for a, b in zip(ref, out):
         assert torch.equal(a, b)
+
+
+def _bwd_inputs(hn, torch, M, K1, K2, seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")  # noqa: E731
+    K = K1 + K2
+    W = r(K, 64)
+    wt, wb = (torch.empty(K * 64, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    hn.check(hn.load().hn_gnn_cast_weights(K, W.data_ptr(), wt.data_ptr(), wb.data_ptr(), None))
+    return r(M, K1), r(M, K2) if K2 else None, wb, r(M, 64), r(M, 64), torch.empty(148 * (64 * K + 64), device="cuda")
+
+
+def _bwd(hn, torch, x1, x2, wb, Y, dY, scratch, relu, dX, G, split=None):
+    M, K1, K2 = x1.shape[0], x1.shape[1], 0 if x2 is None else x2.shape[1]
+    dW, db = torch.empty((K1 + K2) * 64, device="cuda"), torch.empty(64, device="cuda")
+    a = (M, K1, K2, x1.data_ptr(), None if x2 is None else x2.data_ptr(), wb.data_ptr(), Y.data_ptr(), dY.data_ptr(),
+         relu, G.data_ptr())
+    z = (dW.data_ptr(), db.data_ptr(), scratch.data_ptr(), scratch.numel(), None)
+    if split is None:
+        hn.check(hn.load().hn_gnn_linear_bwd(*a, None if dX is None else dX.data_ptr(), *z))
+    else:
+        hn.check(hn.load().hn_gnn_linear_bwd_split(*a, split[0].data_ptr(), split[1].data_ptr(), *z))
+    hn.check(hn.load().hn_gnn_check(None))
+    return dW, db
+
+
+@pytest.mark.parametrize("M", [1, 63, 64, 65, 128, 129, 148 * 64, 148 * 64 + 1, 30_001])
+@pytest.mark.parametrize("relu", [0, 1])
+def test_backward_routes_agree(hn, torch_cuda, M, relu):
+    """G formed in the weight-gradient kernel, or in a pass of its own (dY and Y
+    off the 16-byte grid; G over dY), and dX whole or as two arrays: the same bits."""
+    torch = torch_cuda
+    x1, x2, wb, Y, dY, scratch = _bwd_inputs(hn, torch, M, 64, 64, M + relu)
+    G, dX = torch.empty(M, 64, device="cuda"), torch.empty(M, 128, device="cuda")
+    dW, db = _bwd(hn, torch, x1, x2, wb, Y, dY, scratch, relu, dX, G)
+    assert torch.equal(G, torch.where(Y > 0, dY, torch.zeros_like(dY)) if relu else dY)
+    off = lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(M, 64)  # noqa: E731
+    for Yo, dYo, Go in ((off(Y), off(dY), torch.empty_like(G)), (Y, None, dY.clone())):
+        dX2 = torch.empty_like(dX)
+        dW2, db2 = _bwd(hn, torch, x1, x2, wb, Yo, Go if dYo is None else dYo, scratch, relu, dX2, Go)
+        assert all(torch.equal(a, b) for a, b in ((G, Go), (dX, dX2), (dW, dW2), (db, db2)))
+    d1, d2, G3 = torch.empty(M, 64, device="cuda"), torch.empty(M, 64, device="cuda"), torch.empty_like(G)
+    dW3, db3 = _bwd(hn, torch, x1, x2, wb, Y, dY, scratch, relu, None, G3, split=(d1, d2))
+    assert all(torch.equal(a, b) for a, b in ((G, G3), (dX[:, :64], d1), (dX[:, 64:], d2), (dW, dW3), (db, db3)))
