@@ -283,11 +283,6 @@ __global__ void ada_vd_kernel(int64_t nnz, const double* __restrict__ val, const
         vd[e] = make_double2(val[e], __ldg(d + ci[e]));
 }
 
-__device__ __forceinline__ double term(uint2 pe, const double2* __restrict__ vd, const double* __restrict__ valT) {
-    const double2 q = __ldg(vd + pe.y);
-    return (q.y <= 0.0) ? 0.0 : (q.x * __ldg(valT + pe.x)) * q.y;  // columns with D_j <= 0 skipped
-}
-
 // Numeric phase, two kernels per call:
 //   ada_combine_kernel sums every multi slot's terms in column order (the
 //     order from_triplets' stable sort leaves them in) into the compact mval;
@@ -442,9 +437,29 @@ __global__ void ada_ecs_kernel(int64_t nnz, const int32_t* __restrict__ ci, cons
         ecs[e] = rpT[ci[e]];
 }
 
-// The first kBatch terms of a slot are gathered together; longer lists
-// continue one term at a time.
-constexpr int kBatch = 4;
+// A slot's terms are gathered kBatch at a time (a diagonal has as many as its
+// row of A has entries; one at a time past the first four, each waited for its
+// list entry and then its values: 8.7 us at 2,000 rows of 20, now 7.0), added
+// in column order. Large ones are bound by random 32-byte sectors (39 million
+// in 213 us); four slots per thread with their gathers together took 332 us.
+constexpr int kBatch = 4, kLongBatch = 8;
+template <int B>
+__device__ __forceinline__ void add_terms(double& s, int32_t u, int32_t u1, const uint2* __restrict__ mlist,
+                                          const double2* __restrict__ vd, const double* __restrict__ valT) {
+    uint2 pe[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) pe[k] = (u + k < u1) ? __ldg(mlist + u + k) : make_uint2(0u, 0u);
+    double2 q[B];
+    double b[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+        q[k] = __ldg(vd + pe[k].y);
+        b[k] = __ldg(valT + pe[k].x);
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+        if (u + k < u1) s += (q[k].y <= 0.0) ? 0.0 : (q[k].x * b[k]) * q[k].y;  // columns with D_j <= 0 skipped
+}
 __global__ void ada_combine_kernel(int64_t nms, const int64_t* __restrict__ mpos, const int32_t* __restrict__ mbeg,
                                    const uint2* __restrict__ mlist, const double2* __restrict__ vd,
                                    const double* __restrict__ valT, double* __restrict__ mval,
@@ -452,24 +467,12 @@ __global__ void ada_combine_kernel(int64_t nms, const int64_t* __restrict__ mpos
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nms) return;
     const int32_t u0 = mbeg[t], u1 = mbeg[t + 1];
-    uint2 pe[kBatch];
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) pe[k] = (u0 + k < u1) ? __ldg(mlist + u0 + k) : make_uint2(0u, 0u);
-    double2 q[kBatch];
-    double b[kBatch];
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-        q[k] = __ldg(vd + pe[k].y);
-        b[k] = __ldg(valT + pe[k].x);
-    }
+    const bool diag = mpos[t] & kDiagFlag;
     double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k)
-        if (u0 + k < u1) s += (q[k].y <= 0.0) ? 0.0 : (q[k].x * b[k]) * q[k].y;
-    for (int32_t u = u0 + kBatch; u < u1; ++u) s += term(mlist[u], vd, valT);
+    add_terms<kBatch>(s, u0, u1, mlist, vd, valT);
+    for (int32_t u = u0 + kBatch; u < u1; u += kLongBatch) add_terms<kLongBatch>(s, u, u1, mlist, vd, valT);
     mval[t] = s;
-    if ((mpos[t] & kDiagFlag) && s > 0.0)
-        atomicMax(maxdiag, static_cast<unsigned long long>(__double_as_longlong(s)));
+    if (diag && s > 0.0) atomicMax(maxdiag, static_cast<unsigned long long>(__double_as_longlong(s)));
 }
 
 // Row mode: one CTA per row of N at a time, the row assembled in shared

@@ -71,6 +71,7 @@ struct hn_batch {
     int64_t ntiles = 0;
     int32_t *tile_row = nullptr, *tile_nz = nullptr, *carry_row = nullptr, *head_row = nullptr;
     double *carry_val = nullptr, *head_val = nullptr;
+    bool short_heads = false;
     double* r = nullptr;         // refinement residual, m
     double* ax = nullptr;        // N x, m
     hn::InstInfo* info = nullptr;  // K
@@ -1416,8 +1417,11 @@ KktArgs kkt_args(const hn_batch* B, const double* lam, const double* b, const do
 }
 
 SpmvMat n_mat(const hn_batch* B, const double* nval) {
-    return SpmvMat{(int)B->m, (int)B->P->nnz, B->nrp, B->P->ci, nval, B->tile_row, B->tile_nz, B->carry_row,
-                   B->carry_val, B->head_row, B->head_val, B->ntiles};
+    SpmvMat N{(int)B->m, (int)B->P->nnz, B->nrp, B->P->ci, nval, B->tile_row, B->tile_nz, B->carry_row,
+              B->carry_val, B->head_row, B->head_val, B->ntiles};
+    N.ticket = reinterpret_cast<unsigned*>(B->carry_row + B->ntiles);
+    N.short_heads = B->short_heads;
+    return N;
 }
 
 // x holds the right-hand sides of the taking-part instances on entry, their solutions on return.
@@ -1496,7 +1500,7 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             narrow_rp_kernel<<<(unsigned)((m + 1 + 255) / 256), 256, 0, s>>>(m + 1, P->rp, B->nrp);
             launched("narrow_rp_kernel");
             make_tile_table(B->nrp, m, P->nnz, &B->ntiles, &B->tile_row, &B->tile_nz, &B->carry_row, &B->carry_val,
-                            &B->head_row, &B->head_val, s);
+                            &B->head_row, &B->head_val, &B->short_heads, s);
             // level schedule (instances in decreasing size: the ones with a block
             // at step s form a prefix of `order`)
             const int64_t mmax = row_off_host[order[0] + 1] - row_off_host[order[0]];
@@ -1599,8 +1603,7 @@ int hn_batch_residuals(hn_batch* B, const hn_csr* M, const double* x, const doub
         require_init();
         if (!B || !M || !M->has_t) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
-        spmv_launch(spmv_mat(M, 0), x, EpiResidual{b, mx, rp}, s);
-        spmv_launch(spmv_mat(M, 1), lam, EpiDualResidual{z, c, rd}, s);
+        spmv_launch2(spmv_mat(M, 0), x, EpiResidual{b, mx, rp}, spmv_mat(M, 1), lam, EpiDualResidual{z, c, rd}, s);
         batch_prep_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->col_off, x, z, rd, rp, D, Drd, scal, status,
                                                         iters, iter, tol, ctol, kkt_args(B, lam, b, c));
         launched("batch_prep_kernel");

@@ -193,18 +193,40 @@ __global__ void tiles_kernel(const int32_t* __restrict__ rp, int64_t m, int64_t 
 
 inline unsigned blocks(int64_t n, int t = 256) { return static_cast<unsigned>((n + t - 1) / t); }
 
+// The longest part of a row that lies before the start of the tile it reaches into.
+__global__ void longest_head_kernel(const int32_t* __restrict__ rp, int64_t m, int64_t nnz, int64_t ntiles,
+                                    const int32_t* __restrict__ trow, const int32_t* __restrict__ tnz, int* longest) {
+    int len = 0;
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ntiles; t += (int64_t)gridDim.x * blockDim.x)
+        if (trow[t] < m) len = max(len, tnz[t] - rp[trow[t]]);
+    len = __reduce_max_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0 && len > 0) atomicMax(longest, len);
+}
+
 void build_tiles(const int32_t* rp, int64_t m, int64_t nnz, int64_t& ntiles, int32_t*& trow,
-                 int32_t*& tnz, int32_t*& crow, double*& cval, int32_t*& hrow, double*& hval,
+                 int32_t*& tnz, int32_t*& crow, double*& cval, int32_t*& hrow, double*& hval, bool& short_heads,
                  cudaStream_t s) {
     ntiles = (m + nnz + kSpmvTile - 1) / kSpmvTile;
     trow = dmalloc<int32_t>(ntiles + 1);
     tnz = dmalloc<int32_t>(ntiles + 1);
-    crow = dmalloc<int32_t>(ntiles);
+    crow = dmalloc<int32_t>(ntiles + 1);  // the last entry is the ticket of the one-launch product
+    check_cuda(cudaMemsetAsync(crow + ntiles, 0, sizeof(int32_t), s), "memset ticket");
     cval = dmalloc<double>(ntiles);
     hrow = dmalloc<int32_t>(ntiles);
     hval = dmalloc<double>(ntiles);
     tiles_kernel<<<blocks(ntiles + 1), 256, 0, s>>>(rp, m, nnz, kSpmvTile, ntiles, trow, tnz);
     launched("tiles_kernel");
+    // crow[ntiles] serves as the result before it becomes the ticket (zero)
+    short_heads = false;
+    if (ntiles > 0 && ntiles <= kSpmvSmallTiles) {
+        longest_head_kernel<<<blocks(ntiles), 256, 0, s>>>(rp, m, nnz, ntiles, trow, tnz, crow + ntiles);
+        launched("longest_head_kernel");
+        int longest = 0;
+        check_cuda(cudaMemcpyAsync(&longest, crow + ntiles, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H heads");
+        check_cuda(cudaMemsetAsync(crow + ntiles, 0, sizeof(int32_t), s), "memset ticket");
+        check_cuda(cudaStreamSynchronize(s), "heads sync");
+        short_heads = longest <= kHeadNnz;
+    }
 }
 
 void free_transpose(hn_csr* A) {
@@ -338,7 +360,7 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
     dfree(row_of);
     dfree(kept_d);
     build_tiles(A->rpT, n, A->nnz_t, A->ntiles_t, A->tile_row_t, A->tile_nz_t, A->carry_row_t,
-                A->carry_val_t, A->head_row_t, A->head_val_t, s);
+                A->carry_val_t, A->head_row_t, A->head_val_t, A->short_heads[1], s);
     check_cuda(cudaStreamSynchronize(s), "tiles sync");
     A->has_t = true;
 }
@@ -577,8 +599,8 @@ void coo_to_csr(int64_t m, int64_t n, int64_t nnz, const int32_t* r, const int32
 }  // namespace
 
 void make_tile_table(const int32_t* rp, int64_t m, int64_t nnz, int64_t* ntiles, int32_t** trow, int32_t** tnz,
-                     int32_t** crow, double** cval, int32_t** hrow, double** hval, cudaStream_t s) {
-    build_tiles(rp, m, nnz, *ntiles, *trow, *tnz, *crow, *cval, *hrow, *hval, s);
+                     int32_t** crow, double** cval, int32_t** hrow, double** hval, bool* short_heads, cudaStream_t s) {
+    build_tiles(rp, m, nnz, *ntiles, *trow, *tnz, *crow, *cval, *hrow, *hval, *short_heads, s);
 }
 
 }  // namespace hn
@@ -615,7 +637,7 @@ int hn_csr_create(int64_t m, int64_t n, const uint64_t* rp, const uint64_t* ci, 
                            "H2D values");
             }
             build_tiles(A->rp, m, nnz, A->ntiles, A->tile_row, A->tile_nz, A->carry_row, A->carry_val,
-                        A->head_row, A->head_val, s);
+                        A->head_row, A->head_val, A->short_heads[0], s);
             if (!(flags & HN_CSR_NO_TRANSPOSE)) build_transpose(A, s);
             check_cuda(cudaStreamSynchronize(s), "hn_csr_create sync");
             if (!(flags & HN_CSR_NO_AUTOTUNE)) autotune(A, s);
@@ -669,7 +691,7 @@ int hn_csr_create_coo(int64_t m, int64_t n, int64_t count, const int64_t* rows, 
             dr = dc = nullptr;
             dv = nullptr;
             build_tiles(A->rp, m, A->nnz, A->ntiles, A->tile_row, A->tile_nz, A->carry_row, A->carry_val,
-                        A->head_row, A->head_val, s);
+                        A->head_row, A->head_val, A->short_heads[0], s);
             if (!(flags & HN_CSR_NO_TRANSPOSE)) build_transpose(A, s);
             check_cuda(cudaStreamSynchronize(s), "hn_csr_create_coo sync");
             if (!(flags & HN_CSR_NO_AUTOTUNE)) autotune(A, s);

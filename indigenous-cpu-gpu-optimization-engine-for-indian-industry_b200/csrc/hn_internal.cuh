@@ -111,7 +111,7 @@ void reduce_maxabs(int64_t n, const double* a, double* out, cudaStream_t s);
 // Merge-path tile table + carry buffers for a CSR with int32 row pointer rp
 // (m rows, nnz nonzeros); allocates the six arrays (hn_csr.cu).
 void make_tile_table(const int32_t* rp, int64_t m, int64_t nnz, int64_t* ntiles, int32_t** trow, int32_t** tnz,
-                     int32_t** crow, double** cval, int32_t** hrow, double** hval, cudaStream_t s);
+                     int32_t** crow, double** cval, int32_t** hrow, double** hval, bool* short_heads, cudaStream_t s);
 
 // A D A^T numeric without the regularisation step (hn_ada.cu): N's values
 // with every diagonal still un-regularised. Used by the batched IPM, which
@@ -275,6 +275,7 @@ int guard(const char* name, F&& body) {
 // 2^lg[b] lanes takes about `t` nonzeros per lane; perm lists the rows bin by
 // bin (ascending within a bin); a warp handles 32 / 2^lg rows of one bin.
 constexpr int kSpmvMaxBins = 6;
+constexpr int kHeadNnz = 256;  // entries of a row that a merge-path tile recomputes from the tile before
 struct SpmvBins {
     int nbins = 0;
     int unit_off[kSpmvMaxBins + 1] = {};  // first warp of each bin
@@ -317,6 +318,7 @@ struct hn_csr {
     int spmv_t[2] = {0, 0};
     int32_t* perm[2] = {nullptr, nullptr};
     SpmvBins bins[2];
+    bool short_heads[2] = {false, false};  // no row has more than kHeadNnz entries before a tile's start
 };
 
 struct hn_pattern {

@@ -121,3 +121,48 @@ def test_autotune_choice_and_set_values(hn, torch_cuda, big_lp):
     A.spmv(dev(torch_cuda, lam), t_, trans=1)
     rpT, ciT, valT = O.transposed(lp["rp"], lp["ci"], val, n)
     assert normwise_ok(t_.cpu().numpy(), O.tmultiply(lp["rp"], lp["ci"], val, lam, n), rpT, ciT, valT, lam)
+
+
+def _rows_of(kind, rng):
+    """Row lengths around the merge path's tiles (1,792 row ends and entries)."""
+    if kind == "one tile":
+        return np.full(100, 16)  # 100 + 1,600 items
+    if kind == "tile - 1":
+        return np.array([1790] + [0] * 0)
+    if kind == "tile":
+        return np.array([1791])
+    if kind == "tile + 1":
+        return np.array([1790, 1])
+    if kind == "heads at the limit":  # rows of 256 and 257 entries reach over tile starts
+        return np.array(([256] * 6 + [242]) * 4)
+    if kind == "heads past the limit":
+        return np.array([1400, 600, 300] * 5)
+    if kind == "row over many tiles":
+        return np.array([3, 9000, 0, 5, 4000])
+    if kind == "empty rows":
+        return np.where(rng.random(9000) < 0.8, 0, rng.integers(1, 12, 9000))
+    return rng.integers(0, 40, 5000)
+
+
+@pytest.mark.parametrize("kind", ["one tile", "tile - 1", "tile", "tile + 1", "heads at the limit",
+                                  "heads past the limit", "row over many tiles", "empty rows", "mixed"])
+def test_one_launch_product_has_the_two_launch_bits(hn, torch_cuda, kind):
+    """Few tiles: one launch, the carries recomputed by the tile or fixed up by
+    the last one. hn_spmv_noalloc runs tiles and fix-up as two launches."""
+    torch = torch_cuda
+    rng = np.random.default_rng(len(kind))
+    rows = _rows_of(kind, rng)
+    m, n = rows.size, 10_000
+    rp = np.concatenate([[0], np.cumsum(rows)]).astype(np.int64)
+    ci = np.concatenate([np.sort(rng.choice(n, k, replace=False)) for k in rows] + [np.zeros(0, np.int64)])
+    val, x = rng.standard_normal(ci.size), torch.as_tensor(rng.standard_normal(n), device="cuda")
+    A = hn.Csr(m, n, rp, ci, val)
+    y, want = (torch.full((m,), np.nan, dtype=torch.float64, device="cuda") for _ in range(2))
+    t = lambda a, d: torch.as_tensor(np.ascontiguousarray(a, d), device="cuda")  # noqa: E731
+    rpd, cid, vd = t(rp, np.int32), t(ci, np.int32), t(val, np.float64)
+    hn.check(hn.load().hn_spmv_noalloc(m, n, ci.size, rpd.data_ptr(), cid.data_ptr(), vd.data_ptr(), x.data_ptr(),
+                                       want.data_ptr(), None))
+    for _ in range(3):  # the ticket is back at zero after each
+        y.fill_(np.nan)
+        A.spmv(x, y)
+        assert torch.equal(y, want)
