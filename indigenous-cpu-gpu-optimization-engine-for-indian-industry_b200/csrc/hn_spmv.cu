@@ -6,12 +6,13 @@
 namespace hn {
 namespace {
 
-// C = op(A) B, B row-major (ncols x k). One warp per row; lanes own output
-// columns, kSpmmCols register accumulators each, nonzeros in CSR order so each
-// C entry is summed in the reference's order (gpu_backend.cpp:112-121).
+// C = op(A) B, B row-major (ncols x k), nonzeros in CSR order so each C entry
+// is summed in the reference's order (gpu_backend.cpp:112-121). Two kernels.
+// More than 64 columns: one warp per row, lanes own output columns, kSpmmCols
+// accumulators each.
 constexpr int kSpmmCols = 4;  // 32 lanes x 4 = 128 columns per pass
 
-__global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restrict__ rp,
+__global__ void __launch_bounds__(256) spmm_wide_kernel(int m, const int32_t* __restrict__ rp,
                                                    const int32_t* __restrict__ ci,
                                                    const double* __restrict__ val,
                                                    const double* __restrict__ B, int64_t k,
@@ -41,6 +42,60 @@ __global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restr
     }
 }
 
+// Up to 64 columns: G lanes per row, so that none is idle, CC columns each, and
+// the indices and values of U nonzeros loaded together before their entries of
+// B; with a warp per row, 20,000 x 50,000 with 8 per column took 22.7 us at any
+// k up to 32, now 8.3 (k = 1, 3), 10.3 (8), 12.4 (16), 16.5 (32) and 22.6 (64;
+// 26.8). At k = 100 this form takes 39 us, the wide one 33. Fewer lanes than
+// columns (CC = 2 from 17 on) read B in fewer, longer lines; more nonzeros in
+// flight than U only cost registers.
+template <int G, int CC, int U>
+__global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restrict__ rp,
+                                                   const int32_t* __restrict__ ci,
+                                                   const double* __restrict__ val,
+                                                   const double* __restrict__ B, int64_t k,
+                                                   double* __restrict__ C) {
+    const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+    const int l = threadIdx.x % G;
+    if (row >= m) return;
+    const int32_t p0 = __ldg(rp + row), p1 = __ldg(rp + row + 1);
+    for (int64_t c0 = l; c0 < k; c0 += G * CC) {
+        double acc[CC];
+#pragma unroll
+        for (int q = 0; q < CC; ++q) acc[q] = 0.0;
+        for (int32_t p = p0; p < p1; p += U) {
+            int32_t j[U];
+            double a[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                j[u] = p + u < p1 ? __ldg(ci + p + u) : 0;
+                a[u] = p + u < p1 ? __ldg(val + p + u) : 0.0;
+            }
+            double b[U][CC];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < CC; ++q)
+                    if (p + u < p1 && c0 + q * G < k) b[u][q] = __ldg(B + (int64_t)j[u] * k + c0 + q * G);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int q = 0; q < CC; ++q)
+                    if (p + u < p1 && c0 + q * G < k) acc[q] += a[u] * b[u][q];
+        }
+#pragma unroll
+        for (int q = 0; q < CC; ++q)
+            if (c0 + q * G < k) C[row * k + c0 + q * G] = acc[q];
+    }
+}
+
+template <int G, int CC, int U>
+void spmm_launch(const SpmvMat& M, const double* B, int64_t k, double* C, cudaStream_t s) {
+    const int64_t threads = (int64_t)M.m * G;
+    spmm_kernel<G, CC, U><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(M.m, M.rp, M.ci, M.val, B, k, C);
+    launched("spmm_kernel");
+}
+
 void check_handle(const hn_csr* A, int trans) {
     if (!A) fail(HN_ERR_INVALID_ARG, "null matrix handle");
     if (trans && !A->has_t) fail(HN_ERR_INVALID_ARG, "handle was created without A^T");
@@ -49,9 +104,22 @@ void check_handle(const hn_csr* A, int trans) {
 void spmm_run(const hn_csr* A, int trans, const double* B, int64_t k, double* C, cudaStream_t s) {
     const SpmvMat M = spmv_mat(A, trans);
     if (M.m == 0 || k == 0) return;
-    const int64_t threads = (int64_t)M.m * 32;
-    spmm_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(M.m, M.rp, M.ci, M.val, B, k, C);
-    launched("spmm_kernel");
+    if (k > 64) {
+        spmm_wide_kernel<<<(unsigned)(((int64_t)M.m * 32 + 255) / 256), 256, 0, s>>>(M.m, M.rp, M.ci, M.val, B, k, C);
+        launched("spmm_wide_kernel");
+    } else if (k > 32) {
+        spmm_launch<32, 2, 1>(M, B, k, C, s);
+    } else if (k > 16) {
+        spmm_launch<16, 2, 2>(M, B, k, C, s);
+    } else if (k > 8) {
+        spmm_launch<16, 1, 4>(M, B, k, C, s);
+    } else if (k > 4) {
+        spmm_launch<8, 1, 4>(M, B, k, C, s);
+    } else if (k > 2) {
+        spmm_launch<4, 1, 4>(M, B, k, C, s);
+    } else {
+        spmm_launch<2, 1, 4>(M, B, k, C, s);
+    }
 }
 
 }  // namespace

@@ -186,3 +186,26 @@ def test_spec_literal_zipf_lp_parity(hn, torch_cuda, kind, t):
     yt = run_spmv(hn, torch_cuda, A, lp["y0"], trans=1)
     rpT, ciT, valT = O.transposed(rp, ci, val, lp["n"])
     R.normwise_close(yt, O.matvec_t(rp, ci, val, lp["y0"], lp["n"]), rpT, ciT, valT, lp["y0"])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65, 130])
+@pytest.mark.parametrize("trans", [0, 1])
+def test_spmm_column_counts(hn, torch_cuda, k, trans):
+    """Every lane split of the SpMM, full and ragged: the reference's sums in
+    CSR order, bit for bit; rows of 0 to 40 entries."""
+    rng = np.random.default_rng(k)
+    m, n = 301, 257
+    rows = rng.integers(0, 41, m)
+    rp = np.concatenate([[0], np.cumsum(rows)])
+    ci = np.concatenate([np.sort(rng.choice(n, c, replace=False)) for c in rows])
+    val = rng.standard_normal(ci.size)
+    A = hn.Csr(m, n, rp, ci, val)
+    B = rng.standard_normal((m if trans else n, k))
+    out = torch_cuda.full((n if trans else m, k), np.nan, dtype=torch_cuda.float64, device="cuda")
+    A.spmm(torch_cuda.as_tensor(B, device="cuda"), k, out, trans=trans)
+    r = np.repeat(np.arange(m), rows)
+    want = np.zeros((n if trans else m, k))
+    for e in (np.argsort(ci, kind="stable") if trans else np.arange(ci.size)):
+        i, j = (ci[e], r[e]) if trans else (r[e], ci[e])
+        want[i] += val[e] * B[j]
+    assert np.array_equal(out.cpu().numpy(), want)
