@@ -54,6 +54,7 @@ __global__ void ada_window_kernel(int m, const int32_t* __restrict__ rp, const i
                                   const double* __restrict__ val, const int32_t* __restrict__ rpT,
                                   const int32_t* __restrict__ ciT, int32_t* __restrict__ wbase,
                                   int32_t* __restrict__ wcount, unsigned* __restrict__ wmax) {
+    if (!after_previous()) return;
     const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= m) return;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(kT) ada_count_kernel(int m, const int32_t* __r
                                                        int64_t* __restrict__ len, int64_t* __restrict__ nq,
                                                        int64_t* __restrict__ nms, int64_t* __restrict__ nmq,
                                                        unsigned* __restrict__ maxes) {
+    if (!after_previous()) return;
     extern __shared__ uint32_t smem[];
     uint32_t* b1 = smem;
     uint32_t* b2 = smem + Wmax;
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kT) ada_fill_kernel(
     int64_t* __restrict__ mpos, int32_t* mcnt, int32_t* __restrict__ mbeg, uint2* __restrict__ gmap,
     uint2* __restrict__ mlist, const int64_t* __restrict__ tq, uint16_t* __restrict__ smap,
     uint32_t* __restrict__ rmap, int qbits) {
+    if (!after_previous()) return;
     extern __shared__ uint32_t smem[];
     uint32_t* b1 = smem;
     uint32_t* b2 = smem + Wmax;
@@ -279,6 +282,7 @@ __global__ void __launch_bounds__(kT) ada_fill_kernel(
 // a value load plus a dependent column-index -> d chain.
 __global__ void ada_vd_kernel(int64_t nnz, const double* __restrict__ val, const int32_t* __restrict__ ci,
                               const double* __restrict__ d, double2* __restrict__ vd) {
+    if (!after_previous()) return;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x)
         vd[e] = make_double2(val[e], __ldg(d + ci[e]));
 }
@@ -297,6 +301,7 @@ __global__ void __launch_bounds__(kT, 4) ada_slot_kernel(int64_t nnz, const uint
                                                          const double2* __restrict__ vd,
                                                          const double* __restrict__ valT,
                                                          const double* __restrict__ mval, double* __restrict__ nval) {
+    if (!after_previous()) return;
     const int64_t stride = (int64_t)gridDim.x * kT * kSlotsPerThread;
     int64_t t0 = blockIdx.x * (int64_t)kT * kSlotsPerThread + threadIdx.x;
     uint2 g[kSlotsPerThread];
@@ -363,6 +368,7 @@ __global__ void __launch_bounds__(kRmapT, 3) ada_rmap_kernel(int m, const int32_
                                                              const uint32_t* __restrict__ rmap, int qbits,
                                                              const double* __restrict__ mval,
                                                              double* __restrict__ nval) {
+    if (!after_previous()) return;
     __shared__ double2 s_q[kRmapT / 32][kRmapTerms];
     __shared__ int32_t s_cs[kRmapT / 32][kRmapTerms];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -433,6 +439,7 @@ __global__ void __launch_bounds__(kRmapT, 3) ada_rmap_kernel(int m, const int32_
 
 __global__ void ada_ecs_kernel(int64_t nnz, const int32_t* __restrict__ ci, const int32_t* __restrict__ rpT,
                                int32_t* __restrict__ ecs) {
+    if (!after_previous()) return;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x)
         ecs[e] = rpT[ci[e]];
 }
@@ -464,6 +471,7 @@ __global__ void ada_combine_kernel(int64_t nms, const int64_t* __restrict__ mpos
                                    const uint2* __restrict__ mlist, const double2* __restrict__ vd,
                                    const double* __restrict__ valT, double* __restrict__ mval,
                                    unsigned long long* maxdiag) {
+    if (!after_previous()) return;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nms) return;
     const int32_t u0 = mbeg[t], u1 = mbeg[t + 1];
@@ -495,6 +503,7 @@ __global__ void __launch_bounds__(kRowThreads, 3) ada_row_kernel(
     const int32_t* __restrict__ rpT, const double* __restrict__ valT, const int64_t* __restrict__ tq,
     const uint16_t* __restrict__ smap, const int64_t* __restrict__ rpN, const int64_t* __restrict__ msrow,
     const int64_t* __restrict__ mpos, const double* __restrict__ mval, double* __restrict__ nval) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) double row_smem[];
     double* srow = row_smem;
     double2* s_vd = reinterpret_cast<double2*>(row_smem + kRowWindow);
@@ -562,6 +571,7 @@ __global__ void __launch_bounds__(kRowThreads, 3) ada_row_kernel(
 
 // term counts of a row rounded up to whole 16-byte chunks of the slot map
 __global__ void pad8_kernel(int64_t m, const int64_t* __restrict__ nq, int64_t* __restrict__ out) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < m) out[i] = (nq[i] + 7) & ~int64_t(7);
 }
@@ -569,6 +579,7 @@ __global__ void pad8_kernel(int64_t m, const int64_t* __restrict__ nq, int64_t* 
 __global__ void ada_reg_kernel(int m, const int64_t* __restrict__ diag_pos, double reg,
                                const unsigned long long* __restrict__ maxdiag, double* __restrict__ nval,
                                double* dyn_out) {
+    if (!after_previous()) return;
     const double md = __longlong_as_double(static_cast<long long>(*maxdiag));
     double dyn = 1e-12 * md;
     dyn = (reg < dyn) ? dyn : reg;  // std::max(regularization, 1e-12 * max_diag)
@@ -598,13 +609,13 @@ void launch_numeric(const hn_pattern* P, const double* d, double* nval, cudaStre
     const hn_csr* A = P->A;
     if (A->nnz > 0) {
         const int gv = (int)std::min<int64_t>((A->nnz + kT - 1) / kT, (int64_t)ctx().sm_count * 16);
-        ada_vd_kernel<<<gv, kT, 0, s>>>(A->nnz, A->val, A->ci, d, P->vd);
+        launch_next(ada_vd_kernel, gv, kT, 0, s, A->nnz, A->val, A->ci, d, P->vd);
         launched("ada_vd_kernel");
     }
     check_cuda(cudaMemsetAsync(P->maxdiag, 0, sizeof(unsigned long long), s), "memset maxdiag");
     if (P->nms > 0) {
-        ada_combine_kernel<<<(unsigned)((P->nms + 255) / 256), 256, 0, s>>>(P->nms, P->mpos, P->mbeg, P->mlist,
-                                                                            P->vd, A->valT, P->mval, P->maxdiag);
+        launch_next(ada_combine_kernel, (unsigned)((P->nms + 255) / 256), 256, 0, s, P->nms, P->mpos, P->mbeg,
+                    P->mlist, P->vd, A->valT, P->mval, P->maxdiag);
         launched("ada_combine_kernel");
     }
     if (P->row_mode) {
@@ -616,23 +627,23 @@ void launch_numeric(const hn_pattern* P, const double* d, double* nval, cudaStre
             row_attr_device = ctx().device;
         }
         const int grid = (int)std::min<int64_t>(P->m, (int64_t)ctx().sm_count * 3);
-        ada_row_kernel<<<grid, kRowThreads, kRowSmem, s>>>((int)P->m, A->rp, A->ci, P->vd, A->rpT, A->valT, P->tq,
-                                                       P->smap, P->rp, P->msrow, P->mpos, P->mval, nval);
+        launch_next(ada_row_kernel, grid, kRowThreads, kRowSmem, s, (int)P->m, A->rp, A->ci, P->vd, A->rpT, A->valT,
+                    P->tq, P->smap, P->rp, P->msrow, P->mpos, P->mval, nval);
         launched("ada_row_kernel");
         return;
     }
     if (P->rmap) {
         check_cuda(cudaMemsetAsync(P->row_next, 0, sizeof(unsigned), s), "memset row counter");
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P->m + 7) / 8, (int64_t)ctx().sm_count * 3));
-        ada_rmap_kernel<<<grid, kRmapT, 0, s>>>((int)P->m, P->order, P->row_next, A->rp, P->vd, P->ecs, A->valT,
-                                                A->nnz, P->rp, P->msrow, P->nms, P->rmap, P->qbits, P->mval, nval);
+        launch_next(ada_rmap_kernel, grid, kRmapT, 0, s, (int)P->m, P->order, P->row_next, A->rp, P->vd, P->ecs,
+                    A->valT, A->nnz, P->rp, P->msrow, P->nms, P->rmap, P->qbits, P->mval, nval);
         launched("ada_rmap_kernel");
         return;
     }
     const int64_t per_block = (int64_t)kT * kSlotsPerThread;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P->nnz + per_block - 1) / per_block,
                                                                  (int64_t)ctx().sm_count * 4));
-    ada_slot_kernel<<<grid, kT, 0, s>>>(P->nnz, P->gmap, P->vd, A->valT, P->mval, nval);
+    launch_next(ada_slot_kernel, grid, kT, 0, s, P->nnz, P->gmap, P->vd, A->valT, P->mval, nval);
     launched("ada_slot_kernel");
 }
 
@@ -678,9 +689,8 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
             wmax_d = dmalloc<unsigned>(3);  // widest bitmap, longest row of N, longest row of A
             check_cuda(cudaMemsetAsync(wmax_d, 0, 3 * sizeof(unsigned), s), "memset");
             if (m > 0) {
-                ada_window_kernel<<<(unsigned)((m * 32 + 255) / 256), 256, 0, s>>>((int)m, A->rp, A->ci, A->val,
-                                                                                  A->rpT, A->ciT, wbase, wcount,
-                                                                                  wmax_d);
+                launch_next(ada_window_kernel, (unsigned)((m * 32 + 255) / 256), 256, 0, s, (int)m, A->rp, A->ci,
+                            A->val, A->rpT, A->ciT, wbase, wcount, wmax_d);
                 launched("ada_window_kernel");
             }
             unsigned wmax_h = 0;
@@ -711,14 +721,14 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
                        "smem attribute");
             const int grid = (int)std::min<int64_t>(std::max<int64_t>(m, 1), (int64_t)ctx().sm_count * 8);
             if (m > 0) {
-                ada_count_kernel<<<grid, kT, smem_count, s>>>((int)m, A->rp, A->ci, A->val, A->rpT, A->ciT, (int)W,
-                                                              wbase, wcount, P->rp, nq, nms, nmq, wmax_d);
+                launch_next(ada_count_kernel, grid, kT, smem_count, s, (int)m, A->rp, A->ci, A->val, A->rpT, A->ciT,
+                            (int)W, wbase, wcount, P->rp, nq, nms, nmq, wmax_d);
                 launched("ada_count_kernel");
             }
             tqa = dmalloc<int64_t>(m + 1);
             check_cuda(cudaMemsetAsync(tqa, 0, sizeof(int64_t) * (m + 1), s), "memset");
             if (m > 0) {
-                pad8_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, nq, tqa);
+                launch_next(pad8_kernel, (unsigned)((m + 255) / 256), 256, 0, s, m, nq, tqa);
                 launched("pad8_kernel");
             }
             scan_exclusive_i64(tqa, tqa, m + 1, s);
@@ -773,7 +783,7 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
                 nms = nullptr;  // owned by the pattern now
                 if (A->nnz > 0) {
                     const int ge = (int)std::min<int64_t>((A->nnz + kT - 1) / kT, (int64_t)ctx().sm_count * 16);
-                    ada_ecs_kernel<<<ge, kT, 0, s>>>(A->nnz, A->ci, A->rpT, P->ecs);
+                    launch_next(ada_ecs_kernel, ge, kT, 0, s, A->nnz, A->ci, A->rpT, P->ecs);
                     launched("ada_ecs_kernel");
                 }
                 // rows of N longest first: the counter hands the long rows out early
@@ -797,10 +807,9 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
             const int32_t last = static_cast<int32_t>(P->nmq);
             check_cuda(cudaMemcpyAsync(P->mbeg + P->nms, &last, sizeof(last), cudaMemcpyHostToDevice, s), "H2D");
             if (m > 0) {
-                ada_fill_kernel<<<grid, kT, smem_fill, s>>>((int)m, A->rp, A->ci, A->val, A->rpT, A->ciT, (int)W,
-                                                            wbase, wcount, P->rp, P->msrow ? P->msrow : nms, nmq,
-                                                            P->ci, P->diag_pos, P->mpos, mcnt, P->mbeg, P->gmap,
-                                                            P->mlist, P->tq, P->smap, P->rmap, P->qbits);
+                launch_next(ada_fill_kernel, grid, kT, smem_fill, s, (int)m, A->rp, A->ci, A->val, A->rpT, A->ciT,
+                            (int)W, wbase, wcount, P->rp, P->msrow ? P->msrow : nms, nmq, P->ci, P->diag_pos, P->mpos,
+                            mcnt, P->mbeg, P->gmap, P->mlist, P->tq, P->smap, P->rmap, P->qbits);
                 launched("ada_fill_kernel");
             }
             check_cuda(cudaStreamSynchronize(s), "symbolic sync");
@@ -859,8 +868,8 @@ int hn_ada_numeric(const hn_pattern* P, const double* d, double reg, double* nva
         cudaStream_t s = as_stream(stream);
         if (P->m == 0) return;
         launch_numeric(P, d, nval, s);
-        ada_reg_kernel<<<(unsigned)((P->m + 255) / 256), 256, 0, s>>>((int)P->m, P->diag_pos, reg, P->maxdiag,
-                                                                      nval, dyn_out);
+        launch_next(ada_reg_kernel, (unsigned)((P->m + 255) / 256), 256, 0, s, (int)P->m, P->diag_pos, reg,
+                    P->maxdiag, nval, dyn_out);
         launched("ada_reg_kernel");
     });
 }

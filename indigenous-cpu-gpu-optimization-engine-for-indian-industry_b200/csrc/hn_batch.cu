@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(kT) batch_prep_kernel(const int64_t* __restric
                                                         double* __restrict__ scal, int32_t* __restrict__ status,
                                                         int32_t* __restrict__ iters, int iter, double tol,
                                                         double ctol, KktArgs k) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ int s_save;
     const int64_t i = blockIdx.x;
@@ -236,6 +237,7 @@ __global__ void __launch_bounds__(kT) batch_finish_kernel(const int64_t* __restr
                                                           double* __restrict__ z, double* __restrict__ lam,
                                                           int32_t* __restrict__ status, int32_t* __restrict__ iters,
                                                           KktArgs k) {
+    if (!after_previous()) return;
     __shared__ int s_restore;
     const int64_t i = blockIdx.x;
     const int r = k.ref_iter[i];
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(kT) batch_steps_kernel(const int64_t* __restri
                                                          const double* __restrict__ z, const double* __restrict__ dz,
                                                          const double* __restrict__ dlam, double* __restrict__ scal,
                                                          int32_t* __restrict__ status) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ int s_bad;
     const int64_t i = blockIdx.x;
@@ -301,6 +304,7 @@ __global__ void __launch_bounds__(kT) batch_corr_kernel(const int64_t* __restric
                                                         const double* __restrict__ z, const double* __restrict__ dz,
                                                         double* __restrict__ scal, const int32_t* __restrict__ status,
                                                         double* __restrict__ zs) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ double s_sm;
     const int64_t i = blockIdx.x;
@@ -344,6 +348,7 @@ __global__ void __launch_bounds__(kT) batch_update_kernel(const int64_t* __restr
                                                           const double* __restrict__ scal,
                                                           int32_t* __restrict__ status, int32_t* __restrict__ iters,
                                                           int iter) {
+    if (!after_previous()) return;
     __shared__ int s_bad;
     const int64_t i = blockIdx.x;
     if (status[i] != ST_RUN) return;
@@ -374,6 +379,7 @@ __global__ void __launch_bounds__(kT) batch_update_kernel(const int64_t* __restr
 __global__ void __launch_bounds__(kT) batch_reg_kernel(const int64_t* __restrict__ row_off,
                                                        const int64_t* __restrict__ diag_pos, double reg,
                                                        const int32_t* __restrict__ status, double* __restrict__ nval) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ double s_dyn;
     const int64_t i = blockIdx.x;
@@ -396,6 +402,7 @@ __global__ void batch_dense_kernel(int64_t m, const int64_t* __restrict__ row_of
                                    const int64_t* __restrict__ dn_off, const int32_t* __restrict__ status,
                                    const int64_t* __restrict__ rpN, const int32_t* __restrict__ ciN,
                                    const double* __restrict__ nval, double* __restrict__ dense) {
+    if (!after_previous()) return;
     const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (r >= m) return;
@@ -601,6 +608,7 @@ __global__ void __launch_bounds__(kT) batch_ldlt_diag_kernel(int s, const InstIn
                                                              const int32_t* __restrict__ status,
                                                              double* __restrict__ dense, double* __restrict__ dD,
                                                              double tol) {
+    if (!after_previous()) return;
     __shared__ DiagShared sh;
     const int tid = threadIdx.x;
     const int inst = order[blockIdx.x];
@@ -687,6 +695,7 @@ __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, con
                                                                       const InstInfo* __restrict__ info,
                                                                       const int32_t* __restrict__ status, double* dense,
                                                                       const double* __restrict__ dD) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) double panel_sm[];
     double(*sLt)[kPanelP] = reinterpret_cast<double(*)[kPanelP]>(panel_sm);  // sLt[q][c] = L[k0 + c, k0 + q]
     double* sD = panel_sm + kFb * kPanelP;
@@ -838,6 +847,7 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
                                                                   const int32_t* __restrict__ status,
                                                                   double* __restrict__ dense,
                                                                   const double* __restrict__ dD) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) double upd_smem[];
     __shared__ UpdTile s_tile[kUpdStages];
     double* sC = upd_smem + kUpdStages * kUpdStage;
@@ -1112,6 +1122,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
                        const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
                        const double* __restrict__ dense, const double* __restrict__ dD, double* work, double* part,
                        double* xv) {
+    if (!after_previous()) return;
     extern __shared__ __align__(16) double solve_smem[];
     double(*sLb)[kFb][kSolveP] = reinterpret_cast<double(*)[kFb][kSolveP]>(solve_smem);  // two diagonal blocks
     double* s_x = solve_smem + 2 * kFb * kSolveP;  // a single CTA's instance: right-hand side, y / D, solution
@@ -1339,6 +1350,7 @@ __global__ void __launch_bounds__(kT) batch_refine_check_kernel(const int64_t* _
                                                                 const double* __restrict__ rhs,
                                                                 const double* __restrict__ ax, double* __restrict__ r,
                                                                 int32_t* __restrict__ refine, int32_t* nref) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     const int64_t i = blockIdx.x;
     if (status[i] != ST_RUN || !refine[i]) return;
@@ -1363,6 +1375,7 @@ __global__ void __launch_bounds__(kT) batch_refine_start_kernel(const int64_t* _
                                                                 const int32_t* __restrict__ status,
                                                                 const double* __restrict__ rhs,
                                                                 int32_t* __restrict__ refine) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     const int64_t i = blockIdx.x;
     const int64_t r0 = row_off[i], r1 = row_off[i + 1];
@@ -1383,6 +1396,7 @@ __global__ void __launch_bounds__(kT) batch_refine_start_kernel(const int64_t* _
 __global__ void batch_axpy_masked_kernel(int64_t m, const int32_t* __restrict__ row_inst,
                                          const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
                                          const double* __restrict__ r, double* __restrict__ x) {
+    if (!after_previous()) return;
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= m) return;
     const int inst = row_inst[k];
@@ -1390,11 +1404,13 @@ __global__ void batch_axpy_masked_kernel(int64_t m, const int32_t* __restrict__ 
 }
 
 __global__ void row_inst_kernel(int64_t K, const int64_t* __restrict__ row_off, int32_t* __restrict__ row_inst) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x;
     for (int64_t r = row_off[i] + threadIdx.x; r < row_off[i + 1]; r += blockDim.x) row_inst[r] = (int32_t)i;
 }
 
 __global__ void narrow_rp_kernel(int64_t n, const int64_t* __restrict__ in, int32_t* __restrict__ out) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) out[i] = static_cast<int32_t>(in[i]);
 }
@@ -1426,8 +1442,8 @@ SpmvMat n_mat(const hn_batch* B, const double* nval) {
 
 // x holds the right-hand sides of the taking-part instances on entry, their solutions on return.
 void solve_all(hn_batch* B, const int32_t* status, const int32_t* refine, double* x, cudaStream_t s) {
-    batch_solve_kernel<<<(unsigned)B->nslots, kT, (size_t)B->solve_smem, s>>>(B->slots, B->info, status, refine, B->dense,
-                                                          B->dD, B->work, B->solve_part, x);
+    launch_next(batch_solve_kernel, (unsigned)B->nslots, kT, (size_t)B->solve_smem, s, B->slots, B->info, status,
+                refine, B->dense, B->dD, B->work, B->solve_part, x);
     launched("batch_solve_kernel");
 }
 
@@ -1495,9 +1511,9 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             check_cuda(cudaMemcpy(B->col_off, col_off_host, sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice), "H2D");
             check_cuda(cudaMemcpy(B->dn_off, dn.data(), sizeof(int64_t) * (K + 1), cudaMemcpyHostToDevice), "H2D");
             check_cuda(cudaMemcpy(B->order, order.data(), sizeof(int32_t) * K, cudaMemcpyHostToDevice), "H2D");
-            row_inst_kernel<<<(unsigned)K, 256, 0, s>>>(K, B->row_off, B->row_inst);
+            launch_next(row_inst_kernel, (unsigned)K, 256, 0, s, K, B->row_off, B->row_inst);
             launched("row_inst_kernel");
-            narrow_rp_kernel<<<(unsigned)((m + 1 + 255) / 256), 256, 0, s>>>(m + 1, P->rp, B->nrp);
+            launch_next(narrow_rp_kernel, (unsigned)((m + 1 + 255) / 256), 256, 0, s, m + 1, P->rp, B->nrp);
             launched("narrow_rp_kernel");
             make_tile_table(B->nrp, m, P->nnz, &B->ntiles, &B->tile_row, &B->tile_nz, &B->carry_row, &B->carry_val,
                             &B->head_row, &B->head_val, &B->short_heads, s);
@@ -1604,8 +1620,8 @@ int hn_batch_residuals(hn_batch* B, const hn_csr* M, const double* x, const doub
         if (!B || !M || !M->has_t) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
         spmv_launch2(spmv_mat(M, 0), x, EpiResidual{b, mx, rp}, spmv_mat(M, 1), lam, EpiDualResidual{z, c, rd}, s);
-        batch_prep_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->col_off, x, z, rd, rp, D, Drd, scal, status,
-                                                        iters, iter, tol, ctol, kkt_args(B, lam, b, c));
+        launch_next(batch_prep_kernel, (unsigned)B->K, kT, 0, s, B->row_off, B->col_off, x, z, rd, rp, D, Drd, scal,
+                    status, iters, iter, tol, ctol, kkt_args(B, lam, b, c));
         launched("batch_prep_kernel");
     });
 }
@@ -1651,8 +1667,8 @@ int hn_batch_finish(hn_batch* B, double* x, double* z, double* lam, int32_t* sta
         require_init();
         if (!B || !x || !z || !lam || !status || !iters) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
-        batch_finish_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->col_off, x, z, lam, status, iters,
-                                                          kkt_args(B, lam, nullptr, nullptr));
+        launch_next(batch_finish_kernel, (unsigned)B->K, kT, 0, s, B->row_off, B->col_off, x, z, lam, status, iters,
+                    kkt_args(B, lam, nullptr, nullptr));
         launched("batch_finish_kernel");
     });
 }
@@ -1664,32 +1680,33 @@ int hn_batch_factor(hn_batch* B, const double* D, double reg, double singular_to
         if (!B || !D || !nval || !status) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
         ada_numeric_unregularised(B->P, D, nval, s);
-        batch_reg_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->P->diag_pos, reg, status, nval);
+        launch_next(batch_reg_kernel, (unsigned)B->K, kT, 0, s, B->row_off, B->P->diag_pos, reg, status, nval);
         launched("batch_reg_kernel");
-        batch_dense_kernel<<<(unsigned)((B->m * 32 + 255) / 256), 256, 0, s>>>(
-            B->m, B->row_off, B->row_inst, B->dn_off, status, B->P->rp, B->P->ci, nval, B->dense);
+        launch_next(batch_dense_kernel, (unsigned)((B->m * 32 + 255) / 256), 256, 0, s, B->m, B->row_off, B->row_inst,
+                    B->dn_off, status, B->P->rp, B->P->ci, nval, B->dense);
         launched("batch_dense_kernel");
         // steps in pairs: after an even step only the next block column is
         // brought up to date, after an odd one the rest, by both panels at once
         for (int64_t st = 0; st < B->nsteps; ++st) {
             const int cnt = B->step_cnt[st];
-            batch_ldlt_diag_kernel<<<cnt, kT, 0, s>>>((int)st, B->info, B->order, status, B->dense, B->dD, singular_tol);
+            launch_next(batch_ldlt_diag_kernel, cnt, kT, 0, s, (int)st, B->info, B->order, status, B->dense, B->dD,
+                        singular_tol);
             launched("batch_ldlt_diag_kernel");
             const int64_t nc = B->chunk_off_h[st + 1] - B->chunk_off_h[st];
             if (nc == 0) continue;
-            batch_ldlt_panel_kernel<<<(unsigned)(nc * (kT / kPanelT)), kPanelT, kPanelSmem, s>>>(
-                (int)st, B->chunks + B->chunk_off_h[st], B->info, status, B->dense, B->dD);
+            launch_next(batch_ldlt_panel_kernel, (unsigned)(nc * (kT / kPanelT)), kPanelT, kPanelSmem, s, (int)st,
+                        B->chunks + B->chunk_off_h[st], B->info, status, B->dense, B->dD);
             launched("batch_ldlt_panel_kernel");
             const int64_t nt = B->step_tiles_h[st];
             const unsigned grid = (unsigned)std::min<int64_t>(nt, 2 * (int64_t)ctx().sm_count);
             const int kt = (int)(st + 1) * kFb;
             const int64_t* tiles = B->step_tiles + B->tile_off_h[st];
             if (st % 2 == 0)
-                batch_ldlt_update_kernel<1><<<grid, kUpdT, kUpdSmem, s>>>(kt - kFb, kt, 1, cnt, nt, tiles, B->info,
-                                                                          B->order, status, B->dense, B->dD);
+                launch_next(batch_ldlt_update_kernel<1>, grid, kUpdT, kUpdSmem, s, kt - kFb, kt, 1, cnt, nt, tiles,
+                            B->info, B->order, status, B->dense, B->dD);
             else
-                batch_ldlt_update_kernel<2><<<grid, kUpdT, kUpdSmem, s>>>(kt - 2 * kFb, kt, 0, cnt, nt, tiles, B->info,
-                                                                          B->order, status, B->dense, B->dD);
+                launch_next(batch_ldlt_update_kernel<2>, grid, kUpdT, kUpdSmem, s, kt - 2 * kFb, kt, 0, cnt, nt,
+                            tiles, B->info, B->order, status, B->dense, B->dD);
             launched("batch_ldlt_update_kernel");
         }
     });
@@ -1703,22 +1720,22 @@ int hn_batch_solve(hn_batch* B, const double* nval, const double* rhs, double* x
         cudaStream_t s = as_stream(stream);
         check_cuda(cudaMemcpyAsync(x, rhs, sizeof(double) * B->m, cudaMemcpyDeviceToDevice, s), "copy rhs");
         solve_all(B, status, nullptr, x, s);
-        batch_refine_start_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, status, rhs, B->refine);
+        launch_next(batch_refine_start_kernel, (unsigned)B->K, kT, 0, s, B->row_off, status, rhs, B->refine);
         launched("batch_refine_start_kernel");
         const SpmvMat N = n_mat(B, nval);
         for (int sweep = 0; sweep < 5; ++sweep) {
             spmv_launch(N, x, EpiAxpby{1.0, 0.0, B->ax}, s);
             check_cuda(cudaMemsetAsync(B->nref, 0, sizeof(int32_t), s), "memset");
-            batch_refine_check_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, status, rhs, B->ax, B->r, B->refine,
-                                                                    B->nref);
+            launch_next(batch_refine_check_kernel, (unsigned)B->K, kT, 0, s, B->row_off, status, rhs, B->ax, B->r,
+                        B->refine, B->nref);
             launched("batch_refine_check_kernel");
             int32_t left = 0;
             check_cuda(cudaMemcpyAsync(&left, B->nref, sizeof(left), cudaMemcpyDeviceToHost, s), "D2H");
             check_cuda(cudaStreamSynchronize(s), "refine sync");
             if (left == 0) break;
             solve_all(B, status, B->refine, B->r, s);
-            batch_axpy_masked_kernel<<<(unsigned)((B->m + 255) / 256), 256, 0, s>>>(B->m, B->row_inst, status,
-                                                                                    B->refine, B->r, x);
+            launch_next(batch_axpy_masked_kernel, (unsigned)((B->m + 255) / 256), 256, 0, s, B->m, B->row_inst,
+                        status, B->refine, B->r, x);
             launched("batch_axpy_masked_kernel");
         }
     });
@@ -1730,7 +1747,8 @@ int hn_batch_steps(hn_batch* B, const double* x, const double* dx, const double*
         require_init();
         if (!B) fail(HN_ERR_INVALID_ARG, "null batch");
         cudaStream_t s = as_stream(stream);
-        batch_steps_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->col_off, x, dx, z, dz, dlam, scal, status);
+        launch_next(batch_steps_kernel, (unsigned)B->K, kT, 0, s, B->row_off, B->col_off, x, dx, z, dz, dlam, scal,
+                    status);
         launched("batch_steps_kernel");
     });
 }
@@ -1742,7 +1760,7 @@ int hn_batch_corrector(hn_batch* B, const hn_csr* M, const double* x, const doub
         require_init();
         if (!B || !M) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
-        batch_corr_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->col_off, x, dx, z, dz, scal, status, zs);
+        launch_next(batch_corr_kernel, (unsigned)B->K, kT, 0, s, B->col_off, x, dx, z, dz, scal, status, zs);
         launched("batch_corr_kernel");
         spmv_launch(spmv_mat(M, 0), zs, EpiCorrRhs{rhs_pred, rhs}, s);
     });
@@ -1755,8 +1773,8 @@ int hn_batch_update(hn_batch* B, double* x, const double* dx, double* z, const d
         require_init();
         if (!B) fail(HN_ERR_INVALID_ARG, "null batch");
         cudaStream_t s = as_stream(stream);
-        batch_update_kernel<<<(unsigned)B->K, kT, 0, s>>>(B->row_off, B->col_off, x, dx, z, dz, lam, dlam, scal,
-                                                          status, iters, iter);
+        launch_next(batch_update_kernel, (unsigned)B->K, kT, 0, s, B->row_off, B->col_off, x, dx, z, dz, lam, dlam,
+                    scal, status, iters, iter);
         launched("batch_update_kernel");
     });
 }

@@ -179,6 +179,7 @@ constexpr int64_t kScanTile = kScanThreads * kScanItems;
 template <class T>
 __global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const T* in, T* out, int64_t n,
                                                                   int64_t* tile_sums) {
+    if (!after_previous()) return;
     __shared__ int64_t sh[32];
     const int64_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     int64_t v[kScanItems];
@@ -200,6 +201,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(const T* in, T*
 
 template <class T>
 __global__ void scan_add_kernel(T* out, int64_t n, const int64_t* tile_offsets) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) out[i] += static_cast<T>(tile_offsets[i / kScanTile]);
 }
@@ -209,15 +211,15 @@ void scan_exclusive_impl(const T* in, T* out, int64_t n, cudaStream_t s) {
     if (n <= 0) return;
     const int64_t tiles = (n + kScanTile - 1) / kScanTile;
     if (tiles == 1) {
-        scan_tile_kernel<T><<<1, kScanThreads, 0, s>>>(in, out, n, nullptr);
+        launch_next(scan_tile_kernel<T>, 1, kScanThreads, 0, s, in, out, n, nullptr);
         launched("scan_tile_kernel");
         return;
     }
     int64_t* sums = dmalloc<int64_t>(tiles);
-    scan_tile_kernel<T><<<(unsigned)tiles, kScanThreads, 0, s>>>(in, out, n, sums);
+    launch_next(scan_tile_kernel<T>, (unsigned)tiles, kScanThreads, 0, s, in, out, n, sums);
     launched("scan_tile_kernel");
     scan_exclusive_impl<int64_t>(sums, sums, tiles, s);
-    scan_add_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, n, sums);
+    launch_next(scan_add_kernel<T>, (unsigned)((n + 255) / 256), 256, 0, s, out, n, sums);
     launched("scan_add_kernel");
     check_cuda(cudaStreamSynchronize(s), "scan sync");
     dfree(sums);
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(int64_t n, const do
                                                              const double* __restrict__ b,
                                                              double* partials, unsigned* counter,
                                                              double* out) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ bool last;
     double acc = 0.0;
@@ -279,6 +282,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_kernel(int64_t n, const do
 
 __global__ void axpy_kernel(int64_t n, double alpha, const double* __restrict__ x,
                             double* __restrict__ y) {
+    if (!after_previous()) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
         y[i] += alpha * x[i];
@@ -288,7 +292,7 @@ template <int OP>
 void run_reduce(int64_t n, const double* a, const double* b, double* out, cudaStream_t s) {
     Workspace& w = workspace(s);
     const int grid = grid_for(n, kRedThreads * 4, kMaxReduceBlocks);
-    reduce_kernel<OP><<<grid, kRedThreads, 0, s>>>(n, a, b, w.partials, w.counter, out);
+    launch_next(reduce_kernel<OP>, grid, kRedThreads, 0, s, n, a, b, w.partials, w.counter, out);
     launched("reduce_kernel");
 }
 }  // namespace
@@ -456,8 +460,7 @@ int hn_axpy(int64_t n, double alpha, const double* x, double* y, void* stream) {
         require_init();
         if (n < 0 || (n > 0 && (!x || !y))) fail(HN_ERR_INVALID_ARG, "bad arguments");
         if (n == 0) return;
-        axpy_kernel<<<grid_for(n, 256, ctx().sm_count * 16), 256, 0, as_stream(stream)>>>(n, alpha,
-                                                                                       x, y);
+        launch_next(axpy_kernel, grid_for(n, 256, ctx().sm_count * 16), 256, 0, as_stream(stream), n, alpha, x, y);
         launched("axpy_kernel");
     });
 }

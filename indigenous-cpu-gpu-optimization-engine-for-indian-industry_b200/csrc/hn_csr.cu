@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_upsweep(const int32_t* __r
                                                               int64_t n, int shift,
                                                               int32_t* __restrict__ counts,
                                                               int64_t ntiles) {
+    if (!after_previous()) return;
     __shared__ int hist[kRadix];
     if (threadIdx.x < kRadix) hist[threadIdx.x] = 0;
     __syncthreads();
@@ -44,6 +45,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
     const int32_t* __restrict__ kin, const int32_t* __restrict__ vin, int32_t* __restrict__ kout,
     int32_t* __restrict__ vout, int64_t n, int shift, const int32_t* __restrict__ offsets,
     int64_t ntiles) {
+    if (!after_previous()) return;
     __shared__ int32_t s_cnt[kRadix * kSortThreads];  // digit-major, thread-minor
     __shared__ int64_t s_scan[32];
     const int t = threadIdx.x;
@@ -102,12 +104,14 @@ __global__ void __launch_bounds__(kSortThreads) radix_downsweep(
 }
 
 __global__ void iota_kernel(int32_t* p, int64_t n) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) p[i] = static_cast<int32_t>(i);
 }
 
 // One warp per row writes the row id over the row's nonzeros.
 __global__ void row_of_kernel(const int32_t* __restrict__ rp, int64_t m, int32_t* __restrict__ row_of) {
+    if (!after_previous()) return;
     const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= m) return;
@@ -117,6 +121,7 @@ __global__ void row_of_kernel(const int32_t* __restrict__ rp, int64_t m, int32_t
 __global__ void gather_t_kernel(int64_t nnz, const int32_t* __restrict__ perm,
                                 const int32_t* __restrict__ row_of, const double* __restrict__ val,
                                 int32_t* __restrict__ ci_raw, double* __restrict__ val_raw) {
+    if (!after_previous()) return;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= nnz) return;
     const int32_t k = perm[p];
@@ -128,6 +133,7 @@ __global__ void gather_t_kernel(int64_t nnz, const int32_t* __restrict__ perm,
 __global__ void runs_kernel(int64_t nnz, const int32_t* __restrict__ key,
                             const int32_t* __restrict__ ci_raw, const double* __restrict__ val_raw,
                             double* __restrict__ run_sum, int32_t* __restrict__ keep) {
+    if (!after_previous()) return;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= nnz) return;
     const bool head = (p == 0) || key[p - 1] != key[p] || ci_raw[p - 1] != ci_raw[p];
@@ -146,6 +152,7 @@ __global__ void compact_kernel(int64_t nnz, const int32_t* __restrict__ keep,
                                const int32_t* __restrict__ ci_raw, const double* __restrict__ run_sum,
                                int32_t* __restrict__ ciT, double* __restrict__ valT,
                                int32_t* __restrict__ keyT) {
+    if (!after_previous()) return;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= nnz || !keep[p]) return;
     const int32_t q = pos[p];
@@ -155,11 +162,13 @@ __global__ void compact_kernel(int64_t nnz, const int32_t* __restrict__ keep,
 }
 
 __global__ void histogram_kernel(int64_t n, const int32_t* __restrict__ key, int32_t* __restrict__ cnt) {
+    if (!after_previous()) return;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p < n) atomicAdd(&cnt[key[p]], 1);
 }
 
 __global__ void sum_i32_kernel(int64_t n, const int32_t* __restrict__ v, unsigned long long* out) {
+    if (!after_previous()) return;
     __shared__ int64_t sh[32];
     int64_t acc = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -174,6 +183,7 @@ __global__ void sum_i32_kernel(int64_t n, const int32_t* __restrict__ v, unsigne
 __global__ void tiles_kernel(const int32_t* __restrict__ rp, int64_t m, int64_t nnz, int64_t items,
                              int64_t ntiles, int32_t* __restrict__ tile_row,
                              int32_t* __restrict__ tile_nz) {
+    if (!after_previous()) return;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t > ntiles) return;
     int64_t diag = t * items;
@@ -196,6 +206,7 @@ inline unsigned blocks(int64_t n, int t = 256) { return static_cast<unsigned>((n
 // The longest part of a row that lies before the start of the tile it reaches into.
 __global__ void longest_head_kernel(const int32_t* __restrict__ rp, int64_t m, int64_t nnz, int64_t ntiles,
                                     const int32_t* __restrict__ trow, const int32_t* __restrict__ tnz, int* longest) {
+    if (!after_previous()) return;
     int len = 0;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < ntiles; t += (int64_t)gridDim.x * blockDim.x)
         if (trow[t] < m) len = max(len, tnz[t] - rp[trow[t]]);
@@ -214,12 +225,12 @@ void build_tiles(const int32_t* rp, int64_t m, int64_t nnz, int64_t& ntiles, int
     cval = dmalloc<double>(ntiles);
     hrow = dmalloc<int32_t>(ntiles);
     hval = dmalloc<double>(ntiles);
-    tiles_kernel<<<blocks(ntiles + 1), 256, 0, s>>>(rp, m, nnz, kSpmvTile, ntiles, trow, tnz);
+    launch_next(tiles_kernel, blocks(ntiles + 1), 256, 0, s, rp, m, nnz, kSpmvTile, ntiles, trow, tnz);
     launched("tiles_kernel");
     // crow[ntiles] serves as the result before it becomes the ticket (zero)
     short_heads = false;
     if (ntiles > 0 && ntiles <= kSpmvSmallTiles) {
-        longest_head_kernel<<<blocks(ntiles), 256, 0, s>>>(rp, m, nnz, ntiles, trow, tnz, crow + ntiles);
+        launch_next(longest_head_kernel, blocks(ntiles), 256, 0, s, rp, m, nnz, ntiles, trow, tnz, crow + ntiles);
         launched("longest_head_kernel");
         int longest = 0;
         check_cuda(cudaMemcpyAsync(&longest, crow + ntiles, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H heads");
@@ -258,10 +269,10 @@ void radix_sort_pairs(int32_t*& kA, int32_t*& vA, int32_t*& kB, int32_t*& vB, in
     if (nnz == 0 || bits == 0) return;
     int32_t* counts = dmalloc<int32_t>(kRadix * ntiles);
     for (int shift = 0; shift < bits; shift += kRadixBits) {
-        radix_upsweep<<<(unsigned)ntiles, kSortThreads, 0, s>>>(kA, nnz, shift, counts, ntiles);
+        launch_next(radix_upsweep, (unsigned)ntiles, kSortThreads, 0, s, kA, nnz, shift, counts, ntiles);
         launched("radix_upsweep");
         scan_exclusive_i32(counts, counts, kRadix * ntiles, s);
-        radix_downsweep<<<(unsigned)ntiles, kSortThreads, 0, s>>>(kA, vA, kB, vB, nnz, shift, counts, ntiles);
+        launch_next(radix_downsweep, (unsigned)ntiles, kSortThreads, 0, s, kA, vA, kB, vB, nnz, shift, counts, ntiles);
         launched("radix_downsweep");
         std::swap(kA, kB);
         std::swap(vA, vB);
@@ -272,6 +283,7 @@ void radix_sort_pairs(int32_t*& kA, int32_t*& vA, int32_t*& kB, int32_t*& vB, in
 
 __global__ void gather_i32_kernel(int64_t nnz, const int32_t* __restrict__ perm, const int32_t* __restrict__ src,
                                   int32_t* __restrict__ dst) {
+    if (!after_previous()) return;
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p < nnz) dst[p] = src[perm[p]];
 }
@@ -285,14 +297,14 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
     int32_t* vB = dmalloc<int32_t>(nnz);
     check_cuda(cudaMemcpyAsync(kA, A->ci, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, s), "copy keys");
     if (nnz > 0) {
-        iota_kernel<<<blocks(nnz), 256, 0, s>>>(vA, nnz);
+        launch_next(iota_kernel, blocks(nnz), 256, 0, s, vA, nnz);
         launched("iota_kernel");
     }
     radix_sort_pairs(kA, vA, kB, vB, nnz, n, s);
     // kA: sorted column keys, vA: CSR position of each sorted entry
     int32_t* row_of = dmalloc<int32_t>(nnz);
     if (m > 0 && nnz > 0) {
-        row_of_kernel<<<blocks(m * 32), 256, 0, s>>>(A->rp, m, row_of);
+        launch_next(row_of_kernel, blocks(m * 32), 256, 0, s, A->rp, m, row_of);
         launched("row_of_kernel");
     }
     int32_t* ci_raw = kB;  // reuse
@@ -302,12 +314,12 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
     unsigned long long* kept_d = dmalloc<unsigned long long>(1);
     unsigned long long kept = 0;
     if (nnz > 0) {
-        gather_t_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, vA, row_of, A->val, ci_raw, val_raw);
+        launch_next(gather_t_kernel, blocks(nnz), 256, 0, s, nnz, vA, row_of, A->val, ci_raw, val_raw);
         launched("gather_t_kernel");
-        runs_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, kA, ci_raw, val_raw, run_sum, keep);
+        launch_next(runs_kernel, blocks(nnz), 256, 0, s, nnz, kA, ci_raw, val_raw, run_sum, keep);
         launched("runs_kernel");
         check_cuda(cudaMemsetAsync(kept_d, 0, sizeof(unsigned long long), s), "memset");
-        sum_i32_kernel<<<grid_for(nnz, 256, 1024), 256, 0, s>>>(nnz, keep, kept_d);
+        launch_next(sum_i32_kernel, grid_for(nnz, 256, 1024), 256, 0, s, nnz, keep, kept_d);
         launched("sum_i32_kernel");
         check_cuda(cudaMemcpyAsync(&kept, kept_d, sizeof(kept), cudaMemcpyDeviceToHost, s), "D2H kept");
         check_cuda(cudaStreamSynchronize(s), "transpose sync");
@@ -322,7 +334,7 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
         A->permT = vA;
         A->t_compacted = false;
         if (nnz > 0) {
-            histogram_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, kA, cnt);
+            launch_next(histogram_kernel, blocks(nnz), 256, 0, s, nnz, kA, cnt);
             launched("histogram_kernel");
         }
         dfree(run_sum);
@@ -335,11 +347,11 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
         A->ciT = dmalloc<int32_t>(A->nnz_t);
         A->valT = dmalloc<double>(A->nnz_t);
         int32_t* keyT = dmalloc<int32_t>(A->nnz_t);
-        compact_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, keep, pos, kA, ci_raw, run_sum, A->ciT, A->valT,
-                                                   keyT);
+        launch_next(compact_kernel, blocks(nnz), 256, 0, s, nnz, keep, pos, kA, ci_raw, run_sum, A->ciT, A->valT,
+                    keyT);
         launched("compact_kernel");
         if (A->nnz_t > 0) {
-            histogram_kernel<<<blocks(A->nnz_t), 256, 0, s>>>(A->nnz_t, keyT, cnt);
+            launch_next(histogram_kernel, blocks(A->nnz_t), 256, 0, s, A->nnz_t, keyT, cnt);
             launched("histogram_kernel");
         }
         check_cuda(cudaStreamSynchronize(s), "transpose sync");
@@ -541,12 +553,12 @@ void coo_to_csr(int64_t m, int64_t n, int64_t nnz, const int32_t* r, const int32
     int32_t* vB = dmalloc<int32_t>(nnz);
     if (nnz > 0) {
         check_cuda(cudaMemcpyAsync(kA, c, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, s), "copy keys");
-        iota_kernel<<<blocks(nnz), 256, 0, s>>>(vA, nnz);
+        launch_next(iota_kernel, blocks(nnz), 256, 0, s, vA, nnz);
         launched("iota_kernel");
     }
     radix_sort_pairs(kA, vA, kB, vB, nnz, n, s);  // by column
     if (nnz > 0) {
-        gather_i32_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, vA, r, kA);
+        launch_next(gather_i32_kernel, blocks(nnz), 256, 0, s, nnz, vA, r, kA);
         launched("gather_i32_kernel");
     }
     radix_sort_pairs(kA, vA, kB, vB, nnz, m, s);  // then by row (stable)
@@ -558,12 +570,12 @@ void coo_to_csr(int64_t m, int64_t n, int64_t nnz, const int32_t* r, const int32
     unsigned long long* kept_d = dmalloc<unsigned long long>(1);
     unsigned long long kept = 0;
     if (nnz > 0) {
-        gather_t_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, vA, c, v, ci_raw, val_raw);
+        launch_next(gather_t_kernel, blocks(nnz), 256, 0, s, nnz, vA, c, v, ci_raw, val_raw);
         launched("gather_t_kernel");
-        runs_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, kA, ci_raw, val_raw, run_sum, keep);
+        launch_next(runs_kernel, blocks(nnz), 256, 0, s, nnz, kA, ci_raw, val_raw, run_sum, keep);
         launched("runs_kernel");
         check_cuda(cudaMemsetAsync(kept_d, 0, sizeof(unsigned long long), s), "memset");
-        sum_i32_kernel<<<grid_for(nnz, 256, 1024), 256, 0, s>>>(nnz, keep, kept_d);
+        launch_next(sum_i32_kernel, grid_for(nnz, 256, 1024), 256, 0, s, nnz, keep, kept_d);
         launched("sum_i32_kernel");
         check_cuda(cudaMemcpyAsync(&kept, kept_d, sizeof(kept), cudaMemcpyDeviceToHost, s), "D2H kept");
         check_cuda(cudaStreamSynchronize(s), "coo sync");
@@ -577,11 +589,11 @@ void coo_to_csr(int64_t m, int64_t n, int64_t nnz, const int32_t* r, const int32
     check_cuda(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * (m + 1), s), "memset cnt");
     if (nnz > 0) {
         scan_exclusive_i32(keep, pos, nnz, s);
-        compact_kernel<<<blocks(nnz), 256, 0, s>>>(nnz, keep, pos, kA, ci_raw, run_sum, ci, val, key);
+        launch_next(compact_kernel, blocks(nnz), 256, 0, s, nnz, keep, pos, kA, ci_raw, run_sum, ci, val, key);
         launched("compact_kernel");
     }
     if (nk > 0) {
-        histogram_kernel<<<blocks(nk), 256, 0, s>>>(nk, key, cnt);
+        launch_next(histogram_kernel, blocks(nk), 256, 0, s, nk, key, cnt);
         launched("histogram_kernel");
     }
     int32_t* rp = dmalloc<int32_t>(m + 1);

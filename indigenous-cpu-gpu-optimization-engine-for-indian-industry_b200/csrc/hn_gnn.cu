@@ -46,6 +46,7 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, const uint
 __global__ void gnn_spmm_kernel(int rows, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                 const double* __restrict__ val, const float* __restrict__ H, int accumulate,
                                 float* __restrict__ out) {
+    if (!after_previous()) return;
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (r >= rows) return;
@@ -68,6 +69,7 @@ __global__ void gnn_spmm_kernel(int rows, const int32_t* __restrict__ rp, const 
 // dH += dX[:, :64]; dAgg = dX[:, 64:] (the two halves of a concatenated input)
 __global__ void gnn_split_grad_kernel(int64_t M, const float* __restrict__ dX, float* __restrict__ dH,
                                       float* __restrict__ dAgg) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= M * kH) return;
     const int64_t r = i / kH, c = i % kH;
@@ -79,6 +81,7 @@ __global__ void gnn_split_grad_kernel(int64_t M, const float* __restrict__ dX, f
 // for the other columns; per-block partial sums of the squared errors.
 __global__ void gnn_head_grad_kernel(int64_t M, const float* __restrict__ O, const float* __restrict__ T, int nt,
                                      float scale, float* __restrict__ dO, float* __restrict__ loss_part) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     double l = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < M * kH; i += (int64_t)gridDim.x * blockDim.x) {
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(kGT) gnn_gemm_kernel(int64_t M, int K1, int K2
                                                        const __nv_bfloat16* __restrict__ Bt,
                                                        const float* __restrict__ bias, int relu,
                                                        float* __restrict__ C) {
+    if (!after_previous()) return;
     constexpr int KP = KMAX + 8;  // padded rows: the fragment loads of a warp hit 32 banks
     __shared__ __align__(16) __nv_bfloat16 sA[kRowsPerCta][KP];
     __shared__ __align__(16) __nv_bfloat16 sB[N][KP];
@@ -273,6 +277,7 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_kernel(int64_t M, int K1, 
                                                              const float* __restrict__ bias, int relu,
                                                              float* __restrict__ Y, float* __restrict__ Y2, int* err,
                                                              uint32_t spin) {
+    if (!after_previous()) return;
     using P = UmmaPlan<N, KMAX>;
     extern __shared__ __align__(1024) uint8_t umma_smem[];
     uint8_t* sA = umma_smem + P::kOffA;
@@ -454,6 +459,7 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_kernel(int64_t M, int K1, 
 // G = dY * (Y > 0) (or dY when relu == 0)
 __global__ void gnn_relu_bwd_kernel(int64_t len, const float* __restrict__ dY, const float* __restrict__ Y, int relu,
                                     float* __restrict__ G) {
+    if (!after_previous()) return;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x)
         G[i] = (!relu || Y[i] > 0.f) ? dY[i] : 0.f;
 }
@@ -504,6 +510,7 @@ __global__ void __launch_bounds__(kUmmaT, 1) gnn_umma_wgrad_kernel(int64_t M, in
                                                                    float* __restrict__ part_w,
                                                                    float* __restrict__ part_b, int* err,
                                                                    uint32_t spin) {
+    if (!after_previous()) return;
     extern __shared__ __align__(1024) uint8_t wg_smem[];
     uint8_t* sA = wg_smem + kWOffA;
     uint8_t* sB = wg_smem + kWOffB;
@@ -684,6 +691,7 @@ constexpr int kSumT = 256, kSumB = 256;  // threads, partials staged at a time
 __global__ void __launch_bounds__(kSumT) gnn_sum_parts_kernel(int64_t nb, int64_t len, const float* __restrict__ pw,
                                                               const float* __restrict__ pb, float* __restrict__ dW,
                                                               float* __restrict__ db) {
+    if (!after_previous()) return;
     __shared__ float sp[kSumB][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t i = blockIdx.x * (int64_t)32 + lane;  // len and kH are multiples of 32: a CTA has entries of one kind
@@ -709,6 +717,7 @@ __global__ void __launch_bounds__(kSumT) gnn_sum_parts_kernel(int64_t nb, int64_
 // W (K x 64, FP32 master, row-major) -> Wt (64 x K, BF16) and Wb (K x 64, BF16)
 __global__ void gnn_cast_weights_kernel(int K, const float* __restrict__ W, __nv_bfloat16* __restrict__ Wt,
                                         __nv_bfloat16* __restrict__ Wb) {
+    if (!after_previous()) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= K * kH) return;
     const int k = i / kH, o = i % kH;
@@ -720,6 +729,7 @@ __global__ void gnn_cast_weights_kernel(int K, const float* __restrict__ W, __nv
 __global__ void gnn_adam_kernel(int64_t len, float* __restrict__ w, const float* __restrict__ g,
                                 float* __restrict__ m1, float* __restrict__ m2, float lr, float b1, float b2,
                                 float eps, float c1, float c2) {
+    if (!after_previous()) return;
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= len) return;
     const float gi = g[i];
@@ -755,8 +765,8 @@ void launch_umma(int64_t M, int K1, int K2, const float* X1, const float* X2, co
     static int attr_device = -1;
     smem_attribute(gnn_umma_kernel<N, KMAX>, P::kSmem, attr_device, "umma smem attribute");
     const int64_t tiles = (M + kUmmaM - 1) / kUmmaM;
-    gnn_umma_kernel<N, KMAX><<<(unsigned)std::min<int64_t>(tiles, ctx().sm_count), kUmmaT, P::kSmem, s>>>(
-        M, K1, K2, X1, X2, Bt, bias, relu, Y, Y2, umma_flag(s), g_umma_spin.load());
+    launch_next(gnn_umma_kernel<N, KMAX>, (unsigned)std::min<int64_t>(tiles, ctx().sm_count), kUmmaT, P::kSmem, s, M,
+                K1, K2, X1, X2, Bt, bias, relu, Y, Y2, umma_flag(s), g_umma_spin.load());
     launched("gnn_umma_kernel");
 }
 
@@ -784,8 +794,8 @@ void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, con
         float* gout = G;
         if (misaligned16(dY) || (relu && misaligned16(Y)) || G == dY || G == Y) {
             const int64_t len = M * kH;
-            gnn_relu_bwd_kernel<<<(unsigned)std::min<int64_t>((len + 255) / 256, 148 * 16), 256, 0, s>>>(len, dY, Y,
-                                                                                                     relu, G);
+            launch_next(gnn_relu_bwd_kernel, (unsigned)std::min<int64_t>((len + 255) / 256, 148 * 16), 256, 0, s, len,
+                        dY, Y, relu, G);
             launched("gnn_relu_bwd_kernel");
             dy = G;
             y = nullptr;
@@ -793,8 +803,8 @@ void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, con
         }
         static int attr_device = -1;
         smem_attribute(gnn_umma_wgrad_kernel, kWSmem, attr_device, "wgrad smem attribute");
-        gnn_umma_wgrad_kernel<<<(unsigned)nb, kUmmaT, kWSmem, s>>>(M, K1, K2, X1, X2, dy, y, gout, pw, pb,
-                                                                    umma_flag(s), g_umma_spin.load());
+        launch_next(gnn_umma_wgrad_kernel, (unsigned)nb, kUmmaT, kWSmem, s, M, K1, K2, X1, X2, dy, y, gout, pw, pb,
+                    umma_flag(s), g_umma_spin.load());
         launched("gnn_umma_wgrad_kernel");
         // dX = G W^T on the tcgen05 layer kernel: input G (M x 64), N = K
         // outputs, B = W (K x 64 row-major BF16), no bias, no activation
@@ -807,7 +817,7 @@ void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, con
         check_cuda(cudaMemsetAsync(scratch, 0, sizeof(float) * (kH * K + kH), s), "memset");
     }
     const int64_t len = (int64_t)kH * K;
-    gnn_sum_parts_kernel<<<(unsigned)((len + kH) / 32), kSumT, 0, s>>>(nb, len, pw, pb, dW, db);
+    launch_next(gnn_sum_parts_kernel, (unsigned)((len + kH) / 32), kSumT, 0, s, nb, len, pw, pb, dW, db);
     launched("gnn_sum_parts_kernel");
 }
 
@@ -828,8 +838,8 @@ int hn_gnn_spmm(const hn_csr* A, int trans, const float* H, float* out, int accu
         const int32_t* rp = trans ? A->rpT : A->rp;
         const int32_t* ci = trans ? A->ciT : A->ci;
         const double* val = trans ? A->valT : A->val;
-        gnn_spmm_kernel<<<(unsigned)((rows * 32LL + 255) / 256), 256, 0, as_stream(stream)>>>(rows, rp, ci, val, H,
-                                                                                            accumulate, out);
+        launch_next(gnn_spmm_kernel, (unsigned)((rows * 32LL + 255) / 256), 256, 0, as_stream(stream), rows, rp, ci,
+                    val, H, accumulate, out);
         launched("gnn_spmm_kernel");
     });
 }
@@ -838,8 +848,8 @@ int hn_gnn_cast_weights(int K, const float* W, void* Wt_bf16, void* Wb_bf16, voi
     return guard("hn_gnn_cast_weights", [&] {
         require_init();
         if (K <= 0 || K > kMaxK || !W || !Wt_bf16 || !Wb_bf16) fail(HN_ERR_INVALID_ARG, "bad arguments");
-        gnn_cast_weights_kernel<<<(K * kH + 255) / 256, 256, 0, as_stream(stream)>>>(
-            K, W, static_cast<__nv_bfloat16*>(Wt_bf16), static_cast<__nv_bfloat16*>(Wb_bf16));
+        launch_next(gnn_cast_weights_kernel, (K * kH + 255) / 256, 256, 0, as_stream(stream), K, W,
+                    static_cast<__nv_bfloat16*>(Wt_bf16), static_cast<__nv_bfloat16*>(Wb_bf16));
         launched("gnn_cast_weights_kernel");
     });
 }
@@ -856,10 +866,12 @@ int hn_gnn_linear(int64_t M, int K1, int K2, const float* X1, const float* X2, c
         const unsigned grid = (unsigned)((M + kRowsPerCta - 1) / kRowsPerCta);
         const auto* B = static_cast<const __nv_bfloat16*>(Wt_bf16);
         if (N == 64) {
-            gnn_gemm_kernel<64, kMaxK><<<grid, kGT, 0, as_stream(stream)>>>(M, K1, K2, X1, X2, B, bias, relu, Y);
+            launch_next(gnn_gemm_kernel<64, kMaxK>, grid, kGT, 0, as_stream(stream), M, K1, K2, X1, X2, B, bias, relu,
+                        Y);
         } else {
             if (K > 64) fail(HN_ERR_INVALID_ARG, "N = 128 takes K1 + K2 <= 64");
-            gnn_gemm_kernel<128, 64><<<grid, kGT, 0, as_stream(stream)>>>(M, K1, K2, X1, X2, B, bias, relu, Y);
+            launch_next(gnn_gemm_kernel<128, 64>, grid, kGT, 0, as_stream(stream), M, K1, K2, X1, X2, B, bias, relu,
+                        Y);
         }
         launched("gnn_gemm_kernel");
     });
@@ -924,7 +936,8 @@ int hn_gnn_split_grad(int64_t M, const float* dX, float* dH, float* dAgg, void* 
         require_init();
         if (M < 0 || (M && (!dX || !dH || !dAgg))) fail(HN_ERR_INVALID_ARG, "bad arguments");
         if (M == 0) return;
-        gnn_split_grad_kernel<<<(unsigned)((M * kH + 255) / 256), 256, 0, as_stream(stream)>>>(M, dX, dH, dAgg);
+        launch_next(gnn_split_grad_kernel, (unsigned)((M * kH + 255) / 256), 256, 0, as_stream(stream), M, dX, dH,
+                    dAgg);
         launched("gnn_split_grad_kernel");
     });
 }
@@ -936,7 +949,7 @@ int hn_gnn_head_grad(int64_t M, const float* O, const float* T, int nt, float sc
         if (M < 0 || nt < 1 || nt > 2 || nparts < 1 || (M && (!O || !T || !dO)) || !loss_part)
             fail(HN_ERR_INVALID_ARG, "bad arguments");
         const int grid = (int)std::min<int64_t>(nparts, std::max<int64_t>(1, (M * kH + 255) / 256));
-        gnn_head_grad_kernel<<<grid, 256, 0, as_stream(stream)>>>(M, O, T, nt, scale, dO, loss_part);
+        launch_next(gnn_head_grad_kernel, grid, 256, 0, as_stream(stream), M, O, T, nt, scale, dO, loss_part);
         launched("gnn_head_grad_kernel");
         if (grid < nparts)
             check_cuda(cudaMemsetAsync(loss_part + grid, 0, sizeof(float) * (nparts - grid), as_stream(stream)),
@@ -951,8 +964,8 @@ int hn_gnn_adam(int64_t len, float* w, const float* g, float* m1, float* m2, flo
         if (len < 0 || step < 1 || (len && (!w || !g || !m1 || !m2))) fail(HN_ERR_INVALID_ARG, "bad arguments");
         if (len == 0) return;
         const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-        gnn_adam_kernel<<<(unsigned)((len + 255) / 256), 256, 0, as_stream(stream)>>>(len, w, g, m1, m2, lr, beta1,
-                                                                                      beta2, eps, c1, c2);
+        launch_next(gnn_adam_kernel, (unsigned)((len + 255) / 256), 256, 0, as_stream(stream), len, w, g, m1, m2, lr,
+                    beta1, beta2, eps, c1, c2);
         launched("gnn_adam_kernel");
     });
 }

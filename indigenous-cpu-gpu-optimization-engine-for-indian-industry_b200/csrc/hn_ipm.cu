@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kT) prep_kernel(int64_t n, int64_t m, const do
                                                   const double* __restrict__ rp, double* __restrict__ D,
                                                   double* __restrict__ Drd, double* partials, unsigned* counter,
                                                   double* scal) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     double smu = 0.0, mrd = 0.0, mrp = 0.0;
     const int64_t stride = (int64_t)gridDim.x * kT;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(kT) steps_kernel(int64_t n, int64_t m, const d
                                                    const double* __restrict__ dx, const double* __restrict__ z,
                                                    const double* __restrict__ dz, const double* __restrict__ dlam,
                                                    double* partials, unsigned* counter, double* scal) {
+    if (!after_previous()) return;
     __shared__ double2 sh[kT / 32];
     double ap = 1.0, ad = 1.0;
     bool bad = false;
@@ -158,6 +160,7 @@ __global__ void __launch_bounds__(kT) mu_aff_kernel(int64_t n, const double* __r
                                                     const double* __restrict__ dx, const double* __restrict__ z,
                                                     const double* __restrict__ dz, double* partials,
                                                     unsigned* counter, double* scal) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     const double ap = scal[HN_IPM_AP], ad = scal[HN_IPM_AD];
     double s = 0.0;
@@ -189,6 +192,7 @@ __global__ void __launch_bounds__(kT) mu_aff_kernel(int64_t n, const double* __r
 __global__ void corr_term_kernel(int64_t n, const double* __restrict__ dx, const double* __restrict__ dz,
                                  const double* __restrict__ z, const double* __restrict__ scal,
                                  double* __restrict__ zs) {
+    if (!after_previous()) return;
     const double sm = scal[HN_IPM_SIGMA] * scal[HN_IPM_MU];
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += stride) {
@@ -201,6 +205,7 @@ __global__ void __launch_bounds__(kT) update_kernel(int64_t n, int64_t m, double
                                                     const double* __restrict__ dx, double* __restrict__ z,
                                                     const double* __restrict__ dz, double* __restrict__ lam,
                                                     const double* __restrict__ dlam, double* scal) {
+    if (!after_previous()) return;
     __shared__ int s_bad;
     if (threadIdx.x == 0) s_bad = 0;
     __syncthreads();
@@ -223,6 +228,7 @@ __global__ void __launch_bounds__(kT) update_kernel(int64_t n, int64_t m, double
 __global__ void __launch_bounds__(kT) max_step_kernel(int64_t n, const double* __restrict__ v,
                                                       const double* __restrict__ d, double* partials,
                                                       unsigned* counter, double* out) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     double a = 1.0;
     const int64_t stride = (int64_t)gridDim.x * kT;
@@ -253,6 +259,7 @@ __global__ void __launch_bounds__(kT) kkt_kernel(int64_t n, int64_t m, const dou
                                                  const double* __restrict__ rd, const double* __restrict__ ru,
                                                  const double* __restrict__ cu, double offset, double* partials,
                                                  unsigned* counter, double* out) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     double pr = 0.0, bn = 0.0, du = 0.0, cn = 0.0, cx = 0.0, by = 0.0;
     const int64_t stride = (int64_t)gridDim.x * kT;
@@ -332,7 +339,8 @@ int hn_ipm_residuals(const hn_csr* A, const double* x, const double* lam, const 
         spmv_launch2(spmv_mat(A, 0), x, EpiResidual{b, mx, rp}, spmv_mat(A, 1), lam, EpiDualResidual{z, c, rd}, s);
         Workspace& w = workspace(s);
         const int64_t big = A->n > A->m ? A->n : A->m;
-        prep_kernel<<<red_grid(big), kT, 0, s>>>(A->n, A->m, x, z, rd, rp, D, Drd, w.partials, w.counter, scal);
+        launch_next(prep_kernel, red_grid(big), kT, 0, s, A->n, A->m, x, z, rd, rp, D, Drd, w.partials, w.counter,
+                    scal);
         launched("prep_kernel");
     });
 }
@@ -361,7 +369,8 @@ int hn_ipm_step_lengths(int64_t n, int64_t m, const double* x, const double* dx,
         require_init();
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
-        steps_kernel<<<grid_for(n > m ? n : m, kT, kMaxReduceBlocks), kT, 0, s>>>(n, m, x, dx, z, dz, dlam, w.partials, w.counter, scal);
+        launch_next(steps_kernel, grid_for(n > m ? n : m, kT, kMaxReduceBlocks), kT, 0, s, n, m, x, dx, z, dz, dlam,
+                    w.partials, w.counter, scal);
         launched("steps_kernel");
     });
 }
@@ -374,9 +383,9 @@ int hn_ipm_corrector(const hn_csr* A, const double* x, const double* dx, const d
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
         const int64_t n = A->n;
-        mu_aff_kernel<<<red_grid(n), kT, 0, s>>>(n, x, dx, z, dz, w.partials, w.counter, scal);
+        launch_next(mu_aff_kernel, red_grid(n), kT, 0, s, n, x, dx, z, dz, w.partials, w.counter, scal);
         launched("mu_aff_kernel");
-        corr_term_kernel<<<grid_for(n, kT, ctx().sm_count * 16), kT, 0, s>>>(n, dx, dz, z, scal, zs);
+        launch_next(corr_term_kernel, grid_for(n, kT, ctx().sm_count * 16), kT, 0, s, n, dx, dz, z, scal, zs);
         launched("corr_term_kernel");
         spmv_launch(spmv_mat(A, 0), zs, EpiCorrRhs{rhs_pred, rhs}, s);
     });
@@ -387,8 +396,8 @@ int hn_ipm_update(int64_t n, int64_t m, double* x, const double* dx, double* z, 
     return guard("hn_ipm_update", [&] {
         require_init();
         cudaStream_t s = as_stream(stream);
-        update_kernel<<<grid_for(n > m ? n : m, kT, ctx().sm_count * 16), kT, 0, s>>>(n, m, x, dx, z, dz, lam,
-                                                                                     dlam, scal);
+        launch_next(update_kernel, grid_for(n > m ? n : m, kT, ctx().sm_count * 16), kT, 0, s, n, m, x, dx, z, dz,
+                    lam, dlam, scal);
         launched("update_kernel");
     });
 }
@@ -402,8 +411,8 @@ int hn_ipm_kkt(int64_t n, int64_t m, const double* x, const double* lam, const d
             fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
-        kkt_kernel<<<grid_for(n > m ? n : m, kT * 4, kKktMaxBlocks), kT, 0, s>>>(n, m, x, lam, b, c, rp, rd, ru, cu,
-                                                                                  offset, w.partials, w.counter, kkt);
+        launch_next(kkt_kernel, grid_for(n > m ? n : m, kT * 4, kKktMaxBlocks), kT, 0, s, n, m, x, lam, b, c, rp, rd,
+                    ru, cu, offset, w.partials, w.counter, kkt);
         launched("kkt_kernel");
     });
 }
@@ -414,7 +423,7 @@ int hn_max_step(int64_t n, const double* v, const double* d, double* result, voi
         if (n < 0 || !result) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
         Workspace& w = workspace(s);
-        max_step_kernel<<<red_grid(n), kT, 0, s>>>(n, v, d, w.partials, w.counter, result);
+        launch_next(max_step_kernel, red_grid(n), kT, 0, s, n, v, d, w.partials, w.counter, result);
         launched("max_step_kernel");
     });
 }

@@ -40,6 +40,7 @@ static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 // table hn_csr_create builds).
 __global__ void noalloc_tiles_kernel(const int32_t* __restrict__ rp, int64_t m, int64_t nnz, int64_t ntiles,
                                      NoAllocScratch* sc) {
+    if (!after_previous()) return;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t > ntiles) return;
     int64_t diag = t * kSpmvTile;
@@ -97,7 +98,7 @@ int hn_spmv_noalloc(int64_t m, int64_t n, int64_t nnz, const int32_t* rp, const 
         const int64_t ntiles = (m + nnz + kSpmvTile - 1) / kSpmvTile;
         if (ntiles == 0) return;
         cudaStream_t s = as_stream(stream);
-        noalloc_tiles_kernel<<<(unsigned)((ntiles + 1 + 255) / 256), 256, 0, s>>>(rp, m, nnz, ntiles, sc);
+        launch_next(noalloc_tiles_kernel, (unsigned)((ntiles + 1 + 255) / 256), 256, 0, s, rp, m, nnz, ntiles, sc);
         launched("noalloc_tiles_kernel");
         SpmvMat M{(int)m, (int)nnz, rp, ci, val, sc->tile_row, sc->tile_nz, sc->carry_row, sc->carry_val,
                   sc->head_row, sc->head_val, ntiles};

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(kPT) devex_scale_kernel(int64_t n, const doubl
                                                           const int32_t* __restrict__ nonbasis,
                                                           double* __restrict__ partials,
                                                           unsigned* __restrict__ counter, double* __restrict__ out) {
+    if (!after_previous()) return;
     __shared__ double sh[32];
     __shared__ bool last;
     double v = 0.0;
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(kPT) devex_apply_kernel(int64_t n, const doubl
                                                           const int32_t* __restrict__ nonbasis,
                                                           const double* __restrict__ scale,
                                                           double* __restrict__ w) {
+    if (!after_previous()) return;
     const double s = *scale;
     if (s == 0.0) return;
     for (int64_t j = blockIdx.x * (int64_t)kPT + threadIdx.x; j < n; j += (int64_t)gridDim.x * kPT) {
@@ -214,6 +216,7 @@ __device__ __forceinline__ void select_chunks(int64_t first, int64_t step, int64
 __global__ void __launch_bounds__(kSelT, 1) price_ranked_kernel(PriceArgs a, int k, Pick* lists,
                                                              unsigned long long* counts, unsigned* ticket,
                                                              int64_t* out) {
+    if (!after_previous()) return;
     __shared__ Pick list[HN_PRICE_MAX_K];
     __shared__ Pick sw[2][16];
     __shared__ int64_t sh[32];
@@ -267,6 +270,7 @@ __global__ void __launch_bounds__(kSelT, 1) price_ranked_kernel(PriceArgs a, int
 // Count of improving columns and the first one (Bland), the last block closing.
 __global__ void __launch_bounds__(kPT) price_bland_kernel(PriceArgs a, unsigned long long* part, unsigned* ticket,
                                                           int64_t* out) {
+    if (!after_previous()) return;
     __shared__ int64_t sh[32];
     __shared__ bool s_last;
     int64_t cnt = 0, first = INT64_MAX;
@@ -314,6 +318,7 @@ __global__ void __launch_bounds__(kPT) column_gather_kernel(int64_t m, int64_t n
                                                             const double* __restrict__ valT,
                                                             const int64_t* __restrict__ cols, double* __restrict__ out,
                                                             unsigned long long* bad) {
+    if (!after_previous()) return;
     __shared__ int64_t sh[32];
     const int64_t slices = m > 0 ? (m + kColRows - 1) / kColRows : 1;
     const int64_t r = blockIdx.x / slices, i0 = (blockIdx.x % slices) * kColRows;
@@ -367,9 +372,9 @@ int hn_price_devex_update(const hn_csr* A, const double* u, const int32_t* nonba
         spmv_launch(spmv_mat(A, 1), u, EpiAxpby{1.0, 0.0, alpha}, s);
         const int g = price_grid(A->n);
         double* scale = w.partials + 4 * kMaxReduceBlocks;
-        devex_scale_kernel<<<g, kPT, 0, s>>>(A->n, alpha, nonbasis, w.partials, w.counter, scale);
+        launch_next(devex_scale_kernel, g, kPT, 0, s, A->n, alpha, nonbasis, w.partials, w.counter, scale);
         launched("devex_scale_kernel");
-        devex_apply_kernel<<<g, kPT, 0, s>>>(A->n, alpha, nonbasis, scale, weights);
+        launch_next(devex_apply_kernel, g, kPT, 0, s, A->n, alpha, nonbasis, scale, weights);
         launched("devex_apply_kernel");
     });
 }
@@ -386,14 +391,14 @@ int hn_price_select(int64_t n, const double* rc, const double* weights, const in
         Workspace& w = workspace(s);
         const PriceArgs a{n, rc, weights, nonbasis, artificial, phase1, maximize, optimality_tol};
         if (rule == HN_PRICE_BLAND) {
-            price_bland_kernel<<<price_grid(n), kPT, 0, s>>>(a, w.price, w.counter + 1, out);
+            launch_next(price_bland_kernel, price_grid(n), kPT, 0, s, a, w.price, w.counter + 1, out);
             launched("price_bland_kernel");
             return;
         }
         const int64_t chunks = (n + kSelChunk - 1) / kSelChunk;
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>(chunks, kPriceLists));
-        price_ranked_kernel<<<g, kSelT, 0, s>>>(a, (int)k, reinterpret_cast<Pick*>(w.price),
-                                                w.price + 2 * kPriceLists * HN_PRICE_MAX_K, w.counter + 1, out);
+        launch_next(price_ranked_kernel, g, kSelT, 0, s, a, (int)k, reinterpret_cast<Pick*>(w.price),
+                    w.price + 2 * kPriceLists * HN_PRICE_MAX_K, w.counter + 1, out);
         launched("price_ranked_kernel");
     });
 }
@@ -408,8 +413,8 @@ int hn_price_columns(const hn_csr* A, int64_t k, const int64_t* cols, double* ou
         Workspace& w = workspace(s);
         const int64_t slices = std::max<int64_t>(1, (A->m + kColRows - 1) / kColRows);
         if (k > INT32_MAX / slices) fail(HN_ERR_INVALID_ARG, "too many columns for one call");
-        column_gather_kernel<<<(unsigned)(k * slices), kPT, 0, s>>>(A->m, A->n, k, A->rpT, A->ciT, A->valT, cols, out,
-                                                                    w.select + W_BAD);
+        launch_next(column_gather_kernel, (unsigned)(k * slices), kPT, 0, s, A->m, A->n, k, A->rpT, A->ciT, A->valT,
+                    cols, out, w.select + W_BAD);
         launched("column_gather_kernel");
         unsigned long long bad = 0;
         check_cuda(cudaMemcpyAsync(&bad, w.select + W_BAD, sizeof(bad), cudaMemcpyDeviceToHost, s), "D2H flag");

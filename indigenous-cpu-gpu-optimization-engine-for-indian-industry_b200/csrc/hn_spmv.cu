@@ -17,6 +17,7 @@ __global__ void __launch_bounds__(256) spmm_wide_kernel(int m, const int32_t* __
                                                    const double* __restrict__ val,
                                                    const double* __restrict__ B, int64_t k,
                                                    double* __restrict__ C) {
+    if (!after_previous()) return;
     const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= m) return;
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restr
                                                    const double* __restrict__ val,
                                                    const double* __restrict__ B, int64_t k,
                                                    double* __restrict__ C) {
+    if (!after_previous()) return;
     const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
     const int l = threadIdx.x % G;
     if (row >= m) return;
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restr
 template <int G, int CC, int U>
 void spmm_launch(const SpmvMat& M, const double* B, int64_t k, double* C, cudaStream_t s) {
     const int64_t threads = (int64_t)M.m * G;
-    spmm_kernel<G, CC, U><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(M.m, M.rp, M.ci, M.val, B, k, C);
+    launch_next(spmm_kernel<G, CC, U>, (unsigned)((threads + 255) / 256), 256, 0, s, M.m, M.rp, M.ci, M.val, B, k, C);
     launched("spmm_kernel");
 }
 
@@ -105,7 +107,8 @@ void spmm_run(const hn_csr* A, int trans, const double* B, int64_t k, double* C,
     const SpmvMat M = spmv_mat(A, trans);
     if (M.m == 0 || k == 0) return;
     if (k > 64) {
-        spmm_wide_kernel<<<(unsigned)(((int64_t)M.m * 32 + 255) / 256), 256, 0, s>>>(M.m, M.rp, M.ci, M.val, B, k, C);
+        launch_next(spmm_wide_kernel, (unsigned)(((int64_t)M.m * 32 + 255) / 256), 256, 0, s, M.m, M.rp, M.ci, M.val,
+                    B, k, C);
         launched("spmm_wide_kernel");
     } else if (k > 32) {
         spmm_launch<32, 2, 1>(M, B, k, C, s);

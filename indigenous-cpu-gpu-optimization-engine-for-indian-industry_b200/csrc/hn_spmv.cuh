@@ -88,6 +88,7 @@ __device__ __forceinline__ int tile_search(const int32_t* s_rowend, int k0, int 
 template <class Epi>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_tile_kernel(SpmvMat a, const double* __restrict__ x,
                                                                  Epi epi) {
+    if (!after_previous()) return;
     __shared__ int32_t s_rowend[kSpmvTile + 1];
     __shared__ int32_t s_crow[kSpmvThreads];
     __shared__ double s_cval[kSpmvThreads];
@@ -205,6 +206,7 @@ __device__ __forceinline__ void fix_up(const SpmvMat& a, int64_t tile, const Epi
 
 template <class Epi>
 __global__ void spmv_fixup_kernel(SpmvMat a, Epi epi) {
+    if (!after_previous()) return;
     const int64_t tile = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (tile < a.ntiles) fix_up(a, tile, epi);
 }
@@ -356,6 +358,7 @@ __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __res
 
 template <class Epi>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_small_kernel(SpmvMat a, const double* __restrict__ x, Epi epi) {
+    if (!after_previous()) return;
     __shared__ SmallTile sh;
     small_tile(a, x, epi, blockIdx.x, sh);
 }
@@ -364,6 +367,7 @@ template <class Epi, class Epi2>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_small2_kernel(SpmvMat a, const double* __restrict__ x, Epi epi,
                                                                    SpmvMat b, const double* __restrict__ x2,
                                                                    Epi2 epi2) {
+    if (!after_previous()) return;
     __shared__ SmallTile sh;
     if (blockIdx.x < (unsigned)a.ntiles)
         small_tile(a, x, epi, blockIdx.x, sh);
@@ -413,6 +417,7 @@ __device__ __forceinline__ void vec_rows(const SpmvMat& a, int bin, int unit, co
 
 template <class Epi>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_vec_kernel(SpmvMat a, const double* __restrict__ x, Epi epi) {
+    if (!after_previous()) return;
     const int w = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     if (w >= a.bins.unit_off[a.bins.nbins]) return;  // whole warps leave together
     int bin = 0;
@@ -435,21 +440,21 @@ void spmv_launch(const SpmvMat& M, const double* x, const Epi& epi, cudaStream_t
     if (M.kind == 1) {
         const int64_t units = M.bins.unit_off[M.bins.nbins];
         if (units == 0) return;
-        spmv_vec_kernel<Epi><<<(unsigned)((units * 32 + kSpmvThreads - 1) / kSpmvThreads), kSpmvThreads, 0, s>>>(
-            M, x, epi);
+        launch_next(spmv_vec_kernel<Epi>, (unsigned)((units * 32 + kSpmvThreads - 1) / kSpmvThreads), kSpmvThreads, 0,
+                    s, M, x, epi);
         launched("spmv_vec_kernel");
         return;
     }
     if (M.ntiles == 0) return;
     if (spmv_small(M)) {
-        spmv_small_kernel<Epi><<<(unsigned)M.ntiles, kSpmvThreads, 0, s>>>(M, x, epi);
+        launch_next(spmv_small_kernel<Epi>, (unsigned)M.ntiles, kSpmvThreads, 0, s, M, x, epi);
         launched("spmv_small_kernel");
         return;
     }
-    spmv_tile_kernel<Epi><<<(unsigned)M.ntiles, kSpmvThreads, 0, s>>>(M, x, epi);
+    launch_next(spmv_tile_kernel<Epi>, (unsigned)M.ntiles, kSpmvThreads, 0, s, M, x, epi);
     launched("spmv_tile_kernel");
     if (M.ntiles > 1) {
-        spmv_fixup_kernel<Epi><<<(unsigned)((M.ntiles + 255) / 256), 256, 0, s>>>(M, epi);
+        launch_next(spmv_fixup_kernel<Epi>, (unsigned)((M.ntiles + 255) / 256), 256, 0, s, M, epi);
         launched("spmv_fixup_kernel");
     }
 }
@@ -459,7 +464,8 @@ template <class Epi, class Epi2>
 void spmv_launch2(const SpmvMat& M, const double* x, const Epi& epi, const SpmvMat& M2, const double* x2,
                   const Epi2& epi2, cudaStream_t s) {
     if (spmv_small(M) && spmv_small(M2) && M.ntiles > 0 && M2.ntiles > 0) {
-        spmv_small2_kernel<Epi, Epi2><<<(unsigned)(M.ntiles + M2.ntiles), kSpmvThreads, 0, s>>>(M, x, epi, M2, x2, epi2);
+        launch_next(spmv_small2_kernel<Epi, Epi2>, (unsigned)(M.ntiles + M2.ntiles), kSpmvThreads, 0, s, M, x, epi,
+                    M2, x2, epi2);
         launched("spmv_small2_kernel");
         return;
     }
