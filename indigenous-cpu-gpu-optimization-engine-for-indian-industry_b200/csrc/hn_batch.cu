@@ -664,51 +664,64 @@ __device__ __forceinline__ int item_instance(const int64_t* cum, int cnt, int64_
     return lo;
 }
 
-// L[r, k0:k1] = A[r, k0:k1] (L_blk D)^-T for kPanelT rows of one instance's
-// panel, a row per thread (kT / kPanelT CTAs per chunk). A panel row exists
-// only below a full block, so all 64 columns are there. As soon as L[r, q] is
-// final it is taken from every later column, which leaves independent updates
-// in flight instead of one chain of subtractions per column; each element
-// sees the same products in the same order (q ascending). The columns go in
-// two halves of 32 registers through the same code (a loop over the first
-// half's columns, then the unrolled triangle): half the code of 64 unrolled
-// columns, which missed the instruction cache. What bounds it is the L1 data
-// path: 16 bytes of L to every lane per four FP64 instructions, and, while
-// each thread read and wrote its own row of memory, 32 sectors per access. The
-// rows now pass through shared memory (16-byte copies in, whole lines out)
-// except the second half's way in, which there is no room for at three CTAs
-// per SM. Two rows per thread halve the L loads but also the warps: 2,880
-// against 1,475 us over the 30 panels of 384 LPs of m 50-2000.
-// 384 LPs of m 50-2000 (30 panels): 1,209 us; 2,156 with a chain per column.
+// L[r, k0:k1] = A[r, k0:k1] (L_blk D)^-T for kPanelT / G rows of one
+// instance's panel per CTA: G neighbouring lanes share a row, each with every
+// G-th pair of columns. A panel row exists only below a full block, so all 64
+// columns are there. As soon as L[r, q] is final it is taken from every later
+// column, which leaves independent updates in flight instead of one chain of
+// subtractions per column; each element sees the same products in the same
+// order (q ascending). The lanes of a row take column q from its owner by a
+// shuffle and all form the quotient; a finished pair goes to shared memory, so
+// a pair in which some lane still has a column left is updated in all of them.
+// The columns go in two halves of 32 through the same code (a loop over the
+// first half's columns, then the unrolled triangle): half the code of 64
+// unrolled columns, which missed the instruction cache. The rows pass through
+// shared memory (16-byte copies in, whole lines out) except the second half's
+// way in, which there is no room for at three CTAs per SM.
+// What bounds it is the latency of a row's 64 steps and the L1 data path (16
+// bytes of L to every lane per four FP64 instructions). A lane per row has the
+// fewest instructions and is the form for panels that fill the GPU: 1,209 us
+// for the 30 panels of 384 LPs of m 50-2000 (2,156 with a chain per column);
+// with two rows for two lanes, which halves the loads of L, the iteration
+// takes 8,081 us instead of 7,798, with four for four 9,007. Where a panel is
+// small a warp's 4,000 FP64 instructions per row are its time, and four lanes
+// per row take it from 16 to 8 us: an iteration of 48 LPs of m 50-300 takes
+// 421 us instead of 450 (428 with eight lanes). The line: kPanelWide chunks,
+// about one wave of the four-lane form's CTAs. The iteration of the 384 LPs,
+// whose last panels are small, by the line: 7,798 us at none, 7,781 at 100,
+// 7,798 at 160, 7,860 at 260, 8,295 at all.
+constexpr int64_t kPanelWide = 100;
 constexpr int kPanelT = 128;
 constexpr int kPanelP = kFb + 2;  // even: 16-byte loads of two entries
 constexpr int kHalf = kFb / 2;
 constexpr int kRowP = kHalf + 2;  // staged rows: 16-byte accesses of eight lanes hit distinct banks
-constexpr size_t kPanelSmem = sizeof(double) * (kFb * kPanelP + 2 * kFb + kPanelT * kRowP);
+constexpr size_t panel_smem(int rows) { return sizeof(double) * (kFb * kPanelP + 2 * kFb + rows * kRowP); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
 }
 
+template <int G>
 __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, const Chunk* __restrict__ chunks,
                                                                       const InstInfo* __restrict__ info,
                                                                       const int32_t* __restrict__ status, double* dense,
                                                                       const double* __restrict__ dD) {
     if (!after_previous()) return;
+    constexpr int kRows = kPanelT / G, kPairs = kHalf / 2 / G;
     extern __shared__ __align__(16) double panel_sm[];
     double(*sLt)[kPanelP] = reinterpret_cast<double(*)[kPanelP]>(panel_sm);  // sLt[q][c] = L[k0 + c, k0 + q]
     double* sD = panel_sm + kFb * kPanelP;
     double* sY = sD + kFb;  // 1 / D, zero where a quotient needs the division
     double(*sRow)[kRowP] = reinterpret_cast<double(*)[kRowP]>(sY + kFb);  // half the columns of every row
     const int tid = threadIdx.x;
-    const Chunk ch = chunks[blockIdx.x / (kT / kPanelT)];
+    const Chunk ch = chunks[blockIdx.x / (kT / kRows)];
     if (status[ch.inst] != ST_RUN) return;
     const InstInfo in = info[ch.inst];
     const int ld = dense_ld(in.m);
     const int k0 = s * kFb;
-    const int rb = k0 + kFb + ch.local * kT + static_cast<int>(blockIdx.x % (kT / kPanelT)) * kPanelT;
-    const int rows = min(kPanelT, in.m - rb);
+    const int rb = k0 + kFb + ch.local * kT + static_cast<int>(blockIdx.x % (kT / kRows)) * kRows;
+    const int rows = min(kRows, in.m - rb);
     if (rows <= 0) return;
     double* A = dense + in.dn;
     double* P = A + (int64_t)rb * ld + k0;  // the panel's rows
@@ -728,64 +741,69 @@ __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, con
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    double* mine = sRow[tid];
-    // whole lines of half h of the rows; called by all threads once the half is in sRow
-    auto store = [&](int h) {
-        __syncthreads();
-#pragma unroll 4
-        for (int r = line; r < rows; r += kPanelT / 16)
-            *reinterpret_cast<double2*>(P + (int64_t)r * ld + h * kHalf + 2 * piece) =
-                *reinterpret_cast<const double2*>(&sRow[r][2 * piece]);
+    // columns 2 (G i + side) and the next of a half belong to this lane
+    const int side = tid % G;
+    double* mine = sRow[tid / G];
+    double v[2 * kPairs];
+    auto load = [&](const double* from) {
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+            const double2 t = *reinterpret_cast<const double2*>(from + 2 * (G * i + side));
+            v[2 * i] = t.x;
+            v[2 * i + 1] = t.y;
+        }
     };
-    double v[kHalf];
+    load(mine);
+    __syncwarp();
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
-        const double* from = h == 0 ? mine : P + (int64_t)min(tid, rows - 1) * ld + kHalf;
-#pragma unroll
-        for (int c = 0; c < kHalf; c += 2) {
-            const double2 t = *reinterpret_cast<const double2*>(from + c);
-            v[c] = t.x;
-            v[c + 1] = t.y;
-        }
         if (h == 1) {
 #pragma unroll 1
             for (int q = 0; q < kHalf; q += 2) {
                 // L[r, q] D_q, rounded once as every column uses it
                 const double2 lq = *reinterpret_cast<const double2*>(mine + q);
                 const double w0 = lq.x * sD[q], w1 = lq.y * sD[q + 1];
-                const double *l0 = &sLt[q][kHalf], *l1 = &sLt[q + 1][kHalf];
+                const double *l0 = &sLt[q][kHalf + 2 * side], *l1 = &sLt[q + 1][kHalf + 2 * side];
 #pragma unroll
-                for (int c = 0; c < kHalf; c += 2) {
-                    const double2 t = *reinterpret_cast<const double2*>(l0 + c);
-                    const double2 u = *reinterpret_cast<const double2*>(l1 + c);
-                    v[c] -= w0 * t.x;
-                    v[c + 1] -= w0 * t.y;
-                    v[c] -= w1 * u.x;
-                    v[c + 1] -= w1 * u.y;
+                for (int i = 0; i < kPairs; ++i) {
+                    const double2 t = *reinterpret_cast<const double2*>(l0 + 2 * G * i);
+                    const double2 u = *reinterpret_cast<const double2*>(l1 + 2 * G * i);
+                    v[2 * i] -= w0 * t.x;
+                    v[2 * i + 1] -= w0 * t.y;
+                    v[2 * i] -= w1 * u.x;
+                    v[2 * i + 1] -= w1 * u.y;
                 }
             }
+            __syncthreads();  // the first half has been used and has left sRow
         }
-        const double* sLh = &sLt[h * kHalf][h * kHalf];
+        const double* sLh = &sLt[h * kHalf][h * kHalf + 2 * side];
+        double l[2];
 #pragma unroll
         for (int q = 0; q < kHalf; ++q) {
+            const int owner = q / 2 % G, i0 = q / 2 / G;
             const double d = sD[h * kHalf + q], y = sY[h * kHalf + q];
-            double l = quotient(v[q], d, y);
-            if (y == 0.0 || !(in_range(v[q]) || v[q] == 0.0)) l = v[q] / d;
-            const double w = l * d;
-            v[q] = l;
-            const int c0 = q + 1;
-            if ((c0 & 1) && c0 < kHalf) v[c0] -= w * sLh[q * kPanelP + c0];
+            double a = v[2 * i0 + q % 2];
+            if (G > 1) a = __shfl_sync(0xffffffffu, a, owner, G);
+            l[q % 2] = quotient(a, d, y);
+            if (y == 0.0 || !(in_range(a) || a == 0.0)) l[q % 2] = a / d;
+            const double w = l[q % 2] * d;
+            if (q % 2 == 1 && side == owner) *reinterpret_cast<double2*>(mine + q - 1) = make_double2(l[0], l[1]);
+            // finished columns of pair i0 take part and are not used again
 #pragma unroll
-            for (int c = c0 + (c0 & 1); c < kHalf; c += 2) {
-                const double2 t = *reinterpret_cast<const double2*>(sLh + q * kPanelP + c);
-                v[c] -= w * t.x;
-                v[c + 1] -= w * t.y;
+            for (int i = i0; i < kPairs; ++i) {
+                if (i == i0 && owner == G - 1 && q % 2 == 1) continue;
+                const double2 t = *reinterpret_cast<const double2*>(sLh + q * kPanelP + 2 * G * i);
+                v[2 * i] -= w * t.x;
+                v[2 * i + 1] -= w * t.y;
             }
         }
-        if (h == 1) __syncthreads();  // the first half has left sRow
-#pragma unroll
-        for (int c = 0; c < kHalf; c += 2) *reinterpret_cast<double2*>(mine + c) = make_double2(v[c], v[c + 1]);
-        store(h);
+        if (h == 0) load(P + (int64_t)min(tid / G, rows - 1) * ld + kHalf);
+        // whole lines of half h of the rows
+        __syncthreads();
+#pragma unroll 4
+        for (int r = line; r < rows; r += kPanelT / 16)
+            *reinterpret_cast<double2*>(P + (int64_t)r * ld + h * kHalf + 2 * piece) =
+                *reinterpret_cast<const double2*>(&sRow[r][2 * piece]);
     }
 }
 
@@ -1495,8 +1513,8 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             B->nrp = dmalloc<int32_t>(m + 1);
             B->work = dmalloc<double>(m);
             B->solve_part = dmalloc<double>(2 * kFb * (m / kT + K + 1));
-            check_cuda(cudaFuncSetAttribute(batch_ldlt_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)kPanelSmem),
+            check_cuda(cudaFuncSetAttribute(batch_ldlt_panel_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)panel_smem(kPanelT)),
                        "panel smem attribute");
             for (auto* k : {batch_ldlt_update_kernel<1>, batch_ldlt_update_kernel<2>})
                 check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kUpdSmem),
@@ -1694,8 +1712,13 @@ int hn_batch_factor(hn_batch* B, const double* D, double reg, double singular_to
             launched("batch_ldlt_diag_kernel");
             const int64_t nc = B->chunk_off_h[st + 1] - B->chunk_off_h[st];
             if (nc == 0) continue;
-            launch_next(batch_ldlt_panel_kernel, (unsigned)(nc * (kT / kPanelT)), kPanelT, kPanelSmem, s, (int)st,
-                        B->chunks + B->chunk_off_h[st], B->info, status, B->dense, B->dD);
+            if (nc <= kPanelWide)
+                launch_next(batch_ldlt_panel_kernel<4>, (unsigned)(nc * (kT / (kPanelT / 4))), kPanelT,
+                            panel_smem(kPanelT / 4), s, (int)st, B->chunks + B->chunk_off_h[st], B->info, status,
+                            B->dense, B->dD);
+            else
+                launch_next(batch_ldlt_panel_kernel<1>, (unsigned)(nc * (kT / kPanelT)), kPanelT, panel_smem(kPanelT),
+                            s, (int)st, B->chunks + B->chunk_off_h[st], B->info, status, B->dense, B->dD);
             launched("batch_ldlt_panel_kernel");
             const int64_t nt = B->step_tiles_h[st];
             const unsigned grid = (unsigned)std::min<int64_t>(nt, 2 * (int64_t)ctx().sm_count);

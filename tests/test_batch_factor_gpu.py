@@ -85,3 +85,12 @@ def test_many_instances_one_cta_each(hn, torch_cuda):
     r = solve_batch(hn, torch_cuda, ms)
     for i in list(range(0, 800, 97)) + [800]:
         check(i, *r, 1.0)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-140, 1e130])
+def test_many_panel_rows(hn, torch_cuda, scale):
+    """Enough rows below the first block for a panel row per lane (few: four lanes per row)."""
+    ms = [65, 128, 193, 257, 321] * 24
+    r = solve_batch(hn, torch_cuda, ms, scale)
+    for i in [0, 1, 2, 3, 4, 61, 117, 118, 119]:
+        check(i, *r, scale)
