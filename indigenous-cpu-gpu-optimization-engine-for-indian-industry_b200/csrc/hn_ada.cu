@@ -281,8 +281,13 @@ __global__ void __launch_bounds__(kT) ada_fill_kernel(
 // vd[e] = (A value e, d of its column): one 16-byte gather per term instead of
 // a value load plus a dependent column-index -> d chain.
 __global__ void ada_vd_kernel(int64_t nnz, const double* __restrict__ val, const int32_t* __restrict__ ci,
-                              const double* __restrict__ d, double2* __restrict__ vd) {
+                              const double* __restrict__ d, double2* __restrict__ vd, unsigned long long* maxdiag,
+                              unsigned* row_next) {
     if (!after_previous()) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // for the kernels after it: a fill of its own takes 4 us
+        *maxdiag = 0;
+        if (row_next) *row_next = 0;
+    }
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x)
         vd[e] = make_double2(val[e], __ldg(d + ci[e]));
 }
@@ -607,12 +612,9 @@ int64_t d2h_i64(const int64_t* p, cudaStream_t s) {
 
 void launch_numeric(const hn_pattern* P, const double* d, double* nval, cudaStream_t s) {
     const hn_csr* A = P->A;
-    if (A->nnz > 0) {
-        const int gv = (int)std::min<int64_t>((A->nnz + kT - 1) / kT, (int64_t)ctx().sm_count * 16);
-        launch_next(ada_vd_kernel, gv, kT, 0, s, A->nnz, A->val, A->ci, d, P->vd);
-        launched("ada_vd_kernel");
-    }
-    check_cuda(cudaMemsetAsync(P->maxdiag, 0, sizeof(unsigned long long), s), "memset maxdiag");
+    const int gv = (int)std::max<int64_t>(1, std::min<int64_t>((A->nnz + kT - 1) / kT, (int64_t)ctx().sm_count * 16));
+    launch_next(ada_vd_kernel, gv, kT, 0, s, A->nnz, A->val, A->ci, d, P->vd, P->maxdiag, P->rmap ? P->row_next : nullptr);
+    launched("ada_vd_kernel");
     if (P->nms > 0) {
         launch_next(ada_combine_kernel, (unsigned)((P->nms + 255) / 256), 256, 0, s, P->nms, P->mpos, P->mbeg,
                     P->mlist, P->vd, A->valT, P->mval, P->maxdiag);
@@ -633,7 +635,6 @@ void launch_numeric(const hn_pattern* P, const double* d, double* nval, cudaStre
         return;
     }
     if (P->rmap) {
-        check_cuda(cudaMemsetAsync(P->row_next, 0, sizeof(unsigned), s), "memset row counter");
         const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((P->m + 7) / 8, (int64_t)ctx().sm_count * 3));
         launch_next(ada_rmap_kernel, grid, kRmapT, 0, s, (int)P->m, P->order, P->row_next, A->rp, P->vd, P->ecs,
                     A->valT, A->nnz, P->rp, P->msrow, P->nms, P->rmap, P->qbits, P->mval, nval);

@@ -65,7 +65,8 @@ struct hn_batch {
     double* dense = nullptr;     // sum m_i^2
     double* dD = nullptr;        // LDL^T pivots, m
     int32_t* refine = nullptr;   // per-instance refinement flag (1 = keep sweeping)
-    int32_t* nref = nullptr;     // number of instances still refining
+    int32_t* nref = nullptr;     // instances still refining, blocks that have counted; zero between launches
+    int32_t* left_host = nullptr;  // the former, in pinned host memory
     // N as an SpMV operand (int32 row pointer copy + merge-path tables)
     int32_t* nrp = nullptr;
     int64_t ntiles = 0;
@@ -1362,43 +1363,61 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
 
 // Refinement bookkeeping per instance (refinement.cpp:15-30): with r = rhs - N x,
 // rel = max|r| / max|rhs|; an instance keeps sweeping while rel > 1e-10 and
-// sweeps remain; a sweeping instance's r is then solved and added to x.
+// sweeps remain; a sweeping instance's r is then solved and added to x. The
+// start copies the right-hand sides into x; the check's last block puts the
+// number of sweeping instances where the host reads it and clears the counts
+// (nref[0] and nref[1], the blocks that have counted). Copies and fills of
+// their own for these, with one in the assembly, took 34 us of the 421 of an
+// iteration of 48 LPs of m 50-300.
 __global__ void __launch_bounds__(kT) batch_refine_check_kernel(const int64_t* __restrict__ row_off,
                                                                 const int32_t* __restrict__ status,
                                                                 const double* __restrict__ rhs,
                                                                 const double* __restrict__ ax, double* __restrict__ r,
-                                                                int32_t* __restrict__ refine, int32_t* nref) {
+                                                                int32_t* __restrict__ refine, int32_t* nref,
+                                                                int32_t* left_host) {
     if (!after_previous()) return;
     __shared__ double sh[32];
     const int64_t i = blockIdx.x;
-    if (status[i] != ST_RUN || !refine[i]) return;
-    const int64_t r0 = row_off[i], r1 = row_off[i + 1];
-    double nb = 0.0, nr = 0.0;
-    for (int64_t k = r0 + threadIdx.x; k < r1; k += kT) {
-        const double b = rhs[k], d = b - ax[k];
-        nb = fmax(nb, fabs(b));
-        nr = fmax(nr, fabs(d));
-        r[k] = d;
+    if (status[i] == ST_RUN && refine[i]) {
+        const int64_t r0 = row_off[i], r1 = row_off[i + 1];
+        double nb = 0.0, nr = 0.0;
+        for (int64_t k = r0 + threadIdx.x; k < r1; k += kT) {
+            const double b = rhs[k], d = b - ax[k];
+            nb = fmax(nb, fabs(b));
+            nr = fmax(nr, fabs(d));
+            r[k] = d;
+        }
+        nb = block_max<kT>(nb, sh);
+        nr = block_max<kT>(nr, sh);
+        if (threadIdx.x == 0) {
+            const bool go = nb != 0.0 && nb == nb && nr / nb > 1e-10;
+            refine[i] = go ? 1 : 0;
+            if (go) atomicAdd(nref, 1);
+        }
     }
-    nb = block_max<kT>(nb, sh);
-    nr = block_max<kT>(nr, sh);
     if (threadIdx.x == 0) {
-        const bool go = nb != 0.0 && nb == nb && nr / nb > 1e-10;
-        refine[i] = go ? 1 : 0;
-        if (go) atomicAdd(nref, 1);
+        __threadfence();
+        if (atomicAdd(nref + 1, 1) == static_cast<int32_t>(gridDim.x) - 1) {
+            *left_host = atomicExch(nref, 0);
+            nref[1] = 0;
+        }
     }
 }
 
 __global__ void __launch_bounds__(kT) batch_refine_start_kernel(const int64_t* __restrict__ row_off,
                                                                 const int32_t* __restrict__ status,
-                                                                const double* __restrict__ rhs,
-                                                                int32_t* __restrict__ refine) {
+                                                                const double* rhs, int32_t* __restrict__ refine,
+                                                                double* x) {
     if (!after_previous()) return;
     __shared__ double sh[32];
     const int64_t i = blockIdx.x;
     const int64_t r0 = row_off[i], r1 = row_off[i + 1];
     double nb = 0.0;
-    for (int64_t k = r0 + threadIdx.x; k < r1; k += kT) nb = fmax(nb, fabs(rhs[k]));
+    for (int64_t k = r0 + threadIdx.x; k < r1; k += kT) {
+        const double v = rhs[k];
+        x[k] = v;
+        nb = fmax(nb, fabs(v));
+    }
     nb = block_max<kT>(nb, sh);
     // a zero or NaN right-hand side is not refined (refinement.cpp:17-18); fmax drops NaN,
     // so look for one explicitly
@@ -1442,6 +1461,7 @@ void free_batch(hn_batch* B) {
                     (void*)B->info, (void*)B->slots, (void*)B->work, (void*)B->solve_part, (void*)B->kkt, (void*)B->kkt_ref, (void*)B->ref_iter, (void*)B->xb,
                     (void*)B->zb, (void*)B->lb})
         dfree(p);
+    if (B->left_host) cudaFreeHost(B->left_host);
     delete B;
 }
 
@@ -1507,7 +1527,9 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             B->dense = dmalloc<double>(dn[K]);
             B->dD = dmalloc<double>(m);
             B->refine = dmalloc<int32_t>(K);
-            B->nref = dmalloc<int32_t>(1);
+            B->nref = dmalloc<int32_t>(2);
+            check_cuda(cudaMemsetAsync(B->nref, 0, 2 * sizeof(int32_t), s), "memset");
+            check_cuda(cudaMallocHost(reinterpret_cast<void**>(&B->left_host), sizeof(int32_t)), "cudaMallocHost");
             B->r = dmalloc<double>(m);
             B->ax = dmalloc<double>(m);
             B->nrp = dmalloc<int32_t>(m + 1);
@@ -1741,21 +1763,17 @@ int hn_batch_solve(hn_batch* B, const double* nval, const double* rhs, double* x
         require_init();
         if (!B || !nval || !rhs || !x || !status) fail(HN_ERR_INVALID_ARG, "bad arguments");
         cudaStream_t s = as_stream(stream);
-        check_cuda(cudaMemcpyAsync(x, rhs, sizeof(double) * B->m, cudaMemcpyDeviceToDevice, s), "copy rhs");
-        solve_all(B, status, nullptr, x, s);
-        launch_next(batch_refine_start_kernel, (unsigned)B->K, kT, 0, s, B->row_off, status, rhs, B->refine);
+        launch_next(batch_refine_start_kernel, (unsigned)B->K, kT, 0, s, B->row_off, status, rhs, B->refine, x);
         launched("batch_refine_start_kernel");
+        solve_all(B, status, nullptr, x, s);
         const SpmvMat N = n_mat(B, nval);
         for (int sweep = 0; sweep < 5; ++sweep) {
             spmv_launch(N, x, EpiAxpby{1.0, 0.0, B->ax}, s);
-            check_cuda(cudaMemsetAsync(B->nref, 0, sizeof(int32_t), s), "memset");
             launch_next(batch_refine_check_kernel, (unsigned)B->K, kT, 0, s, B->row_off, status, rhs, B->ax, B->r,
-                        B->refine, B->nref);
+                        B->refine, B->nref, B->left_host);
             launched("batch_refine_check_kernel");
-            int32_t left = 0;
-            check_cuda(cudaMemcpyAsync(&left, B->nref, sizeof(left), cudaMemcpyDeviceToHost, s), "D2H");
             check_cuda(cudaStreamSynchronize(s), "refine sync");
-            if (left == 0) break;
+            if (*static_cast<volatile int32_t*>(B->left_host) == 0) break;
             solve_all(B, status, B->refine, B->r, s);
             launch_next(batch_axpy_masked_kernel, (unsigned)((B->m + 255) / 256), 256, 0, s, B->m, B->row_inst,
                         status, B->refine, B->r, x);
