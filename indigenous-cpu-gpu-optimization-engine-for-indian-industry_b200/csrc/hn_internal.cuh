@@ -33,17 +33,19 @@ void check_cuda(cudaError_t e, const char* what);
 void launched(const char* what);
 
 // Every kernel of the library is launched by launch_next and begins with
-// `if (!after_previous()) return;`: its blocks may be set up while the kernel
-// before it in the stream still runs, and wait there until that one has
-// finished and its writes are visible. It lets its own successor be set up
-// only after that wait, so a kernel never starts on anything before all work
-// ahead of it is done, whatever came before it (other libraries' kernels and
-// copies included). The wait must come first, in every thread. Without this a
-// chain of short kernels spends 1-3 us between each two: products of a
-// 200 x 500 matrix and its transpose 12.3 -> 10.0 us, the 16 kernels of an
-// interior-point iteration at m = 2,000 92 -> 70 us, 35 of an iteration of 48
-// LPs of m 50-300 475 -> 444 us, the two kernels of a product with 5,000,000
-// entries 35 -> 33 us.
+// `if (!after_previous()) return;`: its launch is prepared while the kernel
+// before it in the stream still runs, its blocks start when that one's last
+// block has ended, and wait there until all its writes are visible. No kernel
+// lets its successor start earlier (griddepcontrol.launch_dependents): read-only
+// loads (ld.global.nc, what const __restrict__ arguments become) may only touch
+// memory that nobody writes while their kernel is resident, and lines that a
+// running kernel has brought into L1 since would be stale to them. It is no
+// gain either: 48 LPs of m 50-300 366 us an iteration with it, 353 without, 384
+// of m 50-2000 7,603 and 7,397. Without programmatic launches a chain of short
+// kernels spends 1-3 us between each two: products of a 200 x 500 matrix and
+// its transpose 12.3 -> 9.5 us, the 16 kernels of an interior-point iteration
+// at m = 2,000 88 -> 62 us, the two kernels of a product with 5,000,000 entries
+// 35 -> 33 us.
 template <class... P, class... A>
 void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at{};
@@ -65,7 +67,6 @@ void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t sme
 __device__ __forceinline__ bool after_previous() {
     unsigned n;
     asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%nctaid.x;" : "=r"(n) : : "memory");
-    asm volatile("griddepcontrol.launch_dependents;" : : : "memory");
     return n != 0;
 }
 
