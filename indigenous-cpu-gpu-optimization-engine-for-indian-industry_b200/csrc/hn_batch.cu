@@ -609,12 +609,12 @@ __global__ void __launch_bounds__(kT) batch_ldlt_diag_kernel(int s, const InstIn
                                                              const int32_t* __restrict__ status,
                                                              double* __restrict__ dense, double* __restrict__ dD,
                                                              double tol) {
+    const int inst = order[blockIdx.x];
+    const InstInfo in = info[inst];
     if (!after_previous()) return;
     __shared__ DiagShared sh;
     const int tid = threadIdx.x;
-    const int inst = order[blockIdx.x];
     if (status[inst] != ST_RUN) return;
-    const InstInfo in = info[inst];
     const int ld = dense_ld(in.m);
     const int k0 = s * kFb;
     const int nb = min(kFb, in.m - k0);
@@ -681,12 +681,13 @@ __device__ __forceinline__ int item_instance(const int64_t* cum, int cnt, int64_
 // way in, which there is no room for at three CTAs per SM.
 // What bounds it is the latency of a row's 64 steps and the L1 data path (16
 // bytes of L to every lane per four FP64 instructions). A lane per row has the
-// fewest instructions and is the form for panels that fill the GPU: 1,209 us
-// for the 30 panels of 384 LPs of m 50-2000 (2,156 with a chain per column);
+// fewest instructions and is the form for panels that fill the GPU: 954 us for
+// the 17 such panels of 384 LPs of m 50-2000 (all 30: 1,163; 2,156 with a chain
+// per column; 32 instead of 8 loads of L in flight give 4 of 100);
 // with two rows for two lanes, which halves the loads of L, the iteration
 // takes 8,081 us instead of 7,798, with four for four 9,007. Where a panel is
 // small a warp's 4,000 FP64 instructions per row are its time, and four lanes
-// per row take it from 16 to 8 us: an iteration of 48 LPs of m 50-300 takes
+// per row take it from 16.6 to 13.2 us: an iteration of 48 LPs of m 50-300 takes
 // 421 us instead of 450 (428 with eight lanes). The line: kPanelWide chunks,
 // about one wave of the four-lane form's CTAs. The iteration of the 384 LPs,
 // whose last panels are small, by the line: 7,798 us at none, 7,781 at 100,
@@ -708,6 +709,8 @@ __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, con
                                                                       const InstInfo* __restrict__ info,
                                                                       const int32_t* __restrict__ status, double* dense,
                                                                       const double* __restrict__ dD) {
+    const Chunk ch = chunks[blockIdx.x / (kT / (kPanelT / G))];
+    const InstInfo in = info[ch.inst];
     if (!after_previous()) return;
     constexpr int kRows = kPanelT / G, kPairs = kHalf / 2 / G;
     extern __shared__ __align__(16) double panel_sm[];
@@ -716,9 +719,7 @@ __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, con
     double* sY = sD + kFb;  // 1 / D, zero where a quotient needs the division
     double(*sRow)[kRowP] = reinterpret_cast<double(*)[kRowP]>(sY + kFb);  // half the columns of every row
     const int tid = threadIdx.x;
-    const Chunk ch = chunks[blockIdx.x / (kT / kRows)];
     if (status[ch.inst] != ST_RUN) return;
-    const InstInfo in = info[ch.inst];
     const int ld = dense_ld(in.m);
     const int k0 = s * kFb;
     const int rb = k0 + kFb + ch.local * kT + static_cast<int>(blockIdx.x % (kT / kRows)) * kRows;
@@ -730,7 +731,7 @@ __global__ void __launch_bounds__(kPanelT, 3) batch_ldlt_panel_kernel(int s, con
 #pragma unroll 4
     for (int r = line; r < rows; r += kPanelT / 16) cp_async16(&sRow[r][2 * piece], P + (int64_t)r * ld + 2 * piece);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-#pragma unroll 8
+#pragma unroll
     for (int idx = tid; idx < kFb * kFb; idx += kPanelT) {
         const int rr = idx / kFb, c = idx % kFb;
         sLt[c][rr] = c < rr ? A[(int64_t)(k0 + rr) * ld + k0 + c] : 0.0;
@@ -866,7 +867,6 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
                                                                   const int32_t* __restrict__ status,
                                                                   double* __restrict__ dense,
                                                                   const double* __restrict__ dD) {
-    if (!after_previous()) return;
     extern __shared__ __align__(16) double upd_smem[];
     __shared__ UpdTile s_tile[kUpdStages];
     double* sC = upd_smem + kUpdStages * kUpdStage;
@@ -877,9 +877,16 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
     if (warp == kUpdWarps) {
         bool out_used = false;  // the consumers still have to release the output tile
         int64_t n = 0;  // slices issued; slice i goes to stage i mod kUpdStages
+        int b = item_instance(tiles, cnt, blockIdx.x);
+        int inst = order[min(b, cnt - 1)];
+        InstInfo in = info[inst];
+        if (!after_previous()) return;
         for (int64_t idx = blockIdx.x; idx < ntiles; idx += gridDim.x) {
-            const int b = item_instance(tiles, cnt, idx);
-            const int inst = order[b];
+            if (idx != blockIdx.x) {
+                b = item_instance(tiles, cnt, idx);
+                inst = order[b];
+                in = info[inst];
+            }
             if (status[inst] != ST_RUN) continue;
             const int64_t local = idx - (b > 0 ? tiles[b - 1] : 0);
             int I = static_cast<int>(local), J = 0;
@@ -889,7 +896,6 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
                 while ((int64_t)I * (I + 1) / 2 > local) --I;
                 J = static_cast<int>(local - (int64_t)I * (I + 1) / 2);
             }
-            const InstInfo in = info[inst];
             UpdTile t;
             t.m = in.m;
             t.ld = dense_ld(t.m);
@@ -947,6 +953,7 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
         if (out_used) named_sync(kOut);
         return;
     }
+    if (!after_previous()) return;
     const int wr = (warp >> 1) * 32, wc = (warp & 1) * 32;
     const int fr = lane >> 2, fk = lane & 3, sw = (fk >> 1) ^ fr;
     int st = 0;
@@ -1040,8 +1047,12 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
 // the warps, then the chunks.
 // An instance takes part when it is iterating and, with a refine mask, still
 // refining.
-// 384 LPs of m 50-2000, both solves of an iteration: 1,139 us; 3,853 with a
-// launch per block (the factors alone are 3 GB of reads, 470 us).
+// A warp takes 16 rows of a chunk, then 16 of its second half, so that chunks
+// of up to 128 rows are one batch, and the quotients by D are formed beside the
+// products: 36 us a solve of 48 LPs of m 50-300, 42 with 32 rows in a run and
+// the quotients before them. 384 LPs of m 50-2000, both solves of an
+// iteration: 1,075 us; 3,853 with a launch per block (the factors alone are 3
+// GB of reads, 470 us).
 __device__ __forceinline__ bool solving(const int32_t* status, const int32_t* refine, int inst) {
     return status[inst] == ST_RUN && (!refine || refine[inst]);
 }
@@ -1109,16 +1120,9 @@ __device__ __forceinline__ void forward_block(const double (*sL)[kSolveP], doubl
     }
 }
 
-// x = L^-T v likewise, columns descending from nb - 1.
-__device__ __forceinline__ void backward_block(const double (*sL)[kSolveP], double& v0, double& v1, int nb, int lane) {
-    if (nb < kFb) {  // the instance's last block: one column per step
-        for (int j = nb - 1; j >= 0; --j) {
-            const double xj = __shfl_sync(0xffffffffu, j < 32 ? v0 : v1, j & 31);
-            if (lane < j) v0 -= sL[j][lane] * xj;
-            if (lane + 32 < j) v1 -= sL[j][lane + 32] * xj;
-        }
-        return;
-    }
+// x = L^-T v likewise, columns descending. Rows past the instance's last one
+// are zero in L and v and change nothing.
+__device__ __forceinline__ void backward_block(const double (*sL)[kSolveP], double& v0, double& v1, int lane) {
 #pragma unroll
     for (int j = kFb - 1; j >= 0; j -= 4) {
         double y[4];  // entries j, j - 1, j - 2, j - 3
@@ -1141,6 +1145,9 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
                        const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
                        const double* __restrict__ dense, const double* __restrict__ dD, double* work, double* part,
                        double* xv) {
+    const SolveSlot slot = slots[blockIdx.x];
+    InstInfo in = {0, 0, 0, {0, 0, 0}};
+    if (slot.inst >= 0) in = info[slot.inst];
     if (!after_previous()) return;
     extern __shared__ __align__(16) double solve_smem[];
     double(*sLb)[kFb][kSolveP] = reinterpret_cast<double(*)[kFb][kSolveP]>(solve_smem);  // two diagonal blocks
@@ -1148,10 +1155,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
     __shared__ double sacc[kT / 32][kFb];
     __shared__ double sx[kFb];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const SolveSlot slot = slots[blockIdx.x];
-    const bool on = slot.inst >= 0 && solving(status, refine, slot.inst);
-    InstInfo in = {0, 0, 0, {0, 0, 0}};
-    if (on) in = info[slot.inst];
+    if (slot.inst >= 0 && !solving(status, refine, slot.inst)) in = {0, 0, 0, {0, 0, 0}};
     const int m = in.m, ld = dense_ld(m);
     const double* L = dense + in.dn;
     double* x = xv + in.r0;
@@ -1174,7 +1178,9 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
 
     // ---- forward ----
     // batch h of this warp's rows in chunk c below the block at k0: rows first, first + 1, ...
-    auto fwd_row = [&](int k0, int c, int h) { return k0 + kFb + c * kT + warp * (kT / 8) + h * kSolveRows; };
+    auto fwd_row = [&](int k0, int c, int h) {
+        return k0 + kFb + c * kT + h * kSolveRows * (kT / 32) + warp * kSolveRows;
+    };
     auto fwd_load = [&](int k0, int c, int h) {
         const int r = fwd_row(k0, c, h);
 #pragma unroll
@@ -1203,6 +1209,10 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
             // a lane's share of each row batch: row first + mine
             const int mine = (lane >> 1);
             double xr = 0.0;
+            // y / D is formed beside the products, by the warps that more often have no rows
+            const int dr = tid - (kT - kFb);
+            const bool divides = slot.rank == 0 && dr >= 0 && dr < nb;
+            const double d = divides ? D[k0 + dr] : 0.0;
             if (!alone) {
                 const int r = fwd_row(k0, slot.rank, 0) + mine;
                 if (r < m) xr = ld_l2(x + r);
@@ -1222,27 +1232,20 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
                 forward_block(sL, v0, v1, lane);
                 sx[lane] = v0;
                 sx[lane + 32] = v1;
-                if (slot.rank == 0) {
-                    double* o = alone ? s_x : y;
-                    if (lane < nb) o[k0 + lane] = v0 / D[k0 + lane];
-                    if (lane + 32 < nb) o[k0 + lane + 32] = v1 / D[k0 + lane + 32];
-                }
             }
             __syncthreads();
+            if (divides) (alone ? s_x : y)[k0 + dr] = sx[dr] / d;
             const double x0 = sx[lane], x1 = sx[lane + 32];
             for (int c = slot.rank; k0 + kFb + c * kT < m; c += slot.size) {
 #pragma unroll 1
-                for (int h = 0; h < kSolveBatches; ++h) {
+                for (int h = 0;; ++h) {
                     double p[kSolveRows];
 #pragma unroll
                     for (int u = 0; u < kSolveRows; ++u) p[u] = p0[u] * x0 + p1[u] * x1;
                     const int row = fwd_row(k0, c, h) + mine;
                     const double old = alone ? (row < m ? s_x[row] : 0.0) : xr;
-                    int nc = c, nh = h + 1;
-                    if (nh == kSolveBatches) {
-                        nc = c + slot.size;
-                        nh = 0;
-                    }
+                    const bool more = h + 1 < kSolveBatches && fwd_row(k0, c, h + 1) < m;
+                    const int nc = more ? c : c + slot.size, nh = more ? h + 1 : 0;
                     if (k0 + kFb + nc * kT < m) {
                         fwd_load(k0, nc, nh);
                         const int r = fwd_row(k0, nc, nh) + mine;
@@ -1257,6 +1260,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
                     double t = p[0];
                     t = t + __shfl_xor_sync(0xffffffffu, t, 1);
                     if (!(lane & 1) && row < m) (alone ? s_x : x)[row] = old - t;
+                    if (!more) break;
                 }
             }
         }
@@ -1283,7 +1287,10 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
     double* part_i = part + 2 * 64 * (in.r0 / kT + (slot.inst >= 0 ? slot.inst : 0));
     int s = nblk - 1;
     if (s >= 0) {
-        if (slot.rank == 0) copy_diag_block(sLb[s & 1], L, ld, s * kFb, m - s * kFb);
+        if (slot.rank == 0) {
+            for (int u = (m - s * kFb) * kFb + tid; u < kFb * kFb; u += kT) sLb[s & 1][u / kFb][u % kFb] = 0.0;
+            copy_diag_block(sLb[s & 1], L, ld, s * kFb, m - s * kFb);
+        }
         bwd_load(s * kFb, slot.rank, 0);
     }
     for (int i = 0; i < steps; ++i, --s) {
@@ -1301,7 +1308,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
         for (int c = slot.rank; c < nch; c += slot.size) {
             double a0 = 0.0, a1 = 0.0;
 #pragma unroll 1
-            for (int h = 0; h < kSolveBatches; ++h) {
+            for (int h = 0;; ++h) {
                 const int r = bwd_row(k0, c, h);
                 double xc[kSolveRows];
 #pragma unroll
@@ -1317,12 +1324,14 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
                     a0 = row ? t0 : a0;
                     a1 = row ? t1 : a1;
                 }
-                if (h + 1 < kSolveBatches)
+                const bool more = h + 1 < kSolveBatches && bwd_row(k0, c, h + 1) < m;
+                if (more)
                     bwd_load(k0, c, h + 1);
                 else if (c + slot.size < nch)
                     bwd_load(k0, c + slot.size, 0);
                 else if (s > 0)
                     bwd_load(k0 - kFb, slot.rank, 0);
+                if (!more) break;
             }
             sacc[warp][lane] = a0;
             sacc[warp][lane + 32] = a1;
@@ -1349,7 +1358,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
             __syncthreads();
             if (warp == 0) {
                 double v0 = sx[lane], v1 = sx[lane + 32];
-                backward_block(sL, v0, v1, nb, lane);
+                backward_block(sL, v0, v1, lane);
                 double* o = alone ? s_x : x;
                 if (lane < nb) o[k0 + lane] = v0;
                 if (lane + 32 < nb) o[k0 + lane + 32] = v1;

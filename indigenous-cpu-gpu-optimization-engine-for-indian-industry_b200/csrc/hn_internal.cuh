@@ -35,7 +35,9 @@ void launched(const char* what);
 // Every kernel of the library is launched by launch_next and begins with
 // `if (!after_previous()) return;`: its launch is prepared while the kernel
 // before it in the stream still runs, its blocks start when that one's last
-// block has ended, and wait there until all its writes are visible. No kernel
+// block has ended, and wait there until all its writes are visible (a kernel
+// that finds its work in a plan which was complete before any launch using it
+// reads that first). No kernel
 // lets its successor start earlier (griddepcontrol.launch_dependents): read-only
 // loads (ld.global.nc, what const __restrict__ arguments become) may only touch
 // memory that nobody writes while their kernel is resident, and lines that a
