@@ -18,8 +18,8 @@ and keeps only when its KKT residual beats the default start.
 Every step runs on the sm_100a library (include/hn_sm100.h, hn_gnn_*):
 aggregations are its 64-wide SpMM over the device A and A^T, the forward
 layers are BF16 tcgen05 MMAs with FP32 accumulation in tensor memory, the
-backward's GEMMs BF16 mma.sync tiles, and Adam updates FP32 master weights. PyTorch only holds the device
-buffers.
+backward's two GEMMs likewise, and Adam updates FP32 master weights. PyTorch
+only holds the device buffers.
 """
 from __future__ import annotations
 

@@ -52,3 +52,20 @@ def test_threads(hn):
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not errors, errors
+
+
+def test_old_blocks_make_room(hn):
+    """Freed blocks past the cache's size push the oldest out, and the newest stay."""
+    lib = hn.load()
+    big = [alloc(hn, (200 << 20) + 4096 * i) for i in range(7)]
+    for p in big:
+        hn.check(lib.hn_free(p))
+    for n in (777 << 10, 255 << 20):
+        p = alloc(hn, n)
+        hn.check(lib.hn_free(p))
+        q = alloc(hn, n)
+        assert q.value == p.value
+        hn.check(lib.hn_free(q))
+    for p in big:
+        with pytest.raises(hn.HnError):  # idle or gone
+            hn.check(lib.hn_free(p))
