@@ -247,3 +247,32 @@ def test_row_layout_long_rows_bit_identical_to_gather(hn, torch_cuda):
         del P, nval
     for v, d in out[1:]:
         assert np.array_equal(out[0][0], v) and out[0][1] == d
+
+
+@pytest.mark.parametrize("compact", [False, True])
+@pytest.mark.parametrize("counts", [[1100, 1024, 1025, 512, 513, 511], [3] * 900, [1199] * 3 + [2] * 40])
+def test_batches_of_entries(hn, torch_cuda, counts, compact):
+    """Rows of up to some 100 entries, columns on both sides of a batch's
+    512 terms, explicit zeros: every multi slot sums its terms in column
+    order, so the values are the bits of a sum over the columns in turn."""
+    m, rng = 1200, np.random.default_rng(len(counts))
+    counts = counts + list(rng.integers(0, 20, 300))
+    n = len(counts)
+    cols = [np.sort(rng.choice(m, size=c, replace=False)) for c in counts]
+    rows, cidx = np.concatenate(cols), np.repeat(np.arange(n), counts)
+    val = rng.uniform(-1, 1, rows.size)
+    val[rng.random(rows.size) < 0.05] = 0.0
+    order = np.argsort(rows, kind="stable")
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))]).astype(np.int64)
+    lp = {"m": m, "n": n, "rp": rp, "ci": cidx[order].astype(np.int64), "val": val[order]}
+    D = rng.uniform(0.1, 10.0, n)
+    *_, rpN, ciN, vals, dyn = assemble(hn, torch_cuda, lp, D, compact=compact)
+    want, start = np.zeros((m, m)), np.concatenate([[0], np.cumsum(counts)])
+    for j in range(n):
+        r, v = cols[j], val[start[j]:start[j + 1]]
+        want[np.ix_(r, r)] += np.outer(v, v) * D[j]
+    want[np.diag_indices(m)] += dyn
+    assert np.array_equal(vals, want[np.repeat(np.arange(m), np.diff(rpN)), ciN])
+    got = np.zeros((m, m), bool)
+    got[np.repeat(np.arange(m), np.diff(rpN)), ciN] = True
+    assert not want[~got].any()
