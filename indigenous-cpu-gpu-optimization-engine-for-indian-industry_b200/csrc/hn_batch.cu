@@ -492,7 +492,7 @@ __device__ __forceinline__ double reciprocal(double d) {
 // takes A_rc -= (l_rj d_j) l_cj for j ascending, each product and difference
 // rounded, the reference's elimination order; what a thread computes above
 // the diagonal or past the block is never read.
-// 384 LPs of m 50-2000 (31 blocks): 588 us, 1,558 with the block in shared
+// 384 LPs of m 50-2000 (31 blocks): 585 us, 1,558 with the block in shared
 // memory and two barriers per pivot; one wave of blocks 15 us (41 before).
 struct DiagShared {
     double A[kFb][kFbP];

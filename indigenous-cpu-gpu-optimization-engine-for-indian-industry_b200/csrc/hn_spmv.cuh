@@ -223,8 +223,8 @@ __global__ void spmv_fixup_kernel(SpmvMat a, Epi epi) {
 // kSpmvIpt items; otherwise the last tile to finish does the fix-ups, 2 us
 // more. Two products can share a launch.
 // y = A x - b and A^T lam of 200 x 500: 10.0 us of kernels in two launches, 17.5
-// in four (24.6 -> 12.3 us a pair of calls); the one iteration's products of
-// 2,000 x 5,000: 6 us each instead of 9.5.
+// in four (24.6 -> 12.3 us a pair of calls, 9.5 with launches prepared ahead);
+// the one iteration's products of 2,000 x 5,000: 6 us each instead of 9.5.
 constexpr int64_t kSpmvSmallTiles = 2048;
 struct SmallTile {
     double prod[kSpmvTile];
