@@ -339,6 +339,9 @@ int hn_batch_factor(hn_batch* B, const double* D_dev, double reg, double singula
  * (refinement.cpp:7-37: <= 5 sweeps, 1e-10 relative). */
 int hn_batch_solve(hn_batch* B, const double* nval_dev, const double* rhs_dev, double* x_dev,
                    const int32_t* status_dev, void* stream);
+/* q = a / d, n of them, each formed as the factorisation forms its quotients
+ * (the rounded ones, by a method of its own; exported for the test of that). */
+int hn_batch_quotients(int64_t n, const double* a_dev, const double* d_dev, double* q_dev, void* stream);
 /* per-instance step lengths (:134-142) and non-finite guard (:617-627). */
 int hn_batch_steps(hn_batch* B, const double* x_dev, const double* dx_dev, const double* z_dev,
                    const double* dz_dev, const double* dlam_dev, double* scal_dev, int32_t* status_dev, void* stream);

@@ -118,6 +118,7 @@ SIGNATURES = {
     "hn_batch_residuals": [_vp, _vp] + [_vp] * 13 + [C.c_int, C.c_double, C.c_double, _vp],
     "hn_batch_factor": [_vp, _vp, C.c_double, C.c_double, _vp, _vp, _vp],
     "hn_batch_solve": [_vp, _vp, _vp, _vp, _vp, _vp],
+    "hn_batch_quotients": [_i64, _vp, _vp, _vp, _vp],
     "hn_batch_steps": [_vp] + [_vp] * 7 + [_vp],
     "hn_batch_corrector": [_vp, _vp] + [_vp] * 9 + [_vp],
     "hn_batch_update": [_vp] + [_vp] * 9 + [C.c_int, _vp],
