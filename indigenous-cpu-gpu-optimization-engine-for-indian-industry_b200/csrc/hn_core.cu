@@ -106,7 +106,7 @@ Pool& pool() {
 }  // namespace
 
 void* pool_alloc(size_t bytes) {
-    const size_t size = (bytes + 511) & ~size_t(511);
+    const size_t size = bytes > SIZE_MAX - 511 ? bytes : (bytes + 511) & ~size_t(511);  // the former fails below
     int device = 0;
     check_cuda(cudaGetDevice(&device), "cudaGetDevice");
     if (void* p = pool().take(device, size)) return p;
