@@ -127,6 +127,16 @@ void* pool_alloc(size_t bytes) {
     return p;
 }
 
+// What cudaFree does beside freeing: it waits for the work on every stream, and
+// is refused where a stream capture forbids it. cudaDeviceSynchronize is
+// refused beside any capture, and breaks it, so an allocation of no use is made
+// and freed: 2.7 us (1.6 the synchronisation).
+cudaError_t wait_as_free() {
+    void* q = nullptr;
+    const cudaError_t e = cudaMalloc(&q, 512);
+    return e == cudaSuccess ? cudaFree(q) : e;
+}
+
 cudaError_t pool_free(void* p) {
     Pool& P = pool();
     PoolBlock b{0, -1};
@@ -141,8 +151,15 @@ cudaError_t pool_free(void* p) {
     }
     int device = -1;
     if (b.device < 0 || b.bytes > kPoolBlock || cudaGetDevice(&device) != cudaSuccess || device != b.device ||
-        cudaDeviceSynchronize() != cudaSuccess)
-        return cudaFree(p);
+        wait_as_free() != cudaSuccess) {
+        cudaGetLastError();  // this call's result is cudaFree's
+        const cudaError_t e = cudaFree(p);
+        if (e != cudaSuccess && b.device >= 0) {
+            std::lock_guard<std::mutex> lk(P.mu);
+            P.live.emplace(p, b);
+        }
+        return e;
+    }
     std::vector<void*> out;
     {
         std::lock_guard<std::mutex> lk(P.mu);
