@@ -1,6 +1,8 @@
 // Context, error plumbing, device-memory helpers, scans and BLAS-1 kernels.
 #include "hn_internal.cuh"
 
+#include <cuda.h>
+
 #include <cstring>
 #include <map>
 #include <vector>
@@ -46,14 +48,45 @@ void require_init() {
 // ones freed longest ago making room (blocks of a model that is gone would
 // otherwise keep the next one's out: after a batch of 384 LPs a 20,000-row
 // set-up took 5.1 ms, 2.9 now). All go back when an allocation fails for lack
-// of memory and in hn_shutdown. Any thread may allocate or free.
+// of memory and in hn_shutdown. Any thread may allocate or free. A block is
+// known by its allocation's id: one that was freed past the library and whose
+// address the driver gave to somebody else is not taken for it.
 namespace {
+// The driver's id of the allocation that p lies in, unique in the process's
+// life; 0 if there is none (0.1 us).
+unsigned long long allocation_id(const void* p) {
+    using Get = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Get>(f);
+    }();
+    if (!get) return 0;
+    const auto at = reinterpret_cast<CUdeviceptr>(p);
+    unsigned long long id = 0;
+    CUresult r = get(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, at);
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {  // a thread's first call; the context becomes its own
+        int device = 0;
+        if (cudaGetDevice(&device) == cudaSuccess) cudaSetDevice(device);
+        r = get(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, at);
+    }
+    return r == CUDA_SUCCESS ? id : 0;
+}
+
 constexpr size_t kPoolBlock = size_t(256) << 20, kPoolBytes = size_t(1) << 30;
 struct PoolBlock {
     size_t bytes;
     int device;
-    uint64_t freed = 0;  // when, in frees
+    unsigned long long id;  // allocation_id
+    uint64_t freed = 0;     // when, in frees
 };
+// Frees an idle block, unless it is gone already.
+cudaError_t give_back(void* p, const PoolBlock& b) { return allocation_id(p) == b.id ? cudaFree(p) : cudaSuccess; }
 struct Pool {
     std::mutex mu;
     std::unordered_map<void*, PoolBlock> live, idle;
@@ -62,37 +95,34 @@ struct Pool {
     size_t idle_bytes = 0;
     uint64_t frees = 0;
 
-    // the entry of by_size is the caller's to erase
-    void forget(void* p) {
+    // takes an idle block out
+    PoolBlock remove(void* p) {
         auto it = idle.find(p);
-        idle_bytes -= it->second.bytes;
-        by_age.erase(it->second.freed);
+        const PoolBlock b = it->second;
         idle.erase(it);
-    }
-    // takes the oldest idle block out
-    void* evict() {
-        void* p = by_age.begin()->second;
-        const PoolBlock b = idle[p];
+        idle_bytes -= b.bytes;
+        by_age.erase(b.freed);
         auto range = by_size.equal_range({b.device, b.bytes});
         while (range.first->second != p) ++range.first;
         by_size.erase(range.first);
-        forget(p);
-        return p;
+        return b;
     }
     void* take(int device, size_t bytes) {
         std::lock_guard<std::mutex> lk(mu);
-        auto it = by_size.lower_bound({device, bytes});
-        if (it == by_size.end() || it->first.first != device || it->first.second > bytes + bytes / 4 + 4096)
-            return nullptr;
-        void* p = it->second;
-        live[p] = idle[p];
-        by_size.erase(it);
-        forget(p);
-        return p;
+        for (;;) {
+            auto it = by_size.lower_bound({device, bytes});
+            if (it == by_size.end() || it->first.first != device || it->first.second > bytes + bytes / 4 + 4096)
+                return nullptr;
+            void* p = it->second;
+            const PoolBlock b = remove(p);
+            if (allocation_id(p) != b.id) continue;  // freed past the library
+            live[p] = b;
+            return p;
+        }
     }
     void release() {
         std::lock_guard<std::mutex> lk(mu);
-        for (auto& kv : idle) cudaFree(kv.first);
+        for (auto& kv : idle) give_back(kv.first, kv.second);
         idle.clear();
         by_size.clear();
         by_age.clear();
@@ -122,8 +152,9 @@ void* pool_alloc(size_t bytes) {
         fail(e == cudaErrorMemoryAllocation ? HN_ERR_OUT_OF_MEMORY : HN_ERR_CUDA,
              std::string("cudaMalloc of ") + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
     }
+    const PoolBlock b{size, device, allocation_id(p)};
     std::lock_guard<std::mutex> lk(pool().mu);
-    pool().live[p] = PoolBlock{size, device};
+    pool().live[p] = b;
     return p;
 }
 
@@ -139,18 +170,23 @@ cudaError_t wait_as_free() {
 
 cudaError_t pool_free(void* p) {
     Pool& P = pool();
-    PoolBlock b{0, -1};
+    PoolBlock b{0, -1, 0};
+    const unsigned long long id = allocation_id(p);
     {
         std::lock_guard<std::mutex> lk(P.mu);
-        if (P.idle.count(p)) return cudaErrorInvalidValue;  // freed before
+        auto free_one = P.idle.find(p);
+        if (free_one != P.idle.end()) {
+            if (free_one->second.id == id) return cudaErrorInvalidValue;  // freed before
+            P.remove(p);
+        }
         auto it = P.live.find(p);
         if (it != P.live.end()) {
-            b = it->second;
+            if (it->second.id == id) b = it->second;
             P.live.erase(it);
         }
     }
     int device = -1;
-    if (b.device < 0 || b.bytes > kPoolBlock || cudaGetDevice(&device) != cudaSuccess || device != b.device ||
+    if (b.device < 0 || b.id == 0 || b.bytes > kPoolBlock || cudaGetDevice(&device) != cudaSuccess || device != b.device ||
         wait_as_free() != cudaSuccess) {
         cudaGetLastError();  // this call's result is cudaFree's
         const cudaError_t e = cudaFree(p);
@@ -160,10 +196,13 @@ cudaError_t pool_free(void* p) {
         }
         return e;
     }
-    std::vector<void*> out;
+    std::vector<std::pair<void*, PoolBlock>> out;  // the oldest
     {
         std::lock_guard<std::mutex> lk(P.mu);
-        while (P.idle_bytes + b.bytes > kPoolBytes) out.push_back(P.evict());
+        while (P.idle_bytes + b.bytes > kPoolBytes) {
+            void* o = P.by_age.begin()->second;
+            out.emplace_back(o, P.remove(o));
+        }
         b.freed = P.frees++;
         P.idle[p] = b;
         P.by_size.emplace(std::pair{b.device, b.bytes}, p);
@@ -171,8 +210,8 @@ cudaError_t pool_free(void* p) {
         P.idle_bytes += b.bytes;
     }
     cudaError_t e = cudaSuccess;
-    for (void* o : out) {
-        const cudaError_t eo = cudaFree(o);
+    for (auto& o : out) {
+        const cudaError_t eo = give_back(o.first, o.second);
         if (e == cudaSuccess) e = eo;
     }
     return e;

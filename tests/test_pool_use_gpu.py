@@ -78,3 +78,68 @@ def test_free_waits_for_every_stream(hn, torch_cuda):
     hn.check(hn.load().hn_memset(p, 1, n, s.cuda_stream))
     hn.check(hn.load().hn_free(p))
     assert s.query()
+
+
+@pytest.fixture
+def cudart(torch_cuda):
+    """The CUDA runtime that torch loaded: another user of the same device."""
+    rt = C.CDLL("libcudart.so.12")
+    rt.cudaMalloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+    rt.cudaFree.argtypes = [C.c_void_p]
+    yield rt
+    rt.cudaGetLastError()
+
+
+def test_block_freed_past_the_library(hn, cudart):
+    """cudaFree on a block of hn_malloc: the library does not take the address
+    for its block any more, freed or not, nor hand it out."""
+    lib, n = hn.load(), 3 << 20
+    p = alloc(hn, n)
+    assert cudart.cudaFree(p) == 0
+    assert lib.hn_free(p) != 0  # nothing there to free
+    idle = alloc(hn, n)
+    hn.check(lib.hn_free(idle))
+    assert cudart.cudaFree(idle) == 0
+    q, back = alloc(hn, n), (C.c_ubyte * n)()
+    hn.check(lib.hn_memset(q, 5, n, None))
+    hn.check(lib.hn_memcpy_d2h(back, q, n, None))
+    assert set(bytes(back)) == {5}
+    hn.check(lib.hn_free(q))
+    assert lib.hn_free(q) != 0
+
+
+@pytest.mark.parametrize("size", [3 << 20, 2 << 20, 4 << 20])
+@pytest.mark.parametrize("state", ["live", "idle"])
+def test_address_given_to_another(hn, cudart, size, state):
+    """A block of 3 MB was freed past the library and the driver gave its
+    address to another allocation: hn_free frees that one, as cudaFree does."""
+    lib, n, others = hn.load(), 3 << 20, []
+    p = alloc(hn, n)
+    if state == "idle":
+        hn.check(lib.hn_free(p))
+    assert cudart.cudaFree(p) == 0
+    for _ in range(8):
+        q = C.c_void_p()
+        assert cudart.cudaMalloc(C.byref(q), size) == 0
+        others.append(q)
+    hn.check(lib.hn_memset(others[0], 1, size, None))
+    if state == "idle":  # not handed out while another has it
+        r = alloc(hn, n)
+        assert all(abs(r.value - q.value) >= min(n, size) for q in others)
+        hn.check(lib.hn_free(r))
+    for q in others:
+        hn.check(lib.hn_free(q))
+        assert cudart.cudaFree(q) != 0  # gone, not kept
+
+
+def test_a_threads_first_call(hn):
+    """A thread whose first call this is finds the freed blocks, and double frees."""
+    lib, n, got = hn.load(), 5 << 20, []
+    p = alloc(hn, n)
+    hn.check(lib.hn_free(p))
+    for call in (lambda: got.append(alloc(hn, n).value), lambda: got.append(lib.hn_free(p)),
+                 lambda: got.append(lib.hn_free(p) != 0)):
+        t = threading.Thread(target=call)
+        t.start()
+        t.join()
+    assert got == [p.value, 0, True]
