@@ -680,11 +680,8 @@ __global__ void ada_reg_kernel(int m, const int64_t* __restrict__ diag_pos, doub
 
 void free_pattern(hn_pattern* P) {
     if (!P) return;
-    for (void* p : {(void*)P->rp, (void*)P->ci, (void*)P->diag_pos, (void*)P->maxdiag, (void*)P->gmap,
-                    (void*)P->mpos, (void*)P->mbeg, (void*)P->mlist, (void*)P->vd, (void*)P->mval, (void*)P->tq,
-                    (void*)P->smap, (void*)P->msrow, (void*)P->rmap, (void*)P->ecs, (void*)P->order,
-                    (void*)P->row_next})
-        dfree(p);
+    dfree({P->rp, P->ci, P->diag_pos, P->maxdiag, P->gmap, P->mpos, P->mbeg, P->mlist, P->vd, P->mval, P->tq, P->smap,
+           P->msrow, P->rmap, P->ecs, P->order, P->row_next});
     delete P;
 }
 
@@ -901,15 +898,11 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
             }
             check_cuda(cudaStreamSynchronize(s), "symbolic sync");
         } catch (...) {
-            for (void* p : {(void*)nq, (void*)nms, (void*)nmq, (void*)mcnt, (void*)wbase, (void*)wcount,
-                            (void*)wmax_d, (void*)tqa})
-                dfree(p);
+            dfree({nq, nms, nmq, mcnt, wbase, wcount, wmax_d, tqa});
             free_pattern(P);
             throw;
         }
-        for (void* p : {(void*)nq, (void*)nms, (void*)nmq, (void*)mcnt, (void*)wbase, (void*)wcount, (void*)wmax_d,
-                        (void*)tqa})
-            dfree(p);
+        dfree({nq, nms, nmq, mcnt, wbase, wcount, wmax_d, tqa});
         *out = P;
     });
 }

@@ -1477,13 +1477,10 @@ __global__ void narrow_rp_kernel(int64_t n, const int64_t* __restrict__ in, int3
 
 void free_batch(hn_batch* B) {
     if (!B) return;
-    for (void* p : {(void*)B->row_off, (void*)B->col_off, (void*)B->row_inst, (void*)B->dn_off, (void*)B->order,
-                    (void*)B->dense, (void*)B->dD, (void*)B->refine, (void*)B->nref, (void*)B->nrp,
-                    (void*)B->tile_row, (void*)B->tile_nz, (void*)B->carry_row, (void*)B->head_row,
-                    (void*)B->carry_val, (void*)B->head_val, (void*)B->r, (void*)B->ax, (void*)B->step_tiles, (void*)B->chunks,
-                    (void*)B->info, (void*)B->slots, (void*)B->work, (void*)B->solve_part, (void*)B->kkt, (void*)B->kkt_ref, (void*)B->ref_iter, (void*)B->xb,
-                    (void*)B->zb, (void*)B->lb})
-        dfree(p);
+    dfree({B->row_off, B->col_off, B->row_inst, B->dn_off, B->order, B->dense, B->dD, B->refine, B->nref, B->nrp,
+           B->tile_row, B->tile_nz, B->carry_row, B->head_row, B->carry_val, B->head_val, B->r, B->ax, B->step_tiles,
+           B->chunks, B->info, B->slots, B->work, B->solve_part, B->kkt, B->kkt_ref, B->ref_iter, B->xb, B->zb,
+           B->lb});
     if (B->left_host) cudaFreeHost(B->left_host);
     delete B;
 }

@@ -161,22 +161,34 @@ void* pool_alloc(size_t bytes) {
 // What cudaFree does beside freeing: it waits for the work on every stream, and
 // is refused where a stream capture forbids it. cudaDeviceSynchronize is
 // refused beside any capture, and breaks it, so an allocation of no use is made
-// and freed: 2.7 us (1.6 the synchronisation).
+// and freed: 2.7 us (1.6 the synchronisation), once for blocks freed together.
 cudaError_t wait_as_free() {
     void* q = nullptr;
     const cudaError_t e = cudaMalloc(&q, 512);
     return e == cudaSuccess ? cudaFree(q) : e;
 }
 
-cudaError_t pool_free(void* p) {
+cudaError_t pool_free(void* const* ps, size_t n) {
     Pool& P = pool();
-    PoolBlock b{0, -1, 0};
-    const unsigned long long id = allocation_id(p);
-    {
+    cudaError_t e = cudaSuccess;
+    auto done = [&](cudaError_t one) {
+        if (e == cudaSuccess) e = one;
+    };
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) cudaGetLastError();
+    std::vector<std::pair<void*, PoolBlock>> keep, out;  // for the cache; for the driver
+    for (size_t i = 0; i < n; ++i) {
+        void* p = ps[i];
+        if (!p) continue;
+        const unsigned long long id = allocation_id(p);
+        PoolBlock b{0, -1, 0};
         std::lock_guard<std::mutex> lk(P.mu);
         auto free_one = P.idle.find(p);
         if (free_one != P.idle.end()) {
-            if (free_one->second.id == id) return cudaErrorInvalidValue;  // freed before
+            if (free_one->second.id == id) {  // freed before
+                done(cudaErrorInvalidValue);
+                continue;
+            }
             P.remove(p);
         }
         auto it = P.live.find(p);
@@ -184,36 +196,37 @@ cudaError_t pool_free(void* p) {
             if (it->second.id == id) b = it->second;
             P.live.erase(it);
         }
+        (b.id != 0 && b.device == device && b.bytes <= kPoolBlock ? keep : out).emplace_back(p, b);
     }
-    int device = -1;
-    if (b.device < 0 || b.id == 0 || b.bytes > kPoolBlock || cudaGetDevice(&device) != cudaSuccess || device != b.device ||
-        wait_as_free() != cudaSuccess) {
-        cudaGetLastError();  // this call's result is cudaFree's
-        const cudaError_t e = cudaFree(p);
-        if (e != cudaSuccess && b.device >= 0) {
+    if (!keep.empty() && wait_as_free() != cudaSuccess) {
+        cudaGetLastError();  // the results are cudaFree's
+        out.insert(out.end(), keep.begin(), keep.end());
+        keep.clear();
+    }
+    for (auto& o : out) {
+        const cudaError_t one = cudaFree(o.first);
+        done(one);
+        if (one != cudaSuccess && o.second.id != 0) {
             std::lock_guard<std::mutex> lk(P.mu);
-            P.live.emplace(p, b);
+            P.live.emplace(o);
         }
-        return e;
     }
-    std::vector<std::pair<void*, PoolBlock>> out;  // the oldest
+    std::vector<std::pair<void*, PoolBlock>> old;
     {
         std::lock_guard<std::mutex> lk(P.mu);
-        while (P.idle_bytes + b.bytes > kPoolBytes) {
-            void* o = P.by_age.begin()->second;
-            out.emplace_back(o, P.remove(o));
+        for (auto& [p, b] : keep) {
+            while (P.idle_bytes + b.bytes > kPoolBytes) {
+                void* o = P.by_age.begin()->second;
+                old.emplace_back(o, P.remove(o));
+            }
+            b.freed = P.frees++;
+            P.idle[p] = b;
+            P.by_size.emplace(std::pair{b.device, b.bytes}, p);
+            P.by_age[b.freed] = p;
+            P.idle_bytes += b.bytes;
         }
-        b.freed = P.frees++;
-        P.idle[p] = b;
-        P.by_size.emplace(std::pair{b.device, b.bytes}, p);
-        P.by_age[b.freed] = p;
-        P.idle_bytes += b.bytes;
     }
-    cudaError_t e = cudaSuccess;
-    for (auto& o : out) {
-        const cudaError_t eo = give_back(o.first, o.second);
-        if (e == cudaSuccess) e = eo;
-    }
+    for (auto& o : old) done(give_back(o.first, o.second));
     return e;
 }
 
@@ -429,11 +442,7 @@ int hn_shutdown(void) {
         cudaDeviceSynchronize();
         std::lock_guard<std::mutex> lk(c.mu);
         for (auto& kv : c.ws) {
-            dfree(kv.second.partials);
-            dfree(kv.second.counter);
-            dfree(kv.second.select);
-            dfree(kv.second.price);
-            dfree(kv.second.staging_d);
+            dfree({kv.second.partials, kv.second.counter, kv.second.select, kv.second.price, kv.second.staging_d});
             if (kv.second.staging_h) cudaFreeHost(kv.second.staging_h);
         }
         c.ws.clear();
@@ -488,7 +497,7 @@ int hn_malloc(void** ptr_dev, size_t bytes) {
 int hn_free(void* p) {
     return guard("hn_free", [&] {
         require_init();
-        if (p) check_cuda(pool_free(p), "cudaFree");
+        check_cuda(pool_free(&p, 1), "cudaFree");
     });
 }
 

@@ -241,16 +241,8 @@ void build_tiles(const int32_t* rp, int64_t m, int64_t nnz, int64_t& ntiles, int
 }
 
 void free_transpose(hn_csr* A) {
-    dfree(A->rpT);
-    dfree(A->ciT);
-    dfree(A->valT);
-    dfree(A->permT);
-    dfree(A->tile_row_t);
-    dfree(A->tile_nz_t);
-    dfree(A->carry_row_t);
-    dfree(A->carry_val_t);
-    dfree(A->head_row_t);
-    dfree(A->head_val_t);
+    dfree({A->rpT, A->ciT, A->valT, A->permT, A->tile_row_t, A->tile_nz_t, A->carry_row_t, A->carry_val_t,
+           A->head_row_t, A->head_val_t});
     A->rpT = A->ciT = A->permT = A->tile_row_t = A->tile_nz_t = A->carry_row_t = A->head_row_t =
         nullptr;
     A->valT = A->carry_val_t = A->head_val_t = nullptr;
@@ -337,9 +329,7 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
             launch_next(histogram_kernel, blocks(nnz), 256, 0, s, nnz, kA, cnt);
             launched("histogram_kernel");
         }
-        dfree(run_sum);
-        dfree(keep);
-        dfree(kA);
+        dfree({run_sum, keep, kA});
     } else {
         int32_t* pos = dmalloc<int32_t>(nnz);
         scan_exclusive_i32(keep, pos, nnz, s);
@@ -357,20 +347,11 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
         check_cuda(cudaStreamSynchronize(s), "transpose sync");
         A->permT = nullptr;
         A->t_compacted = true;
-        dfree(pos);
-        dfree(keyT);
-        dfree(ci_raw);
-        dfree(val_raw);
-        dfree(run_sum);
-        dfree(keep);
-        dfree(kA);
-        dfree(vA);
+        dfree({pos, keyT, ci_raw, val_raw, run_sum, keep, kA, vA});
     }
     scan_exclusive_i32(cnt, A->rpT, n + 1, s);
     check_cuda(cudaStreamSynchronize(s), "transpose sync");
-    dfree(cnt);
-    dfree(row_of);
-    dfree(kept_d);
+    dfree({cnt, row_of, kept_d});
     build_tiles(A->rpT, n, A->nnz_t, A->ntiles_t, A->tile_row_t, A->tile_nz_t, A->carry_row_t,
                 A->carry_val_t, A->head_row_t, A->head_val_t, A->short_heads[1], s);
     check_cuda(cudaStreamSynchronize(s), "tiles sync");
@@ -380,16 +361,8 @@ void build_transpose(hn_csr* A, cudaStream_t s) {
 void free_csr(hn_csr* A) {
     if (!A) return;
     free_transpose(A);
-    dfree(A->perm[0]);
-    dfree(A->rp);
-    dfree(A->ci);
-    dfree(A->val);
-    dfree(A->tile_row);
-    dfree(A->tile_nz);
-    dfree(A->carry_row);
-    dfree(A->carry_val);
-    dfree(A->head_row);
-    dfree(A->head_val);
+    dfree({A->perm[0], A->rp, A->ci, A->val, A->tile_row, A->tile_nz, A->carry_row, A->carry_val, A->head_row,
+           A->head_val});
     delete A;
 }
 
@@ -505,14 +478,12 @@ void autotune(hn_csr* A, cudaStream_t s) {
         } catch (...) {
             if (e0) cudaEventDestroy(e0);
             if (e1) cudaEventDestroy(e1);
-            dfree(x);
-            dfree(y);
+            dfree({x, y});
             throw;
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        dfree(x);
-        dfree(y);
+        dfree({x, y});
     }
 }
 
@@ -599,9 +570,7 @@ void coo_to_csr(int64_t m, int64_t n, int64_t nnz, const int32_t* r, const int32
     int32_t* rp = dmalloc<int32_t>(m + 1);
     scan_exclusive_i32(cnt, rp, m + 1, s);
     check_cuda(cudaStreamSynchronize(s), "coo sync");
-    for (void* p : {(void*)kA, (void*)kB, (void*)vA, (void*)vB, (void*)val_raw, (void*)run_sum, (void*)kept_d,
-                    (void*)pos, (void*)key, (void*)cnt})
-        dfree(p);
+    dfree({kA, kB, vA, vB, val_raw, run_sum, kept_d, pos, key, cnt});
     *rp_out = rp;
     *ci_out = ci;
     *val_out = val;
@@ -697,9 +666,7 @@ int hn_csr_create_coo(int64_t m, int64_t n, int64_t count, const int64_t* rows, 
             A->m = m;
             A->n = n;
             coo_to_csr(m, n, count, dr, dc, dv, &A->rp, &A->ci, &A->val, &A->nnz, s);
-            dfree(dr);
-            dfree(dc);
-            dfree(dv);
+            dfree({dr, dc, dv});
             dr = dc = nullptr;
             dv = nullptr;
             build_tiles(A->rp, m, A->nnz, A->ntiles, A->tile_row, A->tile_nz, A->carry_row, A->carry_val,
@@ -708,9 +675,7 @@ int hn_csr_create_coo(int64_t m, int64_t n, int64_t count, const int64_t* rows, 
             check_cuda(cudaStreamSynchronize(s), "hn_csr_create_coo sync");
             if (!(flags & HN_CSR_NO_AUTOTUNE)) autotune(A, s);
         } catch (...) {
-            dfree(dr);
-            dfree(dc);
-            dfree(dv);
+            dfree({dr, dc, dv});
             free_csr(A);
             throw;
         }

@@ -114,9 +114,9 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 // Device memory of the library's objects, from a bounded cache of freed
 // blocks (hn_core.cu). pool_free waits for the device, as cudaFree does, so a
-// block in the cache is idle on every stream.
+// block in the cache is idle on every stream; null pointers are passed over.
 void* pool_alloc(size_t bytes);
-cudaError_t pool_free(void* p);
+cudaError_t pool_free(void* const* ps, size_t n);
 void pool_release();  // gives the cached blocks back
 
 template <class T>
@@ -124,9 +124,8 @@ T* dmalloc(size_t count) {
     if (count == 0) count = 1;
     return static_cast<T*>(pool_alloc(count * sizeof(T)));
 }
-inline void dfree(void* p) {
-    if (p) pool_free(p);
-}
+inline void dfree(std::initializer_list<void*> ps) { pool_free(ps.begin(), ps.size()); }
+inline void dfree(void* p) { dfree({p}); }
 
 inline int grid_for(int64_t n, int threads, int cap) {
     int64_t g = (n + threads - 1) / threads;
