@@ -73,7 +73,8 @@ int hn_shutdown(void);
 /* Thread-local text of the last failure (CudaDriverBackend::last_error_). */
 const char* hn_last_error(void);
 /* Device name and memory (CudaDriverBackend::name/device_memory/free_memory,
- * gpu_backend.cpp:150-153,249-259). */
+ * gpu_backend.cpp:150-153,249-259). free_mem counts the library's cached
+ * blocks (hn_trim) as free. */
 int hn_device_info(hn_device_info_t* out);
 /* Kernel launch counter (IComputeBackend::gpu_kernel_executions,
  * gpu_backend.hpp:47-50). */
@@ -88,7 +89,15 @@ int hn_fault_inject(int64_t after_calls, int status);
 /* ---- device memory for callers without a CUDA runtime ----
  * (DriverApi::allocate/free/copy_h2d/copy_d2h/memset_d8, cuda_driver.hpp:44-93) */
 int hn_malloc(void** ptr_dev, size_t bytes);
+/* Waits for the device, as cudaFree does. Freed blocks (and those of destroyed
+ * handles) of up to 256 MB each, 1 GB in all, stay with the library for its
+ * next allocations; to other allocators on the device they are in use until
+ * hn_trim. Also frees what cudaMalloc gave. */
 int hn_free(void* ptr_dev);
+/* Gives the blocks that the library keeps back to the device, for another
+ * allocator (PyTorch's) to use. The library does so by itself where an
+ * allocation of its own would fail, and in hn_shutdown. */
+int hn_trim(void);
 int hn_memcpy_h2d(void* dst_dev, const void* src_host, size_t bytes, void* stream);
 int hn_memcpy_d2h(void* dst_host, const void* src_dev, size_t bytes, void* stream);
 int hn_memcpy_d2d(void* dst_dev, const void* src_dev, size_t bytes, void* stream);

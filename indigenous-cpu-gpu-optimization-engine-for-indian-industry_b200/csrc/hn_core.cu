@@ -48,7 +48,7 @@ void require_init() {
 // ones freed longest ago making room (blocks of a model that is gone would
 // otherwise keep the next one's out: after a batch of 384 LPs a 20,000-row
 // set-up took 5.1 ms, 2.9 now). All go back when an allocation fails for lack
-// of memory and in hn_shutdown. Any thread may allocate or free. A block is
+// of memory, in hn_trim and in hn_shutdown. Any thread may allocate or free. A block is
 // known by its allocation's id: one that was freed past the library and whose
 // address the driver gave to somebody else is not taken for it.
 namespace {
@@ -119,6 +119,13 @@ struct Pool {
             live[p] = b;
             return p;
         }
+    }
+    size_t idle_on(int device) {
+        std::lock_guard<std::mutex> lk(mu);
+        size_t bytes = 0;
+        for (auto& kv : idle)
+            if (kv.second.device == device) bytes += kv.second.bytes;
+        return bytes;
     }
     void release() {
         std::lock_guard<std::mutex> lk(mu);
@@ -465,6 +472,7 @@ int hn_device_info(hn_device_info_t* out) {
         out->cc_major = p.major;
         out->cc_minor = p.minor;
         check_cuda(cudaMemGetInfo(&out->free_mem, &out->total_mem), "cudaMemGetInfo");
+        out->free_mem += pool().idle_on(out->device);  // the next hn_malloc's
     });
 }
 
@@ -498,6 +506,13 @@ int hn_free(void* p) {
     return guard("hn_free", [&] {
         require_init();
         check_cuda(pool_free(&p, 1), "cudaFree");
+    });
+}
+
+int hn_trim(void) {
+    return guard("hn_trim", [&] {
+        require_init();
+        pool_release();
     });
 }
 

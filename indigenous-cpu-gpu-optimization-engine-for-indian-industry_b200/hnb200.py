@@ -54,6 +54,7 @@ SIGNATURES = {
     "hn_reset_stats": [],
     "hn_fault_inject": [_i64, C.c_int],
     "hn_malloc": [C.POINTER(C.c_void_p), C.c_size_t],
+    "hn_trim": [],
     "hn_free": [_vp],
     "hn_memcpy_h2d": [_vp, _vp, C.c_size_t, _vp],
     "hn_memcpy_d2h": [_vp, _vp, C.c_size_t, _vp],

@@ -143,3 +143,21 @@ def test_a_threads_first_call(hn):
         t.start()
         t.join()
     assert got == [p.value, 0, True]
+
+
+def test_freed_memory_is_free(hn, torch_cuda):
+    """free_mem after a free is what it was before the allocation, and after
+    hn_trim the device has the memory for everybody."""
+    lib, n = hn.load(), 200 << 20
+    device_free = lambda: torch_cuda.cuda.mem_get_info()[0]  # noqa: E731
+    hn.check(lib.hn_trim())
+    before = hn.device_info().free_mem
+    assert before == device_free()
+    p = alloc(hn, n)
+    assert hn.device_info().free_mem <= before - n
+    hn.check(lib.hn_free(p))
+    assert hn.device_info().free_mem == before
+    hn.check(lib.hn_trim())
+    assert hn.device_info().free_mem == before == device_free()
+    q = alloc(hn, n)  # and goes on
+    hn.check(lib.hn_free(q))
