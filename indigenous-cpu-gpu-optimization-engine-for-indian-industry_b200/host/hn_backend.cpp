@@ -81,7 +81,7 @@ void B200Backend::initialize() {
 }
 
 void B200Backend::release() {
-    for (auto& kv : cache_) hn_csr_destroy(kv.second.h);
+    for (auto& r : cache_) hn_csr_destroy(r.h);
     cache_.clear();
     if (dev_buf_) hn_free(dev_buf_);
     dev_buf_ = nullptr;
@@ -99,28 +99,44 @@ void B200Backend::require(const char* op) const {
 
 B200Backend::Resident& B200Backend::resident(const std::vector<double>& values,
                                              const std::vector<std::size_t>& col_indices,
-                                             const std::vector<std::size_t>& row_ptr, std::size_t ncols) {
-    const std::size_t nrows = row_ptr.size() - 1;
+                                             const std::vector<std::size_t>& row_ptr, std::size_t ncols,
+                                             bool wider) {
+    const std::size_t nrows = row_ptr.size() - 1, nnz = values.size();
     const uint64_t fp = fingerprint(values, col_indices, row_ptr);
-    auto it = cache_.find(values.data());
-    if (it != cache_.end()) {
-        Resident& r = it->second;
-        if (r.nnz == values.size() && r.nrows == nrows && r.ncols >= ncols && r.fingerprint == fp) return r;
-        hn_csr_destroy(r.h);
-        cache_.erase(it);
+    for (auto it = cache_.begin(); it != cache_.end(); ++it) {
+        if (it->fingerprint != fp || it->nnz != nnz || it->nrows != nrows) continue;
+        const std::size_t n = ncols > it->used ? ncols : it->used;
+        if (it->ncols != n && !(wider && it->ncols > n)) continue;
+        cache_.splice(cache_.begin(), cache_, it);  // the last used one first
+        cache_.front().host = values.data();
+        return cache_.front();
     }
-    std::size_t n = ncols;
-    for (std::size_t c : col_indices) n = c + 1 > n ? c + 1 : n;
+    // the buffer held another matrix before: that one is gone
+    for (auto it = cache_.begin(); it != cache_.end();) {
+        if (it->host != values.data()) {
+            ++it;
+            continue;
+        }
+        hn_csr_destroy(it->h);
+        it = cache_.erase(it);
+    }
+    while (cache_.size() >= kResidentMax) {
+        hn_csr_destroy(cache_.back().h);
+        cache_.pop_back();
+    }
     Resident r;
+    for (std::size_t c : col_indices) r.used = c + 1 > r.used ? c + 1 : r.used;
+    r.ncols = ncols > r.used ? ncols : r.used;
     static_assert(sizeof(std::size_t) == sizeof(uint64_t), "size_t must be 64-bit");
-    if (hn_csr_create((int64_t)nrows, (int64_t)n, reinterpret_cast<const uint64_t*>(row_ptr.data()),
+    if (hn_csr_create((int64_t)nrows, (int64_t)r.ncols, reinterpret_cast<const uint64_t*>(row_ptr.data()),
                       reinterpret_cast<const uint64_t*>(col_indices.data()), values.data(), 0, &r.h) != HN_OK)
         throw std::runtime_error(std::string("B200 matrix upload failed: ") + hn_last_error());
-    r.nnz = values.size();
+    r.host = values.data();
+    r.nnz = nnz;
     r.nrows = nrows;
-    r.ncols = n;
     r.fingerprint = fp;
-    return cache_.emplace(values.data(), r).first->second;
+    cache_.push_front(r);
+    return cache_.front();
 }
 
 double* B200Backend::staging(std::size_t doubles) {
@@ -144,7 +160,7 @@ void B200Backend::spmv(const std::vector<double>& values, const std::vector<std:
         y.assign(nrows, 0.0);
         return;
     }
-    Resident& r = resident(values, col_indices, row_ptr, x.size());
+    Resident& r = resident(values, col_indices, row_ptr, x.size(), false);
     if (x.size() < r.ncols) throw std::runtime_error("B200 spmv: x shorter than the matrix's column count");
     y.resize(nrows);
     if (hn_spmv_host(r.h, 0, x.data(), y.data()) != HN_OK)
@@ -161,7 +177,7 @@ void B200Backend::spmv_t(const std::vector<double>& values, const std::vector<st
         y.assign(ncols, 0.0);
         return;
     }
-    Resident& r = resident(values, col_indices, row_ptr, ncols);
+    Resident& r = resident(values, col_indices, row_ptr, ncols, true);
     if (x.size() < nrows) throw std::runtime_error("B200 spmv_t: x shorter than the row count");
     std::vector<double> out(r.ncols);
     if (hn_spmv_host(r.h, 1, x.data(), out.data()) != HN_OK)
@@ -180,7 +196,7 @@ void B200Backend::spmm(const std::vector<double>& values, const std::vector<std:
         C.assign(nrows * ncols_B, 0.0);
         return;
     }
-    Resident& r = resident(values, col_indices, row_ptr, B.size() / ncols_B);
+    Resident& r = resident(values, col_indices, row_ptr, B.size() / ncols_B, false);
     if (B.size() < r.ncols * ncols_B) throw std::runtime_error("B200 spmm: B smaller than ncols x k");
     C.resize(nrows * ncols_B);
     if (hn_spmm_host(r.h, 0, B.data(), (int64_t)ncols_B, C.data()) != HN_OK)

@@ -12,10 +12,10 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <list>
 #include <memory>
 #include <mutex>
 #include <string>
-#include <unordered_map>
 #include <vector>
 
 struct hn_csr;
@@ -84,15 +84,20 @@ public:
 private:
     struct Resident {
         hn_csr* h = nullptr;
-        std::size_t nnz = 0, nrows = 0, ncols = 0;
+        const void* host = nullptr;  // the values it was last found by
+        std::size_t nnz = 0, nrows = 0;
+        std::size_t ncols = 0, used = 0;  // columns of the handle, of the entries
         uint64_t fingerprint = 0;
     };
-    // Device copy of a matrix, keyed by the host values pointer like the
-    // reference's cache (gpu_backend.cpp:289-306) but also checked against
-    // sizes and a hash of every entry of the three arrays, so a reused buffer
-    // with new contents is uploaded again instead of returning stale data.
+    // Device copy of a matrix, found by its sizes and a hash of every entry of
+    // the three arrays. (The reference's cache goes by the values' address,
+    // gpu_backend.cpp:289-306; callers of the C interface pass copies, whose
+    // address is the allocator's choice.) A buffer with new contents takes the
+    // place of the matrix that it held, and the kResidentMax matrices used last
+    // are kept. ncols columns are wanted, or more too if `wider`.
+    static constexpr std::size_t kResidentMax = 16;
     Resident& resident(const std::vector<double>& values, const std::vector<std::size_t>& col_indices,
-                       const std::vector<std::size_t>& row_ptr, std::size_t ncols);
+                       const std::vector<std::size_t>& row_ptr, std::size_t ncols, bool wider);
     void require(const char* op) const;
     double* staging(std::size_t doubles);
     void release();
@@ -102,7 +107,7 @@ private:
     bool available_ = false;
     std::string last_error_;
     std::string device_name_;
-    std::unordered_map<const void*, Resident> cache_;
+    std::list<Resident> cache_;  // the last used one first
     double* dev_buf_ = nullptr;
     std::size_t dev_buf_len_ = 0;
     uint64_t launches_at_reset_ = 0;
