@@ -346,10 +346,9 @@ __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __res
     }
     __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        sh.last = atomicAdd(a.ticket, 1u) == (unsigned)(a.ntiles - 1);
-        if (sh.last) *a.ticket = 0u;
-    }
+    // the count wraps to zero by itself: a reset of its own would lose the counts of
+    // a product that overlaps this one (against the rules), and with them every later fix-up
+    if (tid == 0) sh.last = atomicInc(a.ticket, (unsigned)(a.ntiles - 1)) == (unsigned)(a.ntiles - 1);
     __syncthreads();
     if (!sh.last) return;
     __threadfence();
