@@ -858,8 +858,13 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ void named_sync(int id) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(kUpdT) : "memory"); }
+// Whole warps meet here (bar.sync and bar.arrive are .aligned), after branches by lane as well.
+__device__ __forceinline__ void named_sync(int id) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(kUpdT) : "memory");
+}
 __device__ __forceinline__ void named_arrive(int id) {
+    __syncwarp();
     asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(kUpdT) : "memory");
 }
 
@@ -960,7 +965,6 @@ __global__ void __launch_bounds__(kUpdT, 2) batch_ldlt_update_kernel(int k0, int
         const int st = static_cast<int>(n % kUpdStages);
         if (n >= kUpdStages) named_sync(kEmpty + st);
         if (lane == 0) s_tile[st].A = nullptr;
-        __syncwarp();
         named_arrive(kFull + st);
         for (int64_t i = n >= kUpdStages ? n - kUpdStages + 1 : 0; i < n; ++i)
             named_sync(kEmpty + static_cast<int>(i % kUpdStages));
@@ -1182,6 +1186,7 @@ __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
         for (int i = tid; i < m; i += kT) s_x[i] = x[i];
     auto barrier = [&]() {
         if (slot.steps > 0) {
+            __syncwarp();  // .aligned, and rows past the instance's end branch by lane
             asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         } else {
