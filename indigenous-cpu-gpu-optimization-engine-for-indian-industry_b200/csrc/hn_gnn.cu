@@ -772,6 +772,9 @@ void launch_umma(int64_t M, int K1, int K2, const float* X1, const float* X2, co
 
 bool misaligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
 
+// Whether na floats at a and nb floats at b share any.
+bool overlap(const float* a, int64_t na, const float* b, int64_t nb) { return a < b + nb && b < a + na; }
+
 void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, const void* Wb_bf16, const float* Y,
                 const float* dY, int relu, float* G, float* dX, float* dX2, float* dW, float* db, float* scratch,
                 int64_t scratch_floats, cudaStream_t s) {
@@ -789,11 +792,13 @@ void linear_bwd(int64_t M, int K1, int K2, const float* X1, const float* X2, con
     float* pb = scratch + nb * kH * K;
     if (M > 0) {
         // the weight-gradient kernel forms G; dY and Y that no bulk copy can
-        // read, or dY that G overwrites, take a pass of their own
+        // read, or that lie in G or the scratch, which other CTAs are writing
+        // meanwhile, take a pass of their own
+        const int64_t len = M * kH, parts = nb * (int64_t)(kH * K + kH);
+        auto written = [&](const float* p) { return overlap(p, len, G, len) || overlap(p, len, scratch, parts); };
         const float *dy = dY, *y = relu ? Y : nullptr;
         float* gout = G;
-        if (misaligned16(dY) || (relu && misaligned16(Y)) || G == dY || G == Y) {
-            const int64_t len = M * kH;
+        if (misaligned16(dY) || (relu && misaligned16(Y)) || written(dY) || (relu && written(Y))) {
             launch_next(gnn_relu_bwd_kernel, (unsigned)std::min<int64_t>((len + 255) / 256, 148 * 16), 256, 0, s, len,
                         dY, Y, relu, G);
             launched("gnn_relu_bwd_kernel");

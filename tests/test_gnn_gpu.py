@@ -327,3 +327,20 @@ def test_backward_routes_agree(hn, torch_cuda, M, relu):
     d1, d2, G3 = torch.empty(M, 64, device="cuda"), torch.empty(M, 64, device="cuda"), torch.empty_like(G)
     dW3, db3 = _bwd(hn, torch, x1, x2, wb, Y, dY, scratch, relu, None, G3, split=(d1, d2))
     assert all(torch.equal(a, b) for a, b in ((G, G3), (dX[:, :64], d1), (dX[:, 64:], d2), (dW, dW3), (db, db3)))
+
+
+@pytest.mark.parametrize("M", [63, 200, 148 * 64 + 1])
+@pytest.mark.parametrize("which", ["dY", "Y", "both"])
+def test_backward_gradients_in_the_scratch(hn, torch_cuda, M, which):
+    """dY and Y may lie in the scratch: they are read before it is written."""
+    torch = torch_cuda
+    x1, x2, wb, Y, dY, scratch = _bwd_inputs(hn, torch, M, 64, 64, M)
+    G, dX = torch.empty(M, 64, device="cuda"), torch.empty(M, 128, device="cuda")
+    dW, db = _bwd(hn, torch, x1, x2, wb, Y, dY, scratch, 1, dX, G)
+    big = torch.empty(max(scratch.numel(), 2 * M * 64 + 64), device="cuda")
+    at = lambda k, t: big[k:k + M * 64].copy_(t.reshape(-1)).view(M, 64)  # noqa: E731
+    dYs = at(32, dY) if which != "Y" else dY
+    Ys = at(32 + M * 64, Y) if which != "dY" else Y
+    G2, dX2 = torch.empty_like(G), torch.empty_like(dX)
+    dW2, db2 = _bwd(hn, torch, x1, x2, wb, Ys, dYs, big, 1, dX2, G2)
+    assert all(torch.equal(a, b) for a, b in ((G, G2), (dX, dX2), (dW, dW2), (db, db2)))
