@@ -1486,7 +1486,7 @@ void free_batch(hn_batch* B) {
            B->tile_row, B->tile_nz, B->carry_row, B->head_row, B->carry_val, B->head_val, B->r, B->ax, B->step_tiles,
            B->chunks, B->info, B->slots, B->work, B->solve_part, B->kkt, B->kkt_ref, B->ref_iter, B->xb, B->zb,
            B->lb});
-    if (B->left_host) cudaFreeHost(B->left_host);
+    host_word_free(B->left_host);
     delete B;
 }
 
@@ -1554,7 +1554,7 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
             B->refine = dmalloc<int32_t>(K);
             B->nref = dmalloc<int32_t>(2);
             check_cuda(cudaMemsetAsync(B->nref, 0, 2 * sizeof(int32_t), s), "memset");
-            check_cuda(cudaMallocHost(reinterpret_cast<void**>(&B->left_host), sizeof(int32_t)), "cudaMallocHost");
+            B->left_host = host_word();
             B->r = dmalloc<double>(m);
             B->ax = dmalloc<double>(m);
             B->nrp = dmalloc<int32_t>(m + 1);

@@ -119,6 +119,11 @@ void* pool_alloc(size_t bytes);
 cudaError_t pool_free(void* const* ps, size_t n);
 void pool_release();  // gives the cached blocks back
 
+// A word of pinned host memory that kernels may write (hn_core.cu).
+int32_t* host_word();
+void host_word_free(int32_t* w);
+void host_words_release();
+
 template <class T>
 T* dmalloc(size_t count) {
     if (count == 0) count = 1;

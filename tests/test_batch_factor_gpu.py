@@ -94,3 +94,55 @@ def test_many_panel_rows(hn, torch_cuda, scale):
     r = solve_batch(hn, torch_cuda, ms, scale)
     for i in [0, 1, 2, 3, 4, 61, 117, 118, 119]:
         check(i, *r, scale)
+
+
+def test_many_handles_at_once(hn, torch_cuda):
+    """More handles than one slab of their host words has room for, solved in
+    turn; their words are used again."""
+    import threading
+
+    lib, p64, n = hn.load(), C.POINTER(C.c_int64), 1100
+    A = hn.Csr(3, 3, [0, 1, 2, 4], [0, 1, 1, 2], [2.0, 1.0, 1.0, 1.0])
+    P = hn.Pattern(A)
+    ro = np.array([0, 3], np.int64)
+    dev = lambda a: torch_cuda.as_tensor(np.asarray(a), device="cuda")  # noqa: E731
+    D, rhs, st = dev(np.ones(3)), dev([1.0, -2.0, 3.0]), dev(np.zeros(1, np.int32))
+    N = np.array([[4.0, 0, 0], [0, 1, 1], [0, 1, 2]])
+    N[np.diag_indices(3)] += 4e-12
+    want = np.linalg.solve(N, [1.0, -2.0, 3.0])
+
+    def create():
+        h = C.c_void_p()
+        hn.check(lib.hn_batch_create(1, ro.ctypes.data_as(p64), ro.ctypes.data_as(p64), P.h, C.byref(h)))
+        return h
+
+    def solve(h):
+        nval, x = torch_cuda.empty(P.nnz, dtype=torch_cuda.float64, device="cuda"), torch_cuda.empty_like(rhs)
+        hn.check(lib.hn_batch_factor(h, D.data_ptr(), 0.0, 1e-300, nval.data_ptr(), st.data_ptr(), None))
+        hn.check(lib.hn_batch_solve(h, nval.data_ptr(), rhs.data_ptr(), x.data_ptr(), st.data_ptr(), None))
+        torch_cuda.cuda.synchronize()
+        assert np.allclose(x.cpu().numpy(), want, rtol=1e-12, atol=0)
+
+    hs = [create() for _ in range(n)]
+    for h in hs[::97] + hs[-1:]:
+        solve(h)
+    for h in hs[: n // 2]:
+        hn.check(lib.hn_batch_destroy(h))
+    hs = [create() for _ in range(n // 2)] + hs[n // 2:]
+    errors = []
+
+    def work(part):
+        try:
+            for h in part:
+                hn.check(lib.hn_batch_destroy(h))
+        except Exception as e:  # noqa: BLE001 (reported by the main thread)
+            errors.append(e)
+
+    solve(hs[0])
+    ts = [threading.Thread(target=work, args=(hs[t::4],)) for t in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not errors, errors
+    h = create()
+    solve(h)
+    hn.check(lib.hn_batch_destroy(h))
