@@ -191,15 +191,33 @@ __global__ void __launch_bounds__(kSpmvThreads) spmv_tile_kernel(SpmvMat a, cons
     }
 }
 
-// Finishes the row that began before `tile` and ends in it, if there is one.
+// Finishes the row that began before `tile` and ends in it, if there is one:
+// the carries of the tiles before it that hold nothing but that row, in order.
+// kFixBatch loads at a time, past L1 (in one launch other SMs wrote them): one
+// after the other a row over 1,675 tiles took 411 us, with L1 217.
+constexpr int kFixBatch = 16;
 template <class Epi>
 __device__ __forceinline__ void fix_up(const SpmvMat& a, int64_t tile, const Epi& epi) {
     const int r = __ldcg(a.head_row + tile);
     if (r < 0) return;
-    int64_t s = tile - 1;
-    while (s >= 0 && __ldcg(a.carry_row + s) == r) --s;
+    int64_t first = tile;
+    for (int n = kFixBatch; n == kFixBatch; first -= n) {
+        int row[kFixBatch];
+#pragma unroll
+        for (int u = 0; u < kFixBatch; ++u) row[u] = first - 1 - u >= 0 ? __ldcg(a.carry_row + first - 1 - u) : -1;
+        n = 0;
+#pragma unroll
+        for (int u = 0; u < kFixBatch; ++u) n += n == u && row[u] == r;
+    }
     double acc = 0.0;
-    for (int64_t u = s + 1; u < tile; ++u) acc += __ldcg(a.carry_val + u);
+    for (int64_t t = first; t < tile; t += kFixBatch) {
+        double v[kFixBatch];
+#pragma unroll
+        for (int u = 0; u < kFixBatch; ++u) v[u] = t + u < tile ? __ldcg(a.carry_val + t + u) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kFixBatch; ++u)
+            if (t + u < tile) acc += v[u];
+    }
     acc += __ldcg(a.head_val + tile);
     epi(r, acc);
 }
