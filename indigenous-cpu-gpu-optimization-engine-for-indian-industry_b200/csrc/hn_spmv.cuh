@@ -243,7 +243,14 @@ __global__ void spmv_fixup_kernel(SpmvMat a, Epi epi) {
 // y = A x - b and A^T lam of 200 x 500: 10.0 us of kernels in two launches, 17.5
 // in four (24.6 -> 12.3 us a pair of calls, 9.5 with launches prepared ahead);
 // the one iteration's products of 2,000 x 5,000: 6 us each instead of 9.5.
-constexpr int64_t kSpmvSmallTiles = 2048;
+// Where it stops paying, us in one launch and in two. Short heads, rows of 8 and
+// of 40 entries: 600 tiles 9.9 and 13.8, 12.2 and 16.0; 1,184 tiles 16.0 and
+// 17.0, 18.5 and 18.8; 2,000 tiles 23.5 and 24.9, 26.7 and 26.5; 3,000 tiles
+// 33.4 and 32.9, 37.1 and 35.3. With the ticket, where one CTA walks all heads,
+// rows of 2,000 and of 100,000 entries: 296 tiles 19.6 and 18.7, 18.0 and 18.9;
+// 444 tiles 19.9 and 20.0, 18.2 and 20.3; 600 tiles 23.2 and 22.8, 22.7 and
+// 21.7; 1,000 tiles 32.8 and 25.4, 37.3 and 25.5.
+constexpr int64_t kSpmvSmallTiles = 2048, kSpmvTicketTiles = 444;
 struct SmallTile {
     double prod[kSpmvTile];
     int32_t rowend[kSpmvTile + 1];
@@ -254,7 +261,9 @@ struct SmallTile {
     bool last;
 };
 
-template <class Epi>
+// kTicket: the fix-ups are the last tile's. A form of its own, or the other one
+// has its registers too (64 instead of 40 or 48: 11.8 us instead of 9.9 at 600 tiles).
+template <bool kTicket, class Epi>
 __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __restrict__ x, const Epi& epi, int tile,
                                            SmallTile& sh) {
     const int tid = threadIdx.x;
@@ -281,8 +290,7 @@ __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __res
         }
     }
     const int rowstart0 = r0 < a.m ? __ldg(a.rp + r0) : a.nnz;
-    const bool alone = a.ntiles == 1 || a.short_heads;
-    if (!alone) {
+    if constexpr (kTicket) {
         if (tid == 0) a.head_row[tile] = -1;
     } else if (tid >= kSpmvThreads - 32 && k0 > rowstart0 && nrows_t > 0) {
         // the last warp: the carry of the row that ends here and began in the tile before
@@ -341,14 +349,14 @@ __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __res
         for (int u = t + 1; u < tid; ++u) acc += sh.cval[u];
         acc += first_val;
         const bool head = t < 0 && first_row == 0 && k0 > rowstart0;
-        if (head && !alone) {
+        if (kTicket && head) {
             a.head_row[tile] = r0;
             a.head_val[tile] = acc;
         } else {
             epi(r0 + first_row, head ? (0.0 + sh.carry) + acc : acc);
         }
     }
-    if (alone) return;
+    if constexpr (!kTicket) return;
     if (tid == kSpmvThreads - 1) {
         const int crow = sh.crow[tid];
         if (r0 + crow < a.m) {
@@ -373,26 +381,29 @@ __device__ __forceinline__ void small_tile(const SpmvMat& a, const double* __res
     for (int64_t t = tid; t < a.ntiles; t += kSpmvThreads) fix_up(a, t, epi);
 }
 
-template <class Epi>
+template <bool kTicket, class Epi>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_small_kernel(SpmvMat a, const double* __restrict__ x, Epi epi) {
     if (!after_previous()) return;
     __shared__ SmallTile sh;
-    small_tile(a, x, epi, blockIdx.x, sh);
+    small_tile<kTicket>(a, x, epi, blockIdx.x, sh);
 }
 
-template <class Epi, class Epi2>
+template <bool kTicket, bool kTicket2, class Epi, class Epi2>
 __global__ void __launch_bounds__(kSpmvThreads) spmv_small2_kernel(SpmvMat a, const double* __restrict__ x, Epi epi,
                                                                    SpmvMat b, const double* __restrict__ x2,
                                                                    Epi2 epi2) {
     if (!after_previous()) return;
     __shared__ SmallTile sh;
     if (blockIdx.x < (unsigned)a.ntiles)
-        small_tile(a, x, epi, blockIdx.x, sh);
+        small_tile<kTicket>(a, x, epi, blockIdx.x, sh);
     else
-        small_tile(b, x2, epi2, blockIdx.x - (int)a.ntiles, sh);
+        small_tile<kTicket2>(b, x2, epi2, blockIdx.x - (int)a.ntiles, sh);
 }
 
-inline bool spmv_small(const SpmvMat& M) { return M.kind == 0 && M.ticket && M.ntiles <= kSpmvSmallTiles; }
+inline bool spmv_ticket(const SpmvMat& M) { return M.ntiles > 1 && !M.short_heads; }
+inline bool spmv_small(const SpmvMat& M) {
+    return M.kind == 0 && M.ticket && M.ntiles <= (spmv_ticket(M) ? kSpmvTicketTiles : kSpmvSmallTiles);
+}
 
 // ---- binned vector CSR ----
 // A group of G lanes sums one row: lane l takes the row's nonzeros l, l + G,
@@ -464,7 +475,8 @@ void spmv_launch(const SpmvMat& M, const double* x, const Epi& epi, cudaStream_t
     }
     if (M.ntiles == 0) return;
     if (spmv_small(M)) {
-        launch_next(spmv_small_kernel<Epi>, (unsigned)M.ntiles, kSpmvThreads, 0, s, M, x, epi);
+        launch_next(spmv_ticket(M) ? spmv_small_kernel<true, Epi> : spmv_small_kernel<false, Epi>, (unsigned)M.ntiles,
+                    kSpmvThreads, 0, s, M, x, epi);
         launched("spmv_small_kernel");
         return;
     }
@@ -481,8 +493,11 @@ template <class Epi, class Epi2>
 void spmv_launch2(const SpmvMat& M, const double* x, const Epi& epi, const SpmvMat& M2, const double* x2,
                   const Epi2& epi2, cudaStream_t s) {
     if (spmv_small(M) && spmv_small(M2) && M.ntiles > 0 && M2.ntiles > 0) {
-        launch_next(spmv_small2_kernel<Epi, Epi2>, (unsigned)(M.ntiles + M2.ntiles), kSpmvThreads, 0, s, M, x, epi,
-                    M2, x2, epi2);
+        auto* kernel = spmv_ticket(M) ? (spmv_ticket(M2) ? spmv_small2_kernel<true, true, Epi, Epi2>
+                                                         : spmv_small2_kernel<true, false, Epi, Epi2>)
+                                      : (spmv_ticket(M2) ? spmv_small2_kernel<false, true, Epi, Epi2>
+                                                         : spmv_small2_kernel<false, false, Epi, Epi2>);
+        launch_next(kernel, (unsigned)(M.ntiles + M2.ntiles), kSpmvThreads, 0, s, M, x, epi, M2, x2, epi2);
         launched("spmv_small2_kernel");
         return;
     }

@@ -41,3 +41,31 @@ def test_products_after_overlapping_ones(hn, torch_cuda):
     for _ in range(3):
         A.spmv(x, y)
         assert torch.equal(y, want)
+
+
+TILE = 1792  # row ends and entries of a merge-path tile
+
+
+def tiles_of(n, kind):
+    """Row lengths of exactly n tiles: rows of 15 entries (no head over 15), or of 3,583 (heads of 1,791)."""
+    if kind == "short":
+        return np.full(n * TILE // 16, 15)
+    return np.full(n * TILE // 3584, 3583)
+
+
+@pytest.mark.parametrize("n", [2, 4, 444, 446, 2046, 2048, 2050])
+@pytest.mark.parametrize("kind", ["short", "long"])
+def test_lines_between_one_launch_and_two(hn, torch_cuda, n, kind):
+    """Up to 444 tiles (long heads) or 2,048 (short ones) one launch, the same bits on both sides of the lines."""
+    torch, rng = torch_cuda, np.random.default_rng(n)
+    rows, cols = tiles_of(n, kind), 5000
+    rp, ci, val = matrix(rows, cols, rng)
+    x = torch.as_tensor(rng.standard_normal(cols), device="cuda")
+    A = hn.Csr(rows.size, cols, rp, ci, val, transpose=False, autotune=False)
+    assert A.tiles()[1].size == n + 1
+    want = two_launches(hn, torch, rows.size, cols, rp, ci, val, x)
+    for _ in range(2):
+        y, before = torch.full_like(want, np.nan), hn.stats()[0]
+        A.spmv(x, y)
+        assert hn.stats()[0] - before == (1 if n <= (2048 if kind == "short" else 444) else 2)
+        assert torch.equal(y, want)
