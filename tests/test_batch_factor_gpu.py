@@ -146,3 +146,25 @@ def test_many_handles_at_once(hn, torch_cuda):
     h = create()
     solve(h)
     hn.check(lib.hn_batch_destroy(h))
+
+
+@pytest.mark.parametrize("m", [2112, 2113, 2369, 4200])
+def test_several_chunks_per_cta(hn, torch_cuda, m):
+    """One instance on a group of eight CTAs with one chunk of rows each or several, the same bits every time."""
+    r = solve_batch(hn, torch_cuda, [m])
+    check(0, *r, 1.0)
+    for _ in range(3):
+        assert np.array_equal(solve_batch(hn, torch_cuda, [m])[5], r[5])
+
+
+def test_groups_of_two_and_four(hn, torch_cuda):
+    """Enough instances for up to two chunks of rows per CTA: groups of one, two
+    and four CTAs share clusters, some with masked members."""
+    ms = [1100, 1500, 600, 900, 330, 1090, 580] * 30
+    masked = [3, 4, 20, 21, 55, 209]
+    r = solve_batch(hn, torch_cuda, ms, masked=masked)
+    for i in masked:
+        assert np.array_equal(r[5][r[1][i]:r[1][i + 1]], r[4][r[1][i]:r[1][i + 1]])
+    for i in [0, 1, 2, 5, 6, 57, 58, 60, 62, 207, 208]:
+        check(i, *r, 1.0)
+    assert np.array_equal(solve_batch(hn, torch_cuda, ms, masked=masked)[5], r[5])
