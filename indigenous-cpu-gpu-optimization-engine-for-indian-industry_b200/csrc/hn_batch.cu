@@ -82,7 +82,7 @@ struct hn_batch {
     // even step, the whole trailing triangle after an odd one) as cumulative
     // counts per (step, instance), and the kT-row chunks below their diagonal
     // blocks as a list per step, spread every instance's work over the GPU.
-    int64_t nsteps = 0;
+    int64_t mmax = 0, nsteps = 0;  // rows and blocks of the largest instance
     std::vector<int32_t> step_cnt;                       // host, nsteps
     std::vector<int64_t> tile_off_h, chunk_off_h;        // host, nsteps+1 offsets into the two tables
     std::vector<int64_t> step_tiles_h;                   // host, tiles per step
@@ -438,7 +438,6 @@ __device__ __forceinline__ void dmma_m8n8k4(double* d, double a, double b) {
                  : "+d"(d[0]), "+d"(d[1])
                  : "d"(a), "d"(b));
 }
-constexpr int kFbP = kFb + 1;  // padded smem row (conflict-free column walks)
 
 // Quotients by a common divisor, correctly rounded as a / d is, from its
 // correctly rounded reciprocal y: two residual corrections q + (a - d q) y
@@ -508,15 +507,22 @@ __global__ void quotients_kernel(int64_t n, const double* __restrict__ a, const 
 // the diagonal or past the block is never read.
 // 384 LPs of m 50-2000 (31 blocks): 585 us, 1,558 with the block in shared
 // memory and two barriers per pivot; one wave of blocks 15 us (41 before).
+// R: the rows that a CTA has threads for, 16, 32, 48 or 64, so that the step's
+// largest block fits: many small instances are bound by how many CTAs an SM
+// holds. The factorisation of 16,000 instances of 10 rows takes 288 us, of 32
+// rows 914, of 48 rows 1,838 (with 64 rows in every case 668, 1,315 and 1,898;
+// 448, 1,441 and 2,395 with the block in shared memory).
+template <int R>
 struct DiagShared {
-    double A[kFb][kFbP];
-    double lc[2][4][kFb];  // the round's four columns of L, by the parity of the round
-    double pb[4][4];       // the next pivot block (its lower triangle)
-    double d[kFb];
+    double A[R][R + 1];
+    double lc[2][4][R];  // the round's four columns of L, by the parity of the round
+    double pb[4][4];     // the next pivot block (its lower triangle)
+    double d[R];
 };
 
 // a[4] -= a round's four columns: row factors w[q] = l_rq d_q, columns c .. c + 3
-__device__ __forceinline__ void diag_update(double* a, const double* w, const double (*lc)[kFb], int c) {
+template <int R>
+__device__ __forceinline__ void diag_update(double* a, const double* w, const double (*lc)[R], int c) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -566,21 +572,22 @@ __device__ __noinline__ void diag_pivots_plain(const double (*pb)[4], double tol
 // columns right of the previous round's successor still lack that round (row
 // factors w, columns of L of the parity before): each round's owners take it
 // after their pivots, the others before the round's first barrier.
-template <int I>
-__device__ __forceinline__ void diag_rounds(DiagShared& sh, double (*a)[4], double* w, int nb, double tol, int r,
+template <int I, int R>
+__device__ __forceinline__ void diag_rounds(DiagShared<R>& sh, double (*a)[4], double* w, int nb, double tol, int r,
                                             int g) {
+    constexpr int kNext = 16 * (I + 1) < R ? I + 1 : I;  // the quads after these rounds' (or none)
 #pragma unroll 1
     for (int og = 0; og < 4; ++og) {
         const int j0 = 16 * I + 4 * og;
         if (j0 >= nb) return;
-        double(*lc)[kFb] = sh.lc[og & 1];
+        double(*lc)[R] = sh.lc[og & 1];
         // the previous round's update right of this round's quad
         auto rest = [&]() {
             if (I == 0 && og == 0) return;
-            const double(*lp)[kFb] = sh.lc[(og & 1) ^ 1];
+            const double(*lp)[R] = sh.lc[(og & 1) ^ 1];
             if (g > og) diag_update(a[I], w, lp, 16 * I + 4 * g);
 #pragma unroll
-            for (int i = I + 1; i < 4; ++i) diag_update(a[i], w, lp, 16 * i + 4 * g);
+            for (int i = I + 1; i < R / 16; ++i) diag_update(a[i], w, lp, 16 * i + 4 * g);
         };
         if (g == og) {
             double d[4], t[4];
@@ -604,61 +611,62 @@ __device__ __forceinline__ void diag_rounds(DiagShared& sh, double (*a)[4], doub
         if (g == og) rest();
 #pragma unroll
         for (int q = 0; q < 4; ++q) w[q] = lc[q][r] * sh.d[j0 + q];
-        if (g == ((og + 1) & 3) && j0 + 4 < kFb) {  // the next round's owners
+        if (g == ((og + 1) & 3) && j0 + 4 < R) {  // the next round's owners
             if (og < 3)
                 diag_update(a[I], w, lc, j0 + 4);
             else
-                diag_update(a[I < 3 ? I + 1 : 3], w, lc, j0 + 4);
+                diag_update(a[kNext], w, lc, j0 + 4);
             if (r >= j0 + 4 && r < j0 + 8) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) sh.pb[r - j0 - 4][e] = og < 3 ? a[I][e] : a[I < 3 ? I + 1 : 3][e];
+                for (int e = 0; e < 4; ++e) sh.pb[r - j0 - 4][e] = og < 3 ? a[I][e] : a[kNext][e];
             }
         }
         __syncthreads();
     }
 }
 
-__global__ void __launch_bounds__(kT) batch_ldlt_diag_kernel(int s, const InstInfo* __restrict__ info,
-                                                             const int32_t* __restrict__ order,
-                                                             const int32_t* __restrict__ status,
-                                                             double* __restrict__ dense, double* __restrict__ dD,
-                                                             double tol) {
+template <int R>
+__global__ void __launch_bounds__(4 * R) batch_ldlt_diag_kernel(int s, const InstInfo* __restrict__ info,
+                                                                const int32_t* __restrict__ order,
+                                                                const int32_t* __restrict__ status,
+                                                                double* __restrict__ dense, double* __restrict__ dD,
+                                                                double tol) {
     const int inst = order[blockIdx.x];
     const InstInfo in = info[inst];
     if (!after_previous()) return;
-    __shared__ DiagShared sh;
+    __shared__ DiagShared<R> sh;
     const int tid = threadIdx.x;
     if (status[inst] != ST_RUN) return;
     const int ld = dense_ld(in.m);
     const int k0 = s * kFb;
-    const int nb = min(kFb, in.m - k0);
+    const int nb = min(R, in.m - k0);
     double* A = dense + in.dn + (int64_t)k0 * ld + k0;
-    const int col = tid & (kFb - 1), row = tid >> 6;
-    double v[kFb / 4];
+    const int col = tid % R, row = tid / R;
+    double v[R / 4];
 #pragma unroll
-    for (int i = 0; i < kFb / 4; ++i) {
+    for (int i = 0; i < R / 4; ++i) {
         const int rr = 4 * i + row;
         v[i] = (rr < nb && col <= rr) ? A[(int64_t)rr * ld + col] : 0.0;
     }
 #pragma unroll
-    for (int i = 0; i < kFb / 4; ++i) sh.A[4 * i + row][col] = v[i];
+    for (int i = 0; i < R / 4; ++i) sh.A[4 * i + row][col] = v[i];
     __syncthreads();
-    const int r = tid & (kFb - 1), g = tid >> 6;
-    double a[4][4];
+    const int r = tid % R, g = tid / R;
+    double a[R / 16][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < R / 16; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) a[i][e] = sh.A[r][16 * i + 4 * g + e];
     if (tid < 16) sh.pb[tid >> 2][tid & 3] = sh.A[tid >> 2][tid & 3];
     __syncthreads();  // the columns of L overwrite sh.A
     double w[4];
     diag_rounds<0>(sh, a, w, nb, tol, r, g);
-    diag_rounds<1>(sh, a, w, nb, tol, r, g);
-    diag_rounds<2>(sh, a, w, nb, tol, r, g);
-    diag_rounds<3>(sh, a, w, nb, tol, r, g);
+    if constexpr (R > 16) diag_rounds<1>(sh, a, w, nb, tol, r, g);
+    if constexpr (R > 32) diag_rounds<2>(sh, a, w, nb, tol, r, g);
+    if constexpr (R > 48) diag_rounds<3>(sh, a, w, nb, tol, r, g);
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kFb / 4; ++i) {
+    for (int i = 0; i < R / 4; ++i) {
         const int rr = 4 * i + row;
         if (rr < nb && col < rr) A[(int64_t)rr * ld + col] = sh.A[rr][col];
     }
@@ -1584,8 +1592,8 @@ int hn_batch_create(int64_t K, const int64_t* row_off_host, const int64_t* col_o
                             &B->head_row, &B->head_val, &B->short_heads, s);
             // level schedule (instances in decreasing size: the ones with a block
             // at step s form a prefix of `order`)
-            const int64_t mmax = row_off_host[order[0] + 1] - row_off_host[order[0]];
-            B->nsteps = (mmax + kFb - 1) / kFb;
+            B->mmax = row_off_host[order[0] + 1] - row_off_host[order[0]];
+            B->nsteps = (B->mmax + kFb - 1) / kFb;
             B->tile_off_h.assign(1, 0);
             B->chunk_off_h.assign(1, 0);
             std::vector<int64_t> tiles;
@@ -1754,8 +1762,13 @@ int hn_batch_factor(hn_batch* B, const double* D, double reg, double singular_to
         // brought up to date, after an odd one the rest, by both panels at once
         for (int64_t st = 0; st < B->nsteps; ++st) {
             const int cnt = B->step_cnt[st];
-            launch_next(batch_ldlt_diag_kernel, cnt, kT, 0, s, (int)st, B->info, B->order, status, B->dense, B->dD,
-                        singular_tol);
+            const int64_t nb = B->mmax - st * kFb;  // the largest block's rows
+            auto* diag = nb <= 16   ? batch_ldlt_diag_kernel<16>
+                         : nb <= 32 ? batch_ldlt_diag_kernel<32>
+                         : nb <= 48 ? batch_ldlt_diag_kernel<48>
+                                    : batch_ldlt_diag_kernel<64>;
+            launch_next(diag, cnt, (unsigned)std::min<int64_t>((nb + 15) / 16 * 64, 4 * kFb), 0, s, (int)st, B->info, B->order, status,
+                        B->dense, B->dD, singular_tol);
             launched("batch_ldlt_diag_kernel");
             const int64_t nc = B->chunk_off_h[st + 1] - B->chunk_off_h[st];
             if (nc == 0) continue;

@@ -168,3 +168,13 @@ def test_groups_of_two_and_four(hn, torch_cuda):
     for i in [0, 1, 2, 5, 6, 57, 58, 60, 62, 207, 208]:
         check(i, *r, 1.0)
     assert np.array_equal(solve_batch(hn, torch_cuda, ms, masked=masked)[5], r[5])
+
+
+@pytest.mark.parametrize("m", [1, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64])
+@pytest.mark.parametrize("scale", [1.0, 1e-140])
+def test_largest_block(hn, torch_cuda, m, scale):
+    """The diagonal blocks' kernel has as many rows as the step's largest block, 16 at a time."""
+    for ms in ([m, 1, max(1, m - 1), m, 2], [64 + m, 64, 3]):
+        r = solve_batch(hn, torch_cuda, ms, scale)
+        for i in range(len(ms)):
+            check(i, *r, scale)
