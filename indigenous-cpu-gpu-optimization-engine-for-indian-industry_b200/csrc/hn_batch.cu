@@ -1166,6 +1166,63 @@ __device__ __forceinline__ void backward_block(const double (*sL)[kSolveP], doub
     }
 }
 
+// The same for batches whose instances have one block each: a warp per
+// instance, R the largest one's rows (16, 32 or 64). Few are bound by the
+// launch and the chain, many by how many an SM holds: a CTA of the kernel below
+// takes a quarter of the SM and a full block's steps for them. hn_batch_solve of
+// 16,000 instances of 10 rows takes 97 us, of 32 rows 181, of 64 rows 420 (506,
+// 605 and 687 below; 248, 458 and 733 with a launch per direction); of one
+// instance of 10 rows 22, of 64 rows 28 (28 and 28.5 below).
+template <int R>
+__global__ void __launch_bounds__(32) batch_solve_block_kernel(const InstInfo* __restrict__ info,
+                                                               const int32_t* __restrict__ status,
+                                                               const int32_t* __restrict__ refine,
+                                                               const double* __restrict__ dense,
+                                                               const double* __restrict__ dD, double* xv) {
+    const InstInfo in = info[blockIdx.x];
+    if (!after_previous()) return;
+    if (!solving(status, refine, blockIdx.x)) return;
+    __shared__ double sL[R][R + 1];
+    const int lane = threadIdx.x, m = in.m, ld = dense_ld(m);
+    const double* L = dense + in.dn;
+    double* x = xv + in.r0;
+    constexpr int kBatch = R < 32 ? R * R / 32 : 16;  // loads in flight
+#pragma unroll 1
+    for (int q0 = 0; q0 < R * R / 32 && q0 * 32 < m * R; q0 += kBatch) {
+        double t[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+            const int r = (32 * (q0 + q) + lane) / R, c = lane % R + (R > 32 ? 32 * ((q0 + q) % (R / 32)) : 0);
+            t[q] = r < m && c < r ? L[(int64_t)r * ld + c] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q) {
+            const int r = (32 * (q0 + q) + lane) / R, c = lane % R + (R > 32 ? 32 * ((q0 + q) % (R / 32)) : 0);
+            sL[r][c] = t[q];
+        }
+    }
+    const bool on0 = lane < m, on1 = R > 32 && lane + 32 < m;
+    double v0 = on0 ? x[lane] : 0.0, v1 = on1 ? x[lane + 32] : 0.0;
+    const double d0 = on0 ? dD[in.r0 + lane] : 1.0, d1 = on1 ? dD[in.r0 + lane + 32] : 1.0;
+    __syncwarp();
+#pragma unroll 4
+    for (int j = 0; j < m; ++j) {
+        const double y = __shfl_sync(0xffffffffu, R > 32 && j >= 32 ? v1 : v0, j & 31);
+        if (on0 && lane > j) v0 -= sL[lane][j] * y;
+        if (on1 && lane + 32 > j) v1 -= sL[lane + 32][j] * y;
+    }
+    v0 /= d0;
+    v1 /= d1;
+#pragma unroll 4
+    for (int j = m - 1; j >= 0; --j) {
+        const double y = __shfl_sync(0xffffffffu, R > 32 && j >= 32 ? v1 : v0, j & 31);
+        if (lane < j) v0 -= sL[j][lane] * y;
+        if (R > 32 && lane + 32 < j) v1 -= sL[j][lane + 32] * y;
+    }
+    if (on0) x[lane] = v0;
+    if (on1) x[lane + 32] = v1;
+}
+
 __global__ void __cluster_dims__(kSolveCluster, 1, 1) __launch_bounds__(kT, 2)
     batch_solve_kernel(const SolveSlot* __restrict__ slots, const InstInfo* __restrict__ info,
                        const int32_t* __restrict__ status, const int32_t* __restrict__ refine,
@@ -1513,6 +1570,14 @@ SpmvMat n_mat(const hn_batch* B, const double* nval) {
 
 // x holds the right-hand sides of the taking-part instances on entry, their solutions on return.
 void solve_all(hn_batch* B, const int32_t* status, const int32_t* refine, double* x, cudaStream_t s) {
+    if (B->mmax <= kFb) {
+        auto* kernel = B->mmax <= 16   ? batch_solve_block_kernel<16>
+                       : B->mmax <= 32 ? batch_solve_block_kernel<32>
+                                       : batch_solve_block_kernel<64>;
+        launch_next(kernel, (unsigned)B->K, 32, 0, s, B->info, status, refine, B->dense, B->dD, x);
+        launched("batch_solve_block_kernel");
+        return;
+    }
     launch_next(batch_solve_kernel, (unsigned)B->nslots, kT, (size_t)B->solve_smem, s, B->slots, B->info, status,
                 refine, B->dense, B->dD, B->work, B->solve_part, x);
     launched("batch_solve_kernel");

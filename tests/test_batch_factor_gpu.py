@@ -178,3 +178,17 @@ def test_largest_block(hn, torch_cuda, m, scale):
         r = solve_batch(hn, torch_cuda, ms, scale)
         for i in range(len(ms)):
             check(i, *r, scale)
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65])
+def test_instances_of_one_block(hn, torch_cuda, m):
+    """A warp per instance up to 64 rows, beside the form for more (one of 65 rows
+    in the batch); masked ones keep their right-hand sides."""
+    ms, masked = [m, 1, max(1, m - 1), 2, m, max(1, m - 3)], [1, 4]
+    for extra in ([], [65]):
+        r = solve_batch(hn, torch_cuda, ms + extra, masked=masked)
+        for i in range(len(ms)):
+            if i in masked:
+                assert np.array_equal(r[5][r[1][i]:r[1][i + 1]], r[4][r[1][i]:r[1][i + 1]])
+            else:
+                check(i, *r, 1.0)
