@@ -462,8 +462,8 @@ def batched_ipm(K: int, sample_per_stratum: int = 4, rank: int = 0, world: int =
     st = r["status"]
     kkt = r["kkt"][:, 0]
     at_kkt = (st == 1) & (kkt <= 1e-8)
-    # dense LDL^T work: one factorisation of m_i^3 / 3 multiply-adds per iteration of each instance
-    factor_flops = float(np.sum(r["iterations"].astype(np.float64) * sizes.astype(np.float64) ** 3 * 2.0 / 3.0))
+    # dense LDL^T work: one factorisation of m_i^3 / 6 multiply-adds per iteration of each instance
+    factor_flops = float(np.sum(r["iterations"].astype(np.float64) * sizes.astype(np.float64) ** 3 / 3.0))
     # stratified plain sample
     edges = np.exp(np.linspace(np.log(50), np.log(2000) + 1e-9, 9))
     rng = np.random.default_rng(7)

@@ -37,17 +37,15 @@ void launched(const char* what);
 // before it in the stream still runs, its blocks start when that one's last
 // block has ended, and wait there until all its writes are visible (a kernel
 // that finds its work in a plan which was complete before any launch using it
-// reads that first). No kernel
-// lets its successor start earlier (griddepcontrol.launch_dependents): read-only
-// loads (ld.global.nc, what const __restrict__ arguments become) may only touch
-// memory that nobody writes while their kernel is resident, and lines that a
-// running kernel has brought into L1 since would be stale to them. It is no
-// gain either: 48 LPs of m 50-300 366 us an iteration with it, 353 without, 384
-// of m 50-2000 7,603 and 7,397. Without programmatic launches a chain of short
-// kernels spends 1-3 us between each two: products of a 200 x 500 matrix and
-// its transpose 12.3 -> 9.5 us, the 16 kernels of an interior-point iteration
-// at m = 2,000 88 -> 62 us, the two kernels of a product with 5,000,000 entries
-// 35 -> 33 us.
+// reads that first). No kernel lets its successor start earlier
+// (griddepcontrol.launch_dependents): read-only loads (ld.global.nc, what const
+// __restrict__ arguments become) may only touch memory that nobody writes while
+// their kernel is resident, which then is not so. It is no gain either: 48 LPs
+// of m 50-300 366 us an iteration with it, 353 without, 384 of m 50-2000 7,603
+// and 7,397. Without programmatic launches a chain of short kernels spends 1-3
+// us between each two: products of a 200 x 500 matrix and its transpose 12.3 ->
+// 9.5 us, the 14 kernels of an interior-point iteration at m = 2,000 88 -> 62
+// us, the two kernels of a product with 5,000,000 entries 35 -> 33 us.
 template <class... P, class... A>
 void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchAttribute at{};

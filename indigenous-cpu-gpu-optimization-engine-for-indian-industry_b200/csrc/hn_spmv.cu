@@ -47,8 +47,10 @@ __global__ void __launch_bounds__(256) spmm_wide_kernel(int m, const int32_t* __
 // the indices and values of U nonzeros loaded together before their entries of
 // B; with a warp per row, 20,000 x 50,000 with 8 per column took 22.7 us at any
 // k up to 32, now 8.3 (k = 1, 3), 10.3 (8), 12.4 (16), 16.5 (32) and 22.6 (64;
-// 26.8). At k = 100 this form takes 39 us, the wide one 33. Fewer lanes than
-// columns (CC = 2 from 17 on) read B in fewer, longer lines; more nonzeros in
+// 26.8). The line, this form and the wide one: 20,000 x 50,000 with 20 per row
+// 17.2 us and 19.3 at k = 64, 29.8 and 21.4 at 65 (another pass over the row),
+// 34.0 and 30.6 at 128; 50,000 x 50,000 with 40 per row 75 and 84, 134 and 94,
+// 149 and 131. Fewer lanes than columns (CC = 2 from 17 on) read B in fewer, longer lines; more nonzeros in
 // flight than U only cost registers.
 template <int G, int CC, int U>
 __global__ void __launch_bounds__(256) spmm_kernel(int m, const int32_t* __restrict__ rp,

@@ -344,3 +344,13 @@ def test_backward_gradients_in_the_scratch(hn, torch_cuda, M, which):
     G2, dX2 = torch.empty_like(G), torch.empty_like(dX)
     dW2, db2 = _bwd(hn, torch, x1, x2, wb, Ys, dYs, big, 1, dX2, G2)
     assert all(torch.equal(a, b) for a, b in ((G, G2), (dX, dX2), (dW, dW2), (db, db2)))
+
+
+@pytest.mark.parametrize("M", [0, 1, 3, 257])
+def test_split_grad(hn, torch_cuda, M):
+    """dH += dX[:, :64]; dAgg = dX[:, 64:]."""
+    torch = torch_cuda
+    dX, dH = torch.randn(M, 128, device="cuda"), torch.randn(M, 64, device="cuda")
+    want, dAgg = dH + dX[:, :64], torch.full((M, 64), 7.0, device="cuda")
+    hn.check(hn.load().hn_gnn_split_grad(M, dX.data_ptr(), dH.data_ptr(), dAgg.data_ptr(), None))
+    assert torch.equal(dH, want) and torch.equal(dAgg, dX[:, 64:])
