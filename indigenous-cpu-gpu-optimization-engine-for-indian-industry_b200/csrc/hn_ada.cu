@@ -796,11 +796,13 @@ int hn_ada_symbolic_ex(const hn_csr* A, unsigned flags, hn_pattern** out) {
                 check_cuda(cudaMemsetAsync(a, 0, sizeof(int64_t) * (m + 1), s), "memset");
             const size_t smem_count = 2 * sizeof(uint32_t) * (size_t)W;
             const size_t smem_fill = 4 * sizeof(uint32_t) * (size_t)W;
+            // the limit of the widest bitmap, not of this one's: another thread's
+            // smaller one would come between here and the launches
             check_cuda(cudaFuncSetAttribute(ada_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem_count),
+                                            (int)(2 * sizeof(uint32_t) * kMaxBitmapWords)),
                        "smem attribute");
             check_cuda(cudaFuncSetAttribute(ada_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem_fill),
+                                            (int)(4 * sizeof(uint32_t) * kMaxBitmapWords)),
                        "smem attribute");
             const int grid = (int)std::min<int64_t>(std::max<int64_t>(m, 1), (int64_t)ctx().sm_count * 8);
             if (m > 0) {
