@@ -48,9 +48,9 @@ void require_init() {
 // ones freed longest ago making room (blocks of a model that is gone would
 // otherwise keep the next one's out: after a batch of 384 LPs a 20,000-row
 // set-up took 5.1 ms, 2.9 now). All go back when an allocation fails for lack
-// of memory, in hn_trim and in hn_shutdown. Any thread may allocate or free. A block is
-// known by its allocation's id: one that was freed past the library and whose
-// address the driver gave to somebody else is not taken for it.
+// of memory, in hn_trim and in hn_shutdown. Any thread may allocate or free. A
+// block is known by its allocation's id: one that was freed past the library
+// and whose address the driver gave to somebody else is not taken for it.
 namespace {
 // The driver's id of the allocation that p lies in, unique in the process's
 // life; 0 if there is none (0.1 us).
@@ -246,37 +246,46 @@ void pool_release() { pool().release(); }
 // 0.13 ms.
 namespace {
 constexpr int kSlabWords = 1024;
-std::mutex g_words_mu;
-std::vector<int32_t*> g_slabs, g_words;  // the slabs, their free words
+struct HostWords {
+    std::mutex mu;
+    std::vector<int32_t*> slabs, free;  // the slabs, their free words
+};
+HostWords& host_words() {
+    static HostWords* w = new HostWords();  // outlives every object
+    return *w;
+}
 }  // namespace
 
 int32_t* host_word() {
-    std::lock_guard<std::mutex> lk(g_words_mu);
-    if (g_words.empty()) {
-        g_slabs.reserve(g_slabs.size() + 1);
-        g_words.reserve((g_slabs.size() + 1) * kSlabWords);  // room for every word that comes back
+    HostWords& W = host_words();
+    std::lock_guard<std::mutex> lk(W.mu);
+    if (W.free.empty()) {
+        W.slabs.reserve(W.slabs.size() + 1);
+        W.free.reserve((W.slabs.size() + 1) * kSlabWords);  // room for every word that comes back
         void* slab = nullptr;
         check_cuda(cudaHostAlloc(&slab, kSlabWords * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped),
                    "cudaHostAlloc");
-        g_slabs.push_back(static_cast<int32_t*>(slab));
-        for (int i = kSlabWords; i-- > 0;) g_words.push_back(g_slabs.back() + i);
+        W.slabs.push_back(static_cast<int32_t*>(slab));
+        for (int i = kSlabWords; i-- > 0;) W.free.push_back(W.slabs.back() + i);
     }
-    int32_t* w = g_words.back();
-    g_words.pop_back();
+    int32_t* w = W.free.back();
+    W.free.pop_back();
     return w;
 }
 
 void host_word_free(int32_t* w) {
-    std::lock_guard<std::mutex> lk(g_words_mu);
-    if (w) g_words.push_back(w);
+    HostWords& W = host_words();
+    std::lock_guard<std::mutex> lk(W.mu);
+    if (w) W.free.push_back(w);
 }
 
 void host_words_release() {
-    std::lock_guard<std::mutex> lk(g_words_mu);
-    if (g_words.size() < g_slabs.size() * kSlabWords) return;  // a handle has one
-    for (int32_t* slab : g_slabs) cudaFreeHost(slab);
-    g_slabs.clear();
-    g_words.clear();
+    HostWords& W = host_words();
+    std::lock_guard<std::mutex> lk(W.mu);
+    if (W.free.size() < W.slabs.size() * kSlabWords) return;  // a handle has one
+    for (int32_t* slab : W.slabs) cudaFreeHost(slab);
+    W.slabs.clear();
+    W.free.clear();
 }
 
 Workspace& workspace(cudaStream_t s) {

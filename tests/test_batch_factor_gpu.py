@@ -192,3 +192,20 @@ def test_instances_of_one_block(hn, torch_cuda, m):
                 assert np.array_equal(r[5][r[1][i]:r[1][i + 1]], r[4][r[1][i]:r[1][i + 1]])
             else:
                 check(i, *r, 1.0)
+
+
+def test_after_shutdown(hn, torch_cuda):
+    """hn_shutdown gives memory and host words back, with a handle alive or
+    without; the library goes on."""
+    ms = [70, 3, 64]
+    want = solve_batch(hn, torch_cuda, ms)[5]
+    hn.check(hn.load().hn_shutdown())
+    assert np.array_equal(solve_batch(hn, torch_cuda, ms)[5], want)
+    lib, p64, h = hn.load(), C.POINTER(C.c_int64), C.c_void_p()
+    A = hn.Csr(3, 3, [0, 1, 2, 4], [0, 1, 1, 2], [2.0, 1.0, 1.0, 1.0])
+    P, ro = hn.Pattern(A), np.array([0, 3], np.int64)
+    hn.check(lib.hn_batch_create(1, ro.ctypes.data_as(p64), ro.ctypes.data_as(p64), P.h, C.byref(h)))
+    hn.check(lib.hn_shutdown())
+    assert np.array_equal(solve_batch(hn, torch_cuda, ms)[5], want)
+    hn.check(lib.hn_batch_destroy(h))
+    hn.init(0)
